@@ -36,6 +36,7 @@
 #include "common.h"
 #include "kernels.cuh"
 #include "fused_launch.cuh"
+#include "fx64.h"
 #include "music.cuh"
 
 namespace mfx {
@@ -147,6 +148,10 @@ struct mfx_job {
   void *ffC[17] = {};          // C-space [M][M][N/2] complex
   float2 *ff_tw = nullptr;     // W_M^t, t < M
   float2 *ff_twn = nullptr;    // W_N^t, t < N (fused assembly)
+  // plain FP64 form: transforms in 64-bit fixed point (fx64.h) and their tables
+  bool fx = false;
+  longlong2 *fx_twm = nullptr, *fx_twn = nullptr;  // twiddles of M and N
+  double *fx_mode = nullptr, *fx_rinv = nullptr;   // fx::Strided::mode, rinv
   int *dstatus = nullptr;      // device status word: nonzero when a kernel's bounded wait ran out
   size_t rsize = 8;
   cudaStream_t stream = nullptr;
@@ -275,7 +280,7 @@ struct Layout {
   size_t seeds, amp, plt, phase, nfields, region, work_est, total;
   size_t n_field, m_field, asm_bytes, part_bytes, mregion, music;
   int nslots, group;
-  size_t ff_b, ff_d, ff_tw, status;
+  size_t ff_b, ff_d, ff_tw, status, fx;
   int ff_nc;
 };
 
@@ -386,6 +391,19 @@ static bool fused_supported(const mfx_job_desc *d) {
   return (N / 2) % 8 == 0 && ff::ff_length_supported(M);
 }
 
+// The plain FP64 form runs its transforms in 64-bit fixed point (fx64.cuh) for
+// grids whose length and padded length have no prime factor above 7; other
+// grids use cuFFT.  MFX_FUSED=0 sends this form through cuFFT as well.  One
+// padded D2Z at 384^3 took cuFFT 7.15 ms, the three fixed-point passes 1.6 ms
+// without any pruning; at 96^3 0.11 and 0.04 ms: no size favours cuFFT.
+static bool fx_supported(const mfx_job_desc *d) {
+  if (d->precision != MFX_FP64) return false;
+  const char *env = getenv("MFX_FUSED");
+  if (env && env[0] == '0') return false;
+  const int N = d->ngrid;
+  return fx::length_supported(N) && (d->lpt_order < 2 || fx::length_supported(3 * N / 2));
+}
+
 // group_all: hold every sub-lattice's assembled components at once even where
 // that grows the region beyond the padded fields (the fused assembly then
 // assembles each mode once for all sub-lattices)
@@ -418,6 +436,9 @@ static Layout plan_layout(const mfx_job_desc *d, size_t work_bytes, bool group_a
     L.ff_tw = align_up(size_t(M) * 8) + align_up(size_t(N) * 8);
     L.status = align_up(sizeof(int));
   }
+  if (fx_supported(d))
+    L.fx = align_up(size_t(M) * sizeof(longlong2)) + align_up(size_t(N) * sizeof(longlong2)) +
+           align_up(2 * size_t(N) * 8) + align_up(fx::rinv_len(N) * 8);
   const size_t np = size_t(ns) * N * N * N;
   L.part_bytes = 0;
   if (d->want_particles) {
@@ -446,7 +467,7 @@ static Layout plan_layout(const mfx_job_desc *d, size_t work_bytes, bool group_a
       L.music = align_up(n_field_bytes(1 << ml.l0, rs)) +
                 (ml.l0 - ml.lmin >= 2 ? align_up(n_field_bytes(1 << (ml.l0 - 1), rs)) : 0);
   }
-  L.total = L.seeds + L.amp + L.plt + L.phase + L.ff_tw + L.status + L.nfields + L.region + L.work_est + L.music;
+  L.total = L.seeds + L.amp + L.plt + L.phase + L.ff_tw + L.status + L.fx + L.nfields + L.region + L.work_est + L.music;
   return L;
 }
 
@@ -885,6 +906,211 @@ static int run_potentials_fused(mfx_job *j) {
   return MFX_OK;
 }
 
+// ---------------------------------------------------------------------------
+// pruned transforms of the plain FP64 form in fixed point (fx64.h)
+// ---------------------------------------------------------------------------
+// The padded fields stay in their M-grid slots throughout: a slot holds rows
+// (x, y) of M + 2 reals or their kz < M/2 + 1 spectra; after the y pass of an
+// inverse transform only the x < N rows are used (the N-grid kx).  Modes with
+// kz >= N/2 (+ 1 where the noise fills the Nyquist planes) are never touched.
+static int fx_pass(mfx_job *j, const fx::Strided &s, const char *name, double bytes) {
+  KBEGIN(j);
+  const cudaError_t e = fx::run_strided(s, j->stream);
+  if (e != cudaSuccess) return set_error(MFX_ECUDA, "%s (length %d): %s", name, s.L, cudaGetErrorString(e));
+  KEND(j, name, bytes);
+  return MFX_OK;
+}
+static int fx_rows(mfx_job *j, int L, const longlong2 *tw, int kc, void *const *f, int count, bool inverse,
+                   const char *name) {
+  fx::Rows r{};
+  r.L = L;
+  r.tw = tw;
+  r.kc = kc;
+  r.rows = (long long)L * L;
+  r.pitch = L + 2;
+  r.count = count;
+  for (int c = 0; c < count; ++c) r.field[c] = static_cast<double *>(f[c]);
+  KBEGIN(j);
+  const cudaError_t e = inverse ? fx::run_c2r(r, j->stream) : fx::run_r2c(r, j->stream);
+  if (e != cudaSuccess) return set_error(MFX_ECUDA, "%s (length %d): %s", name, L, cudaGetErrorString(e));
+  KEND(j, name, double(count) * L * L * (16.0 * kc + 8.0 * L));
+  return MFX_OK;
+}
+// one op per field in its own group
+static void fx_ops(fx::Strided &s, int count, void *const *src, void *const *dst) {
+  s.ops = s.groups = count;
+  for (int c = 0; c < count; ++c) {
+    s.first[c] = c;
+    s.src[c] = static_cast<const double2 *>(src[c]);
+    s.dst[c] = static_cast<double2 *>(dst[c]);
+  }
+  s.first[count] = count;
+}
+static fx::Strided fx_base(const mfx_job *j, int kc) {
+  fx::Strided s{};
+  s.L = j->M;
+  s.tw = j->fx_twm;
+  s.n = j->N;
+  s.kc = kc;
+  s.mode = j->fx_mode;
+  s.rinv = j->fx_rinv;
+  return s;
+}
+// passes along y (outer: x rows) and x (outer: y rows) of an M-grid slot
+static void fx_slot_y(const mfx_job *j, fx::Strided &s) {
+  s.outer = j->N;
+  s.in_outer = s.out_outer = (long long)j->M * j->mk;
+  s.in_row = s.out_row = j->mk;
+}
+static void fx_slot_x(const mfx_job *j, fx::Strided &s) {
+  s.outer = j->M;
+  s.in_outer = s.out_outer = j->mk;
+  s.in_row = s.out_row = (long long)j->M * j->mk;
+}
+
+// ka kb phi on the padded real grid, k in units of 2 pi / L (the Hessian
+// functor of convolution.hh:136-157 without its factor -(2 pi / L)^2 and the
+// pad factor, which the later passes put in): along y, phi, ky phi and ky^2 phi
+// go to the slots of zz, yz and yy; along x, each of these makes its group's
+// outputs with kx and kz factors, the one in its own slot last
+static int fx_hessians(mfx_job *j, const void *phi, void **H, int kc) {
+  const double N = j->N, M = j->M, by = 16.0 * kc;
+  fx::Strided y = fx_base(j, kc);
+  y.inverse = true;
+  y.pad_in = true;
+  fx_slot_y(j, y);
+  y.in_outer = (long long)j->N * j->nk;
+  y.in_row = j->nk;
+  void *src[3] = {const_cast<void *>(phi), const_cast<void *>(phi), const_cast<void *>(phi)};
+  void *dst[3] = {H[2], H[5], H[1]};
+  fx_ops(y, 3, src, dst);
+  for (int o = 0; o < 3; ++o) y.pr[o] = o;
+  TRY(fx_pass(j, y, "fx_y3", (N * N + 3 * N * M) * by));
+  fx::Strided x = fx_base(j, kc);
+  x.inverse = true;
+  x.pad_in = true;
+  fx_slot_x(j, x);
+  //                 xx       xz       zz       xy       yz       yy
+  const int in[6] = {2, 2, 2, 5, 5, 1}, out[6] = {0, 4, 2, 3, 5, 1}, pr[6] = {2, 1, 0, 1, 0, 0}, pk[6] = {0, 1, 2, 0, 1, 0};
+  x.ops = 6;
+  x.groups = 3;
+  x.first[0] = 0;
+  x.first[1] = 3;
+  x.first[2] = 5;
+  x.first[3] = 6;
+  for (int o = 0; o < 6; ++o) {
+    x.src[o] = static_cast<const double2 *>(H[in[o]]);
+    x.dst[o] = static_cast<double2 *>(H[out[o]]);
+    x.pr[o] = pr[o];
+    x.pk[o] = pk[o];
+  }
+  TRY(fx_pass(j, x, "fx_x6", (3 * N * M + 6 * M * M) * by));
+  return fx_rows(j, j->M, j->fx_twm, kc, H, 6, true, "fx_z_c2r");
+}
+
+// real fields F[count] -> k-space, unpadded: -fac F / |k|^2 (fac includes the
+// Hessians' factors) into N-grid fields out[count]
+static int fx_unpad(mfx_job *j, void **F, void *const *out, int count, double fac) {
+  const double N = j->N, M = j->M, by = 16.0 * j->nh;
+  TRY(fx_rows(j, j->M, j->fx_twm, j->nh, F, count, false, "fx_z_r2c"));
+  fx::Strided x = fx_base(j, j->nh);
+  fx_slot_x(j, x);
+  x.cut_out = true;
+  fx_ops(x, count, F, F);
+  TRY(fx_pass(j, x, "fx_x_fwd", count * (M * M + N * M) * by));
+  fx::Strided y = fx_base(j, j->nh);
+  fx_slot_y(j, y);
+  y.out_outer = (long long)j->N * j->nk;
+  y.out_row = j->nk;
+  y.cut_out = y.inv_lap = true;
+  y.fac = fac;
+  fx_ops(y, count, F, out);
+  return fx_pass(j, y, "fx_y_fwd", count * (N * M + N * N) * by);
+}
+
+// convolve3's first pairs (convolution.hh:525-532): forward, the N-grid modes
+// kept times fac, and back
+static int fx_truncate(mfx_job *j, void **F, int count, double fac) {
+  const double N = j->N, M = j->M, by = 16.0 * j->nh;
+  TRY(fx_rows(j, j->M, j->fx_twm, j->nh, F, count, false, "fx_z_r2c"));
+  fx::Strided x = fx_base(j, j->nh);
+  fx_slot_x(j, x);
+  x.cut_out = true;
+  fx_ops(x, count, F, F);
+  TRY(fx_pass(j, x, "fx_x_fwd", count * (M * M + N * M) * by));
+  fx::Strided y = fx_base(j, j->nh);
+  fx_slot_y(j, y);
+  y.truncate = true;
+  y.fac = fac;
+  fx_ops(y, count, F, F);
+  TRY(fx_pass(j, y, "fx_y_trunc", count * 2 * N * M * by));
+  fx::Strided xi = fx_base(j, j->nh);
+  fx_slot_x(j, xi);
+  xi.inverse = xi.pad_in = true;
+  fx_ops(xi, count, F, F);
+  TRY(fx_pass(j, xi, "fx_x_inv", count * (M * M + N * M) * by));
+  return fx_rows(j, j->M, j->fx_twm, j->nh, F, count, true, "fx_z_c2r");
+}
+
+// in-place N-grid c2r of `count` k-space fields
+static int fx_c2r_n(mfx_job *j, void *const *f, int count) {
+  const int kc = j->d.noise_generator == MFX_NOISE_NGENIC ? j->nh : j->nk;  // NGenIC's Nyquist planes are empty
+  const double by = 32.0 * double(j->N) * j->N * kc * count;
+  for (int axis = 1; axis >= 0; --axis) {
+    fx::Strided s{};
+    s.L = s.n = j->N;
+    s.tw = j->fx_twn;
+    s.kc = kc;
+    s.inverse = true;
+    s.outer = j->N;
+    s.in_outer = s.out_outer = axis ? (long long)j->N * j->nk : j->nk;
+    s.in_row = s.out_row = axis ? j->nk : (long long)j->N * j->nk;
+    fx_ops(s, count, f, f);
+    TRY(fx_pass(j, s, axis ? "fx_n_y" : "fx_n_x", by));
+  }
+  return fx_rows(j, j->N, j->fx_twn, kc, f, count, true, "fx_n_c2r");
+}
+
+// LPT potentials of the plain FP64 form.  Slots as in the cuFFT route: 0..5 the
+// phi1 Hessians, 6..10 sources and pair products, 11..16 the phi2 Hessians.
+static int run_potentials_fx(mfx_job *j) {
+  const int nsm = num_sm();
+  const double M3 = double(j->M) * j->M * j->M, N3 = double(j->N) * j->N * j->N;
+  const double kf = 2.0 * M_PI / j->d.boxlen;
+  // With M = 3N/2 the pad factor 1.5^1.5, the unitary 1 / sqrt(M^3) and
+  // sqrt(M^3 / N^3) of the unpadding combine: a Hessian's factor is -h,
+  // h = kf^2 / sqrt(N^3); an unpadded product of two carries h^2 sqrt(N^3) / M^3,
+  // over kf^2 for the inverse Laplacian; a truncated pair 1 / M^3 and the -h of
+  // the third Hessian.  Evaluated with the fewest roundings: they scale a field.
+  const double ufac = kf * kf / (M3 * std::sqrt(N3)), tfac = -ufac;
+  const size_t mreal = size_t(j->M) * j->M * (j->M + 2);
+  const unsigned grid = grid_for(mreal, 256, nsm);
+  void **H1 = &j->mslot[0], **T = &j->mslot[6], **H2 = &j->mslot[11];
+  SrcArgs s{};
+  TRY(fx_hessians(j, j->nf[0], H1, j->d.noise_generator == MFX_NOISE_NGENIC ? j->nh : j->nk));
+  for (int c = 0; c < 6; ++c) s.h1[c] = H1[c];
+  s.count = mreal;
+  s.out[0] = T[0];
+  KBEGIN(j);
+  k_src2<double><<<grid, 256, 0, j->stream>>>(s);
+  KEND(j, "src2", 7.0 * j->m_field_bytes);
+  TRY(fx_unpad(j, T, &j->nf[1], 1, ufac));
+  if (j->timed) CU(cudaEventRecord(j->ev[2], j->stream));
+  if (j->d.lpt_order < 3) return MFX_OK;
+  for (int t = 0; t < 5; ++t) s.out[t] = T[t];
+  KBEGIN(j);
+  k_pairs3a<double><<<grid, 256, 0, j->stream>>>(s);
+  KEND(j, "pairs3a", 10.0 * j->m_field_bytes);
+  TRY(fx_truncate(j, T, 5, tfac));
+  TRY(fx_hessians(j, j->nf[1], H2, j->nh));
+  for (int c = 0; c < 6; ++c) s.h2[c] = H2[c];
+  for (int t = 0; t < 5; ++t) s.t[t] = T[t];
+  KBEGIN(j);
+  k_src3<double><<<grid, 256, 0, j->stream>>>(s);
+  KEND(j, "src3", 21.0 * j->m_field_bytes);
+  return fx_unpad(j, T, &j->nf[2], 4, ufac);
+}
+
 // default tile shapes: the largest x/y tile of at most 512 threads, and one
 // row per step of the persistent z passes (two fit one CTA per SM only)
 static void ff_default_tiles(mfx_job *j) {
@@ -1233,7 +1459,9 @@ template <typename R> static int assemble_stage(mfx_job *j, int mask) {
     else k_assemble<R, false><<<grid_for(total, 256, nsm), 256, 0, j->stream>>>(a);
     KEND(j, "assemble", ((order == 1 ? 1.0 : (order == 2 ? 2.0 : 6.0)) + 6.0 * g) * j->n_field_bytes);
     for (int s = 0; s < g; ++s) {
-      TRY(exec_fft(j, j->n_c2r, j->asmbuf[s * 6], false));  // the six components (batched)
+      // the six components (batched)
+      if (j->fx) TRY(fx_c2r_n(j, &j->asmbuf[s * 6], 6));
+      else TRY(exec_fft(j, j->n_c2r, j->asmbuf[s * 6], false));
       PartArgs p{};
       for (int q = 0; q < 6; ++q) p.f[q] = j->asmbuf[s * 6 + q];
       p.pos = j->pos;
@@ -1295,6 +1523,8 @@ template <typename R> static int run_pipeline(mfx_job *j) {
   void **H1 = &j->mslot[0];
   if (j->fused) {
     TRY(run_potentials_fused(j));
+  } else if (j->fx && order >= 2) {
+    TRY(run_potentials_fx(j));
   } else {
   if (order >= 2) {
     TRY(hessians<R>(j, j->nf[0], H1));
@@ -1700,16 +1930,17 @@ static int create_job(mfx_engine *eng, const mfx_job_desc *d, mfx_job **out, int
   // plans
   size_t work = 0;
   j->fused = fused_supported(d);
+  j->fx = fx_supported(d);
   if (j->fused) {
     ff_default_tiles(j);
     tune_fused(j);
   }
-  if (d->lpt_order >= 2 && !j->fused) {
+  if (d->lpt_order >= 2 && !j->fused && !j->fx) {
     if ((rc = acquire_plan(eng, j->m_r2c, j->M, j->fp64, true)) != MFX_OK) return fail(rc);
     if ((rc = acquire_plan(eng, j->m_c2r, j->M, j->fp64, false)) != MFX_OK) return fail(rc);
     work = std::max(work, std::max(j->m_r2c.work, j->m_c2r.work));
   }
-  if (d->want_particles && !j->fused) {
+  if (d->want_particles && !j->fused && !j->fx) {
     // the six assembled components of a sub-lattice lie one padded field apart:
     // one batched c2r per sub-lattice
     const long long nfb = (long long)align_up(n_field_bytes(j->N, j->rsize));
@@ -1793,6 +2024,24 @@ static int create_job(mfx_engine *eng, const mfx_job_desc *d, mfx_job **out, int
   p += L.ff_tw;
   j->dstatus = L.status ? reinterpret_cast<int *>(p) : nullptr;
   p += L.status;
+  if (j->fx) {
+    char *f = p;
+    j->fx_twm = reinterpret_cast<longlong2 *>(f);
+    f += align_up(size_t(j->M) * sizeof(longlong2));
+    j->fx_twn = reinterpret_cast<longlong2 *>(f);
+    f += align_up(size_t(j->N) * sizeof(longlong2));
+    j->fx_mode = reinterpret_cast<double *>(f);
+    f += align_up(2 * size_t(j->N) * 8);
+    j->fx_rinv = reinterpret_cast<double *>(f);
+    cudaError_t fe = fx::prepare_device(eng->device);
+    for (const int len : {j->M, j->N})
+      if (fe == cudaSuccess && (len == j->N || d->lpt_order >= 2))
+        fe = cudaMemcpyAsync(len == j->M ? j->fx_twm : j->fx_twn, fx::twiddles(len), size_t(len) * sizeof(longlong2),
+                             cudaMemcpyHostToDevice, j->stream);
+    if (fe == cudaSuccess) fe = fx::fill_tables(j->N, j->fx_mode, j->fx_rinv, j->stream);
+    if (fe != cudaSuccess) return fail(set_error(MFX_ECUDA, "fixed-point transform set-up: %s", cudaGetErrorString(fe)));
+  }
+  p += L.fx;
   if (j->dstatus && (cudaMemsetAsync(j->dstatus, 0, sizeof(int), j->stream) != cudaSuccess))
     return fail(set_error(MFX_ECUDA, "status word reset failed"));
   const int nfield = d->lpt_order == 1 ? 1 : (d->lpt_order == 2 ? 2 : 6);
@@ -2007,7 +2256,7 @@ int mfx_job_footprint(mfx_engine *eng, const mfx_job_desc *desc, size_t *bytes) 
   // padded cuFFT transforms (plain form), the batch of six N-grid c2r
   const int M = 3 * desc->ngrid / 2;
   const size_t rs = desc->precision == MFX_FP64 ? 8 : 4;
-  const bool fused = fused_supported(desc);
+  const bool fused = fused_supported(desc) || fx_supported(desc);
   size_t work = (desc->want_particles && !fused) ? 6 * n_field_bytes(desc->ngrid, rs) : 0;
   if (desc->lpt_order >= 2 && !fused) work = std::max(work, size_t(M) * M * (M / 2 + 1) * 2 * rs);
   if (desc->noise_generator == MFX_NOISE_MUSIC1) work = std::max(work, n_field_bytes(desc->ngrid, rs));

@@ -1,0 +1,565 @@
+// Kernels of the fixed-point transforms (fx64.cuh) of the plain FP64 form and
+// their launches.
+//
+// A 3D transform is three passes over pencils.  A CTA holds P pencils in
+// shared memory (16 L P bytes, one buffer: a step reads all its inputs into
+// registers before it writes), two steps for most lengths up to 576.
+//   load   doubles from HBM into shared memory, largest exponent per pencil
+//   steps  Stockham, the first one converting to fixed point as it reads
+//   store  back to doubles, to HBM
+// Pencils are interleaved ([element][pencil], the pencil index swizzled by the
+// element) so that the eight lanes of a 128-byte shared-memory phase always
+// read eight different columns, whatever the step's stride.
+// Passes skip what the Orszag padding makes zero (the cuFFT route transformed
+// it): of the 1.5 M^2 pencils of a padded c2r only N kz/2 + M kz/2 are run
+// along y and x, and the Hessian and inverse-Laplacian factors and the
+// truncation of convolve3 (convolution.hh:525-532, 552-636) are applied while
+// loading and storing.
+#include "fx64.cuh"
+#include "fx64.h"
+#include "fx64_len.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <map>
+#include <mutex>
+#include <vector>
+
+namespace fx {
+
+// ---------------------------------------------------------------------------
+// plans
+// ---------------------------------------------------------------------------
+namespace {
+constexpr int kRadices[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+constexpr int kSmemMax = 220 * 1024;
+
+// rough cost of a point: real multiplications (three products each, measured
+// 4 a clock) and the shared-memory round trip of a step
+double radix_cost(int R) {
+  switch (R) {
+    case 2: case 4: return 0.0;
+    case 3: return 0.67; case 5: return 2.0; case 6: return 0.67; case 7: return 5.1;
+    case 8: return 0.5; case 9: return 2.0; case 10: return 2.0; case 12: return 0.67;
+    case 14: return 5.1; case 15: return 2.67; case 16: return 1.25; case 18: return 2.0;
+    case 20: return 2.0; default: return 1.17;  // 24
+  }
+}
+
+// best factorisation: fewest steps, then least cost, then smallest largest radix
+void search(int rest, int depth, double cost, int *cur, int &best_n, double &best_c, int *best) {
+  if (rest == 1) {
+    int mx = 0;
+    for (int q = 0; q < depth; ++q) mx = std::max(mx, cur[q]);
+    const double c = cost + 0.02 * mx;
+    if (depth < best_n || (depth == best_n && c < best_c)) {
+      best_n = depth;
+      best_c = c;
+      std::copy(cur, cur + depth, best);
+    }
+    return;
+  }
+  if (depth == kMaxSteps || depth >= best_n) return;
+  for (int R : kRadices)
+    if (rest % R == 0 && (depth == 0 || R <= cur[depth - 1])) {
+      cur[depth] = R;
+      search(rest / R, depth + 1, cost + radix_cost(R), cur, best_n, best_c, best);
+    }
+}
+}  // namespace
+
+int fx_bits(const int *R, int steps, FxKind kind) {
+  double m = kind == FX_C2R ? 1.5 : 0.5, top = m;
+  for (int q = 0; q < steps; ++q) {
+    if (q) m -= 3.0;
+    m += std::log2(double(R[q]));
+    top = std::max(top, m);
+  }
+  if (kind == FX_R2C) top = std::max(top, m + 1.0);
+  return std::min(60, int(std::floor(62.7 - top)));
+}
+
+bool fx_plan(int L, FxKind kind, FxPlan *p) {
+  *p = FxPlan{};
+  p->L = L;
+  int cur[kMaxSteps], best[kMaxSteps], n = kMaxSteps + 1;
+  double c = 1e30;
+  search(L, 0, 0.0, cur, n, c, best);
+  if (n > kMaxSteps) return false;
+  p->steps = n;
+  // smallest radix first: its butterflies, the most, carry no twiddles
+  std::sort(best, best + n);
+  int ns = 1;
+  for (int q = 0; q < n; ++q) {
+    p->R[q] = best[q];
+    p->NS[q] = ns;
+    p->magic[q] = unsigned((0x100000000ULL + unsigned(ns) - 1) / unsigned(ns));
+    ns *= best[q];
+  }
+  p->B = fx_bits(p->R, n, kind);
+  for (int P : {8, 4, 2}) {
+    // threads: at least what the steps' butterflies need, and enough of them
+    // that short pencils still fill a few warps
+    int need = 32, most = 32;
+    for (int q = 0; q < n; ++q) {
+      const int items = P * (L / p->R[q]), mu = radix_mult(p->R[q]);
+      need = std::max(need, (items + mu - 1) / mu);
+      most = std::max(most, items);
+    }
+    int T = std::max(need, std::min(most, 256));
+    T = (T + 31) / 32 * 32;
+    const int smem = L * P * 16 + P * 8;
+    if (T > 384 || smem > kSmemMax) continue;
+    p->P = P;
+    p->lgP = P == 8 ? 3 : (P == 4 ? 2 : 1);
+    p->T = T;
+    p->smem = smem;
+    return true;
+  }
+  return false;
+}
+
+void fx_twiddles(int L, longlong2 *out) {
+  for (int t = 0; t < L; ++t) {
+    const CS w = q62_turn(t, L);
+    out[t] = make_longlong2((long long)((w.c + 1) >> 1), (long long)((-w.s + 1) >> 1));
+  }
+}
+
+bool length_supported(int L) { return fx_supported(L); }
+const longlong2 *twiddles(int L) {
+  static std::mutex mu;
+  static std::map<int, std::vector<longlong2>> tables;
+  std::lock_guard<std::mutex> lk(mu);
+  std::vector<longlong2> &t = tables[L];
+  if (t.empty()) {
+    t.resize(L);
+    fx_twiddles(L, t.data());
+  }
+  return t.data();
+}
+
+// ---------------------------------------------------------------------------
+// device code
+// ---------------------------------------------------------------------------
+struct Core {
+  FxPlan p;
+  const longlong2 *tw;
+};
+
+__device__ __forceinline__ int slot(int e, int q, int lgP) { return (e << lgP) + (q ^ (e & ((1 << lgP) - 1))); }
+
+// one Stockham step of radix R over the CTA's pencils; raw: the values are
+// still doubles (sh: the conversion of this thread's pencil)
+template <int R>
+__device__ __noinline__ void step(const longlong2 *tw, int L, int lgP, int NS, unsigned magic, bool raw, int sh) {
+  extern __shared__ __align__(16) longlong2 s[];
+  constexpr int MU = radix_mult(R);
+  const int T = blockDim.x, t = threadIdx.x;
+  const int nb = L / R, items = nb << lgP;
+  const int pen = t & ((1 << lgP) - 1);
+  I2 v[MU][R];
+  int jn[MU];
+#pragma unroll
+  for (int m = 0; m < MU; ++m) {
+    const int it = t + m * T;
+    jn[m] = -1;
+    if (it < items) {
+      const int j = it >> lgP;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const longlong2 w = s[slot(j + r * nb, pen, lgP)];
+        v[m][r] = {w.x, w.y};
+      }
+      if (NS == 1) {
+        jn[m] = j * R;
+        if (raw) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            v[m][r].x = to_fixed(__longlong_as_double(v[m][r].x), sh);
+            v[m][r].y = to_fixed(__longlong_as_double(v[m][r].y), sh);
+          }
+        }
+      } else {
+        const int hi = int(__umulhi(unsigned(j), magic)), lo = j - hi * NS;
+        jn[m] = hi * NS * R + lo;
+        const int inc = lo * (nb / NS);  // lo L / (NS R)
+        v[m][0] = eighth(v[m][0]);
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[m][r] = twiddle8(v[m][r], __ldg(&tw[r * inc]));
+      }
+      Dft<R>::run(v[m]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < MU; ++m)
+    if (jn[m] >= 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) s[slot(jn[m] + r * NS, pen, lgP)] = make_longlong2(v[m][r].x, v[m][r].y);
+    }
+  __syncthreads();
+}
+
+// all steps; ends with a barrier
+__device__ __forceinline__ void transform(const Core &c, bool raw, int sh) {
+#pragma unroll 1
+  for (int q = 0; q < c.p.steps; ++q) {
+    const bool rw = raw && q == 0;
+    const int L = c.p.L, lgP = c.p.lgP, NS = c.p.NS[q];
+    const unsigned mg = c.p.magic[q];
+    switch (c.p.R[q]) {
+      case 2: step<2>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 3: step<3>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 4: step<4>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 5: step<5>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 6: step<6>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 7: step<7>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 8: step<8>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 9: step<9>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 10: step<10>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 12: step<12>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 14: step<14>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 15: step<15>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 16: step<16>(c.tw, L, lgP, NS, mg, rw, sh); break;
+    }
+  }
+}
+
+struct SArgs {
+  Core c;
+  Strided s;
+};
+
+__global__ void __launch_bounds__(384) k_fx_strided(const __grid_constant__ SArgs a) {
+  extern __shared__ __align__(16) longlong2 sm[];
+  const Strided &d = a.s;
+  const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x;
+  int *emax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));
+  const int kblocks = (d.kc + P - 1) >> lgP;
+  const int o = blockIdx.x / kblocks, kz0 = (blockIdx.x - o * kblocks) << lgP;
+  const int pen = t & (P - 1), kz = kz0 + pen;
+  const bool live = kz < d.kc;
+  const int n = d.n, nh = n >> 1;
+  const int step_l = T >> lgP;
+  for (int op = d.first[blockIdx.y]; op < d.first[blockIdx.y + 1]; ++op) {
+    if (t < P) emax[t] = 0;
+    __syncthreads();
+    // load
+    const double2 *src = d.src[op] + (long long)o * d.in_outer + kz;
+    const int pr = d.pr[op], pk = d.pk[op];
+    const bool scaled = (pr | pk) != 0;
+    const double kf = pk == 0 ? 1.0 : ((d.inverse && kz == nh) ? 0.0 : (pk == 1 ? double(kz) : double(kz) * double(kz)));
+    int em = 0;
+#pragma unroll 4
+    for (int l = t >> lgP; l < L; l += step_l) {
+      double2 v = make_double2(0.0, 0.0);
+      const int i = !d.pad_in ? l : (l <= nh ? l : (l > n ? l - nh : -1));
+      if (live && i >= 0) {
+        v = src[(long long)i * d.in_row];
+        if (scaled) {
+          const double f = (pr ? __ldg(&d.mode[(pr - 1) * n + i]) : 1.0) * kf;
+          v.x *= f;
+          v.y *= f;
+        }
+      }
+      em = max(em, max(dbl_exponent(v.x), dbl_exponent(v.y)));
+      sm[slot(l, pen, lgP)] = d.inverse ? make_longlong2(__double_as_longlong(v.y), __double_as_longlong(v.x))
+                                        : make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
+    }
+    for (int off = P; off < 32; off <<= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, off));
+    if ((t & 31) < P) atomicMax(&emax[pen], em);
+    __syncthreads();
+    em = emax[pen];
+    bool bad = em == 2047;
+    int S = em - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1);
+    transform(a.c, true, em + 63 - a.c.p.B);
+    bool inverse = d.inverse;
+    if (d.truncate) {
+      // keep the N-grid modes, bring the largest back below 2^B, swap for the
+      // inverse transform (inverse = swap, forward, swap)
+      int bits = 0;
+      for (int l = t >> lgP; l < L; l += step_l) {
+        const bool keep = l < nh || l > n;
+        longlong2 &w = sm[slot(l, pen, lgP)];
+        const longlong2 v = w;
+        if (keep) bits = max(bits, 64 - min(__clzll(v.x ^ (v.x >> 63)), __clzll(v.y ^ (v.y >> 63))));
+        w = keep ? make_longlong2(v.y, v.x) : make_longlong2(0, 0);
+      }
+      if (t < P) emax[t] = 0;
+      __syncthreads();
+      for (int off = P; off < 32; off <<= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, off));
+      if ((t & 31) < P) atomicMax(&emax[pen], bits);
+      __syncthreads();
+      const int down = emax[pen] - a.c.p.B;
+      for (int l = t >> lgP; l < L; l += step_l) {
+        longlong2 &w = sm[slot(l, pen, lgP)];
+        if (down > 0) {
+          const long long half = 1LL << (down - 1);
+          w = make_longlong2((w.x + half) >> down, (w.y + half) >> down);
+        } else {
+          w = make_longlong2(w.x << -down, w.y << -down);
+        }
+      }
+      __syncthreads();
+      S += down + 3 * (a.c.p.steps - 1);
+      transform(a.c, false, 0);
+      inverse = true;
+    }
+    // store
+    double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
+    const int so = o > nh ? o - n : o;
+    for (int l = t >> lgP; l < L; l += step_l) {
+      const int i = !d.cut_out ? l : (l <= nh ? l : (l > n ? l - nh : -1));
+      if (i < 0 || !live) continue;
+      const longlong2 w = sm[slot(l, pen, lgP)];
+      double2 v = make_double2(to_double(w.x, S), to_double(w.y, S));
+      if (bad) v = make_double2(nan_of(), nan_of());
+      if (inverse) v = make_double2(v.y, v.x);
+      if (d.cut_out) {
+        if (i == nh || (d.inv_lap && (o == nh || (o | i | kz) == 0))) {
+          v = make_double2(0.0, 0.0);
+        } else if (d.inv_lap) {
+          const int si = i > nh ? i - n : i;
+          const double f = -d.fac * __ldg(&d.rinv[so * so + si * si + kz * kz]);
+          v.x *= f;
+          v.y *= f;
+        }
+      } else if (d.truncate) {
+        v.x *= d.fac;
+        v.y *= d.fac;
+      }
+      dst[(long long)i * d.out_row] = v;
+    }
+    if (d.inv_lap && kz0 + P >= d.kc) {
+      // the kz Nyquist column
+      double2 *z = d.dst[op] + (long long)o * d.out_outer + d.kc;
+      for (int i = t; i < n; i += T) z[(long long)i * d.out_row] = make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+  }
+}
+
+struct RArgs {
+  Core c;
+  Rows r;
+};
+
+// spectra -> real rows: rows 2q and 2q + 1 as the real and imaginary part of
+// one pencil, Z[k] = A[k] + i B[k], Z[L - k] = conj A[k] + i conj B[k]
+__global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a) {
+  extern __shared__ __align__(16) longlong2 sm[];
+  const Rows &d = a.r;
+  const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
+  int *emax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));
+  double *base = d.field[blockIdx.y];
+  const long long row0 = (long long)blockIdx.x * 2 * P;
+  const int h = L >> 1, kc = min(d.kc, h);  // the Nyquist value, if any, is handled apart
+  const bool nyq = d.kc > h;
+  if (t < P) emax[t] = 0;
+  // zero the elements without a mode
+  for (int e = t; e < ((L - 2 * kc + 1) << lgP); e += T) sm[slot(kc + (e >> lgP), e & (P - 1), lgP)] = make_longlong2(0, 0);
+  __syncthreads();
+  for (int q = t >> 5; q < 2 * P; q += T >> 5) {
+    const long long row = row0 + q;
+    const bool live = row < d.rows;
+    const double2 *src = reinterpret_cast<const double2 *>(base + row * d.pitch);
+    const int pen = q >> 1, second = q & 1;
+    int em = 0;
+#pragma unroll 4
+    for (int k = lane; k < kc; k += 32) {
+      double2 v = live ? src[k] : make_double2(0.0, 0.0);
+      if (k == 0) {
+        // only the real part of the k = 0 (and the Nyquist) value is used
+        em = max(em, dbl_exponent(v.x));
+        reinterpret_cast<double *>(&sm[slot(0, pen, lgP)])[second] = v.x;
+      } else {
+        em = max(em, max(dbl_exponent(v.x), dbl_exponent(v.y)));
+        sm[slot(second ? L - k : k, pen, lgP)] = make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
+      }
+    }
+    if (nyq && lane == 0) {
+      const double v = live ? src[h].x : 0.0;
+      em = max(em, dbl_exponent(v));
+      reinterpret_cast<double *>(&sm[slot(h, pen, lgP)])[second] = v;
+    }
+    em = __reduce_max_sync(0xffffffffu, unsigned(em));
+    if (lane == 0) atomicMax(&emax[pen], em);
+  }
+  __syncthreads();
+  {
+    // Z of both rows in fixed point, real and imaginary part exchanged (the
+    // inverse transform)
+    const int pen = t & (P - 1), sh = emax[pen] + 63 - a.c.p.B;
+    for (int k = t >> lgP; k < kc; k += T >> lgP) {
+      longlong2 &wa = sm[slot(k, pen, lgP)];
+      const longlong2 va = wa;
+      const long long ax = to_fixed(__longlong_as_double(va.x), sh), ay = to_fixed(__longlong_as_double(va.y), sh);
+      if (k == 0) {
+        wa = make_longlong2(ay, ax);
+        continue;
+      }
+      longlong2 &wb = sm[slot(L - k, pen, lgP)];
+      const longlong2 vb = wb;
+      const long long bx = to_fixed(__longlong_as_double(vb.x), sh), by = to_fixed(__longlong_as_double(vb.y), sh);
+      wa = make_longlong2(ay + bx, ax - by);
+      wb = make_longlong2(bx - ay, ax + by);
+    }
+    if (nyq && t < P) {
+      longlong2 &w = sm[slot(h, t, lgP)];
+      const longlong2 v = w;
+      w = make_longlong2(to_fixed(__longlong_as_double(v.y), sh), to_fixed(__longlong_as_double(v.x), sh));
+    }
+  }
+  __syncthreads();
+  transform(a.c, false, 0);
+  for (int q = t >> 5; q < 2 * P; q += T >> 5) {
+    const long long row = row0 + q;
+    if (row >= d.rows) break;
+    double *dst = base + row * d.pitch;
+    const int pen = q >> 1, second = q & 1;
+    const int S = emax[pen] - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1);
+    const bool bad = emax[pen] == 2047;
+    for (int e = lane; e < L; e += 32) {
+      // exchanged again: the first row is the imaginary part
+      const long long v = reinterpret_cast<const long long *>(&sm[slot(e, pen, lgP)])[1 - second];
+      dst[e] = bad ? nan_of() : to_double(v, S);
+    }
+  }
+}
+
+// real rows -> spectra of kz < kc, two rows a pencil
+__global__ void __launch_bounds__(384) k_fx_r2c(const __grid_constant__ RArgs a) {
+  extern __shared__ __align__(16) longlong2 sm[];
+  const Rows &d = a.r;
+  const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
+  int *emax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));
+  double *base = d.field[blockIdx.y];
+  const long long row0 = (long long)blockIdx.x * 2 * P;
+  if (t < P) emax[t] = 0;
+  __syncthreads();
+  for (int q = t >> 5; q < 2 * P; q += T >> 5) {
+    const long long row = row0 + q;
+    const bool live = row < d.rows;
+    const double *src = base + row * d.pitch;
+    const int pen = q >> 1, second = q & 1;
+    int em = 0;
+#pragma unroll 8
+    for (int e = lane; e < L; e += 32) {
+      const double v = live ? src[e] : 0.0;
+      em = max(em, dbl_exponent(v));
+      reinterpret_cast<double *>(&sm[slot(e, pen, lgP)])[second] = v;
+    }
+    em = __reduce_max_sync(0xffffffffu, unsigned(em));
+    if (lane == 0) atomicMax(&emax[pen], em);
+  }
+  __syncthreads();
+  transform(a.c, true, emax[t & (P - 1)] + 63 - a.c.p.B);
+  const int kc = d.kc;
+  for (int q = t >> 5; q < 2 * P; q += T >> 5) {
+    const long long row = row0 + q;
+    if (row >= d.rows) break;
+    double2 *dst = reinterpret_cast<double2 *>(base + row * d.pitch);
+    const int pen = q >> 1, second = q & 1;
+    // the sums below are twice the spectra
+    const int S = emax[pen] - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1) - 1;
+    const bool bad = emax[pen] == 2047;
+    for (int k = lane; k < kc; k += 32) {
+      const longlong2 u = sm[slot(k, pen, lgP)], w = sm[slot(k ? L - k : 0, pen, lgP)];
+      // A = (Z[k] + conj Z[L-k]) / 2, B = (Z[k] - conj Z[L-k]) / 2i
+      const long long x = second ? u.y + w.y : u.x + w.x, y = second ? w.x - u.x : u.y - w.y;
+      dst[k] = bad ? make_double2(nan_of(), nan_of()) : make_double2(to_double(x, S), to_double(y, S));
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// launches
+// ---------------------------------------------------------------------------
+// the instance of a length, if it has one
+using LenFn = cudaError_t (*)(FxOp, const void *, dim3, cudaStream_t);
+struct LenEntry {
+  int L;
+  LenFn fn;
+  int steps, R[3];
+};
+template <int L> constexpr LenEntry entry() {
+  return {L, launch_len<L>, Len<L>::steps, {Len<L>::R(0), Len<L>::R(1), Len<L>::R(2)}};
+}
+static const LenEntry kLens[] = {entry<16>(),  entry<24>(),  entry<32>(),  entry<48>(),  entry<64>(),  entry<72>(),
+                                 entry<96>(),  entry<128>(), entry<144>(), entry<192>(), entry<256>(), entry<288>(),
+                                 entry<384>(), entry<512>(), entry<576>(), entry<768>(), entry<1152>()};
+static const LenEntry *find_len(int L) {
+  for (const LenEntry &e : kLens)
+    if (e.L == L) return &e;
+  return nullptr;
+}
+
+static __global__ void k_fx_tables(int n, double *mode, double *rinv, int len) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < len; q += gridDim.x * blockDim.x) {
+    rinv[q] = q ? 1.0 / double(q) : 0.0;
+    if (q < n) {
+      const int i = q == n / 2 ? 0 : (q > n / 2 ? q - n : q);
+      mode[q] = double(i);
+      mode[n + q] = double(i) * double(i);
+    }
+  }
+}
+cudaError_t fill_tables(int n, double *mode, double *rinv, cudaStream_t st) {
+  const int len = int(rinv_len(n));
+  k_fx_tables<<<unsigned(std::min((len + 255) / 256, 608)), 256, 0, st>>>(n, mode, rinv, len);
+  return cudaGetLastError();
+}
+
+cudaError_t prepare_device(int dev) {
+  static std::mutex mu;
+  static std::vector<bool> done;
+  std::lock_guard<std::mutex> lk(mu);
+  if (dev < int(done.size()) && done[dev]) return cudaSuccess;
+  for (const void *f : {(const void *)k_fx_strided, (const void *)k_fx_c2r, (const void *)k_fx_r2c}) {
+    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    if (e != cudaSuccess) return e;
+  }
+  for (const LenEntry &l : kLens) {
+    const cudaError_t e = l.fn(FX_OP_PREPARE, nullptr, dim3(), nullptr);
+    if (e != cudaSuccess) return e;
+  }
+  if (dev >= int(done.size())) done.resize(dev + 1, false);
+  done[dev] = true;
+  return cudaSuccess;
+}
+
+cudaError_t run_strided(const Strided &s, cudaStream_t st) {
+  if (const LenEntry *l = find_len(s.L)) {
+    const LArgs a{s.tw, fx_bits(l->R, l->steps, FX_STRIDED), s};
+    return l->fn(s.truncate ? FX_OP_TRUNCATE : FX_OP_STRIDED, &a,
+                 dim3(unsigned(s.outer * ((s.kc + 7) / 8)), unsigned(s.groups)), st);
+  }
+  SArgs a;
+  if (!fx_plan(s.L, FX_STRIDED, &a.c.p)) return cudaErrorInvalidValue;
+  a.c.tw = s.tw;
+  a.s = s;
+  const int kb = (s.kc + a.c.p.P - 1) / a.c.p.P;
+  k_fx_strided<<<dim3(unsigned(s.outer * kb), unsigned(s.groups)), a.c.p.T, a.c.p.smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+static cudaError_t run_rows(const Rows &r, FxKind kind, cudaStream_t st) {
+  if (const LenEntry *l = find_len(r.L)) {
+    const LRows a{r.tw, fx_bits(l->R, l->steps, kind), r};
+    return l->fn(kind == FX_C2R ? FX_OP_C2R : FX_OP_R2C, &a, dim3(unsigned((r.rows + 15) / 16), unsigned(r.count)), st);
+  }
+  RArgs a;
+  if (!fx_plan(r.L, kind, &a.c.p)) return cudaErrorInvalidValue;
+  a.c.tw = r.tw;
+  a.r = r;
+  const long long per = 2 * a.c.p.P;
+  const dim3 grid(unsigned((r.rows + per - 1) / per), unsigned(r.count));
+  if (kind == FX_C2R) k_fx_c2r<<<grid, a.c.p.T, a.c.p.smem, st>>>(a);
+  else k_fx_r2c<<<grid, a.c.p.T, a.c.p.smem, st>>>(a);
+  return cudaGetLastError();
+}
+cudaError_t run_c2r(const Rows &r, cudaStream_t st) { return run_rows(r, FX_C2R, st); }
+cudaError_t run_r2c(const Rows &r, cudaStream_t st) { return run_rows(r, FX_R2C, st); }
+
+}  // namespace fx

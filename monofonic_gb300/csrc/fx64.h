@@ -1,0 +1,69 @@
+// Transforms of the plain FP64 form in 64-bit fixed point (fx64.cuh): what the
+// engine launches.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace fx {
+
+// a length the transforms are built for: even, no prime factor above 7
+bool length_supported(int L);
+// twiddle table of a length: L entries (host memory, kept for the process:
+// a few KB for each length that was asked for)
+const longlong2 *twiddles(int L);
+// device tables of a grid: mode[2][n] (Strided::mode) and rinv[q] = 1 / q,
+// q = 1 .. 3 (n/2)^2 (rinv[0] = 0)
+cudaError_t fill_tables(int n, double *mode, double *rinv, cudaStream_t st);
+inline size_t rinv_len(int n) { return 3 * size_t(n / 2) * (n / 2) + 1; }
+// the kernels' shared memory limits on the current device `dev`, once (before
+// any capture)
+cudaError_t prepare_device(int dev);
+
+// One pass over pencils along x or y of k-space arrays, 8 (or 4) adjacent kz a
+// CTA.  A pencil element (outer o, row r, kz) lies at base + o * outer + r *
+// row + kz (complex elements).
+struct Strided {
+  int L;                  // transform length
+  const longlong2 *tw;    // its twiddles
+  bool inverse;
+  int n;                  // N (the unpadded grid) for padded or cut rows
+  bool pad_in;            // rows r < n go to the padded positions of a length-L pencil (else r < L)
+  bool cut_out;           // the padded positions of r < n are stored as rows r, Nyquist row zero (else r < L)
+  int outer, kc;          // outer indices, kz values
+  long long in_outer, in_row, out_outer, out_row;
+  // up to 6 outputs in `groups` groups of consecutive ones: a CTA makes the
+  // outputs of one group in turn, so that the last may overwrite their source
+  int ops, groups, first[7];
+  const double2 *src[6];
+  double2 *dst[6];
+  // factors of an output's input: (row index)^pr (kz)^pk, signed mode indices
+  // with the Nyquist index n / 2 zero where the power is positive
+  int pr[6], pk[6];
+  const double *mode;     // [2][n]: signed index and its square, Nyquist zero (padded rows)
+  // cut_out: output factor.  inv_lap: times -fac / (i^2 + j^2 + k^2) with the
+  // Nyquist indices and k = 0 zero, outer index = mode index (rinv[q] = 1 / q),
+  // and the kz = kc column (Nyquist) zeroed
+  bool inv_lap;
+  const double *rinv;
+  double fac;
+  // forward transform, rows cut to n (Nyquist zero), factor fac, transformed
+  // back: convolve3's truncation between its two products
+  bool truncate;
+};
+cudaError_t run_strided(const Strided &s, cudaStream_t st);
+
+// Real rows: `rows` consecutive rows of L reals, `pitch` reals apart, in place
+// with their spectra (kz < kc complex values); two rows share a transform.
+struct Rows {
+  int L;
+  const longlong2 *tw;
+  int kc;                 // kz values of the spectrum (read or written); 2 (kc - 1) == L: with the Nyquist one
+  long long rows, pitch;
+  int count;              // fields
+  double *field[6];
+};
+cudaError_t run_c2r(const Rows &r, cudaStream_t st);
+cudaError_t run_r2c(const Rows &r, cudaStream_t st);
+
+}  // namespace fx

@@ -33,3 +33,16 @@ def oracle():
     from oracle import lpt
     lpt.build_lib()
     return lpt
+
+
+# Tests whose premise is a job that holds the GPU for tens of milliseconds: a
+# 192^3 3LPT job in the plain FP64 form took 95 ms on the cuFFT route and 18 ms
+# on the fixed-point one, less than the waits that these tests measure against
+# it.  They run on the cuFFT route (MFX_FUSED=0).
+SLOW_BLOCKER = {"test_server_small_jobs_beside_the_slots"}
+
+
+@pytest.fixture(autouse=True)
+def _slow_blocker_route(request, monkeypatch):
+    if request.node.name.split("[")[0] in SLOW_BLOCKER:
+        monkeypatch.setenv("MFX_FUSED", "0")
