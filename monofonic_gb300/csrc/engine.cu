@@ -437,7 +437,7 @@ static Layout plan_layout(const mfx_job_desc *d, size_t work_bytes, bool group_a
     L.status = align_up(sizeof(int));
   }
   if (fx_supported(d))
-    L.fx = align_up(size_t(M) * sizeof(longlong2)) + align_up(size_t(N) * sizeof(longlong2)) +
+    L.fx = align_up(fx::twiddle_bytes(M)) + align_up(fx::twiddle_bytes(N)) +
            align_up(2 * size_t(N) * 8) + align_up(fx::rinv_len(N) * 8);
   const size_t np = size_t(ns) * N * N * N;
   L.part_bytes = 0;
@@ -2027,16 +2027,16 @@ static int create_job(mfx_engine *eng, const mfx_job_desc *d, mfx_job **out, int
   if (j->fx) {
     char *f = p;
     j->fx_twm = reinterpret_cast<longlong2 *>(f);
-    f += align_up(size_t(j->M) * sizeof(longlong2));
+    f += align_up(fx::twiddle_bytes(j->M));
     j->fx_twn = reinterpret_cast<longlong2 *>(f);
-    f += align_up(size_t(j->N) * sizeof(longlong2));
+    f += align_up(fx::twiddle_bytes(j->N));
     j->fx_mode = reinterpret_cast<double *>(f);
     f += align_up(2 * size_t(j->N) * 8);
     j->fx_rinv = reinterpret_cast<double *>(f);
     cudaError_t fe = fx::prepare_device(eng->device);
     for (const int len : {j->M, j->N})
       if (fe == cudaSuccess && (len == j->N || d->lpt_order >= 2))
-        fe = cudaMemcpyAsync(len == j->M ? j->fx_twm : j->fx_twn, fx::twiddles(len), size_t(len) * sizeof(longlong2),
+        fe = cudaMemcpyAsync(len == j->M ? j->fx_twm : j->fx_twn, fx::twiddles(len), fx::twiddle_bytes(len),
                              cudaMemcpyHostToDevice, j->stream);
     if (fe == cudaSuccess) fe = fx::fill_tables(j->N, j->fx_mode, j->fx_rinv, j->stream);
     if (fe != cudaSuccess) return fail(set_error(MFX_ECUDA, "fixed-point transform set-up: %s", cudaGetErrorString(fe)));

@@ -119,10 +119,19 @@ bool fx_plan(int L, FxKind kind, FxPlan *p) {
   return false;
 }
 
-void fx_twiddles(int L, longlong2 *out) {
+// (cos, -sin)(2 pi t / L) 2^61, t < L, then the three constants of the products
+// with them, split into signed halves: c and s + c, then s - c (fx64_len.cuh Tw3)
+static void make_twiddles(int L, longlong2 *out) {
+  int4 *cp = reinterpret_cast<int4 *>(out + L);
+  int2 *m = reinterpret_cast<int2 *>(cp + L);
+  auto lo = [](long long w) { return int(w); };
+  auto hi = [](long long w) { return int(w >> 32) + int(unsigned(int(w)) >> 31); };
   for (int t = 0; t < L; ++t) {
     const CS w = q62_turn(t, L);
-    out[t] = make_longlong2((long long)((w.c + 1) >> 1), (long long)((-w.s + 1) >> 1));
+    const long long c = (long long)((w.c + 1) >> 1), s = (long long)((-w.s + 1) >> 1);
+    out[t] = make_longlong2(c, s);
+    cp[t] = make_int4(hi(c), lo(c), hi(s + c), lo(s + c));
+    m[t] = make_int2(hi(s - c), lo(s - c));
   }
 }
 
@@ -133,8 +142,8 @@ const longlong2 *twiddles(int L) {
   std::lock_guard<std::mutex> lk(mu);
   std::vector<longlong2> &t = tables[L];
   if (t.empty()) {
-    t.resize(L);
-    fx_twiddles(L, t.data());
+    t.resize(twiddle_bytes(L) / sizeof(longlong2));
+    make_twiddles(L, t.data());
   }
   return t.data();
 }
@@ -476,23 +485,64 @@ __global__ void __launch_bounds__(384) k_fx_r2c(const __grid_constant__ RArgs a)
 // ---------------------------------------------------------------------------
 // launches
 // ---------------------------------------------------------------------------
-// the instance of a length, if it has one
+// the instance of a length, if it has one: as padded length, as grid length
 using LenFn = cudaError_t (*)(FxOp, const void *, dim3, cudaStream_t);
 struct LenEntry {
   int L;
+  bool padded, grid;
   LenFn fn;
-  int steps, R[3];
+  int steps, R[3];  // in the order of a forward transform
 };
-template <int L> constexpr LenEntry entry() {
-  return {L, launch_len<L>, Len<L>::steps, {Len<L>::R(0), Len<L>::R(1), Len<L>::R(2)}};
+extern template struct Launch<16, false, true>;
+extern template struct Launch<24, true, true>;
+extern template struct Launch<32, false, true>;
+extern template struct Launch<48, true, true>;
+extern template struct Launch<64, false, true>;
+extern template struct Launch<72, true, false>;
+extern template struct Launch<96, true, true>;
+extern template struct Launch<128, false, true>;
+extern template struct Launch<144, true, false>;
+extern template struct Launch<192, true, true>;
+extern template struct Launch<256, false, true>;
+extern template struct Launch<288, true, false>;
+extern template struct Launch<384, true, true>;
+extern template struct Launch<512, false, true>;
+extern template struct Launch<576, true, false>;
+extern template struct Launch<768, true, true>;
+extern template struct Launch<1152, true, false>;
+template <int L, bool PADDED, bool GRID> static LenEntry entry() {
+  return {L, PADDED, GRID, Launch<L, PADDED, GRID>::run, Len<L>::steps, {Len<L>::R(0), Len<L>::R(1), Len<L>::R(2)}};
 }
-static const LenEntry kLens[] = {entry<16>(),  entry<24>(),  entry<32>(),  entry<48>(),  entry<64>(),  entry<72>(),
-                                 entry<96>(),  entry<128>(), entry<144>(), entry<192>(), entry<256>(), entry<288>(),
-                                 entry<384>(), entry<512>(), entry<576>(), entry<768>(), entry<1152>()};
+static const LenEntry kLens[] = {entry<16, false, true>(),
+                                 entry<24, true, true>(),
+                                 entry<32, false, true>(),
+                                 entry<48, true, true>(),
+                                 entry<64, false, true>(),
+                                 entry<72, true, false>(),
+                                 entry<96, true, true>(),
+                                 entry<128, false, true>(),
+                                 entry<144, true, false>(),
+                                 entry<192, true, true>(),
+                                 entry<256, false, true>(),
+                                 entry<288, true, false>(),
+                                 entry<384, true, true>(),
+                                 entry<512, false, true>(),
+                                 entry<576, true, false>(),
+                                 entry<768, true, true>(),
+                                 entry<1152, true, false>()};
 static const LenEntry *find_len(int L) {
   for (const LenEntry &e : kLens)
     if (e.L == L) return &e;
   return nullptr;
+}
+// B of an instance; an inverse transform takes the radices backwards
+static int len_bits(const LenEntry &l, FxKind kind, bool forward, bool inverse) {
+  int rev[3];
+  for (int q = 0; q < l.steps; ++q) rev[q] = l.R[l.steps - 1 - q];
+  int b = 60;
+  if (forward) b = std::min(b, fx_bits(l.R, l.steps, kind));
+  if (inverse) b = std::min(b, fx_bits(rev, l.steps, kind));
+  return b;
 }
 
 static __global__ void k_fx_tables(int n, double *mode, double *rinv, int len) {
@@ -531,9 +581,15 @@ cudaError_t prepare_device(int dev) {
 
 cudaError_t run_strided(const Strided &s, cudaStream_t st) {
   if (const LenEntry *l = find_len(s.L)) {
-    const LArgs a{s.tw, fx_bits(l->R, l->steps, FX_STRIDED), s};
-    return l->fn(s.truncate ? FX_OP_TRUNCATE : FX_OP_STRIDED, &a,
-                 dim3(unsigned(s.outer * ((s.kc + 7) / 8)), unsigned(s.groups)), st);
+    const bool p = l->padded && 3 * s.n == 2 * s.L;
+    const bool single = s.groups == s.ops;
+    FxOp op = FX_OP_PREPARE;
+    if (s.inverse && !s.cut_out && !s.truncate) op = s.pad_in ? (p ? FX_OP_INV_PAD : op) : (l->grid ? FX_OP_INV : op);
+    else if (!s.inverse && !s.pad_in && single) op = !p ? op : (s.truncate ? FX_OP_TRUNC : (s.cut_out ? FX_OP_CUT : op));
+    if (op != FX_OP_PREPARE) {
+      const LArgs a{s.tw, len_bits(*l, FX_STRIDED, !s.inverse, s.inverse || s.truncate), s};
+      return l->fn(op, &a, dim3(unsigned(s.outer * ((s.kc + 7) / 8)), unsigned(s.groups)), st);
+    }
   }
   SArgs a;
   if (!fx_plan(s.L, FX_STRIDED, &a.c.p)) return cudaErrorInvalidValue;
@@ -546,8 +602,13 @@ cudaError_t run_strided(const Strided &s, cudaStream_t st) {
 
 static cudaError_t run_rows(const Rows &r, FxKind kind, cudaStream_t st) {
   if (const LenEntry *l = find_len(r.L)) {
-    const LRows a{r.tw, fx_bits(l->R, l->steps, kind), r};
-    return l->fn(kind == FX_C2R ? FX_OP_C2R : FX_OP_R2C, &a, dim3(unsigned((r.rows + 15) / 16), unsigned(r.count)), st);
+    FxOp op = FX_OP_PREPARE;
+    if (kind == FX_C2R) op = l->padded && r.kc <= r.L / 3 + 1 ? FX_OP_C2R_PAD : (l->grid ? FX_OP_C2R : op);
+    else if (l->padded && r.kc <= r.L / 3) op = FX_OP_R2C;
+    if (op != FX_OP_PREPARE) {
+      const LRows a{r.tw, len_bits(*l, kind, kind == FX_R2C, kind == FX_C2R), r};
+      return l->fn(op, &a, dim3(unsigned((r.rows + 15) / 16), unsigned(r.count)), st);
+    }
   }
   RArgs a;
   if (!fx_plan(r.L, kind, &a.c.p)) return cudaErrorInvalidValue;

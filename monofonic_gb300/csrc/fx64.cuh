@@ -352,7 +352,5 @@ inline bool fx_supported(int L) {
   FxPlan p;
   return L >= 8 && L % 2 == 0 && fx_plan(L, FX_STRIDED, &p) && fx_plan(L, FX_C2R, &p) && fx_plan(L, FX_R2C, &p);
 }
-// (cos, -sin)(2 pi t / L) 2^61, t < L
-void fx_twiddles(int L, longlong2 *out);
 
 }  // namespace fx

@@ -9,9 +9,10 @@ namespace fx {
 
 // a length the transforms are built for: even, no prime factor above 7
 bool length_supported(int L);
-// twiddle table of a length: L entries (host memory, kept for the process:
-// a few KB for each length that was asked for)
+// twiddle tables of a length (host memory, kept for the process: some KB for
+// each length that was asked for)
 const longlong2 *twiddles(int L);
+inline size_t twiddle_bytes(int L) { return (size_t(L) * 40 + 15) / 16 * 16; }
 // device tables of a grid: mode[2][n] (Strided::mode) and rinv[q] = 1 / q,
 // q = 1 .. 3 (n/2)^2 (rinv[0] = 0)
 cudaError_t fill_tables(int n, double *mode, double *rinv, cudaStream_t st);

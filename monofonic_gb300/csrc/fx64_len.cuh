@@ -1,8 +1,22 @@
-// The fixed-point transforms (fx64.cuh) compiled for one length: the kernels
-// of fx64.cu with radices, index arithmetic and thread counts folded to
-// constants, the first step of an x or y pass reading HBM straight into
-// registers and the last one writing from them (one shared-memory exchange for
-// two steps).  Lengths without an instance take the run-time kernels.
+// The fixed-point transforms (fx64.cuh) compiled for one length: radices, index
+// arithmetic and thread counts are constants, the first step of an x or y pass
+// reads HBM straight into registers and the last one writes from them (one
+// shared-memory exchange for two steps).  Lengths without an instance take the
+// run-time kernels of fx64.cu.
+//
+// What bounds them: integer instructions (the ALU pipe was 63% busy in the z
+// passes, issue 56%, HBM 26%, before the zero third was skipped), so what they
+// save is instructions.
+//  * A padded length L = 3N/2 is split so that the step at its N-grid side (the
+//    first of an inverse transform, the last of a forward one) has a radix
+//    divisible by three: inputs r of R / 3 < r < 2R / 3 of that step are the
+//    padding, for every butterfly, and neither loaded, converted, added nor
+//    stored.
+//  * In convolve3's truncation the forward transform's last step and the
+//    inverse one's first step have the same radix: the butterflies' outputs
+//    are the next ones' inputs and stay in registers.
+//  * Twiddles are read as the three constants of the complex product, split
+//    for the 32-bit multiplications.
 #pragma once
 #include "fx64.cuh"
 #include "fx64.h"
@@ -12,66 +26,109 @@ namespace fx {
 __device__ __forceinline__ int dbl_exponent(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
 __device__ __forceinline__ double nan_of() { return __longlong_as_double(0x7ff8000000000000LL); }
 
-// radices of a length (the smallest, whose butterflies carry no twiddles, first)
-// and threads per CTA of eight pencils
+// radices of a length in the order of a forward transform (an inverse one takes
+// them backwards), threads per CTA of eight pencils, CTAs an SM is to hold
 template <int L> struct Len;
-#define FX_LEN(L_, STEPS_, A_, B_, C_, T_)                                    \
+#define FX_LEN(L_, STEPS_, A_, B_, C_, T_, CTAS_, ZCTAS_)                     \
   template <> struct Len<L_> {                                               \
-    static constexpr int steps = STEPS_, T = T_;                              \
+    static constexpr int steps = STEPS_, T = T_, ctas = CTAS_, zctas = ZCTAS_; \
     static FX_HD constexpr int R(int q) { return q == 0 ? A_ : (q == 1 ? B_ : C_); } \
   };
-FX_LEN(16, 2, 4, 4, 1, 32)
-FX_LEN(24, 2, 4, 6, 1, 64)
-FX_LEN(32, 2, 4, 8, 1, 64)
-FX_LEN(48, 2, 6, 8, 1, 64)
-FX_LEN(64, 2, 8, 8, 1, 64)
-FX_LEN(72, 2, 8, 9, 1, 96)
-FX_LEN(96, 2, 8, 12, 1, 96)
-FX_LEN(128, 2, 8, 16, 1, 128)
-FX_LEN(144, 2, 12, 12, 1, 96)
-FX_LEN(192, 2, 12, 16, 1, 128)
-FX_LEN(256, 2, 16, 16, 1, 128)
-FX_LEN(288, 2, 16, 18, 1, 160)
-FX_LEN(384, 2, 16, 24, 1, 192)
-FX_LEN(512, 3, 8, 8, 8, 256)
-FX_LEN(576, 2, 24, 24, 1, 192)
-FX_LEN(768, 3, 8, 8, 12, 256)
-FX_LEN(1152, 3, 8, 12, 12, 384)
+FX_LEN(16, 2, 4, 4, 1, 32, 12, 16)
+FX_LEN(24, 2, 4, 6, 1, 64, 8, 12)
+FX_LEN(32, 2, 4, 8, 1, 64, 8, 12)
+FX_LEN(48, 2, 8, 6, 1, 64, 8, 12)
+FX_LEN(64, 2, 8, 8, 1, 64, 8, 12)
+FX_LEN(72, 2, 8, 9, 1, 96, 5, 8)
+FX_LEN(96, 2, 8, 12, 1, 96, 5, 8)
+FX_LEN(128, 2, 8, 16, 1, 128, 4, 5)
+FX_LEN(144, 2, 12, 12, 1, 96, 5, 7)
+FX_LEN(192, 2, 16, 12, 1, 128, 4, 5)
+FX_LEN(256, 2, 16, 16, 1, 128, 4, 5)
+FX_LEN(288, 2, 16, 18, 1, 160, 3, 4)
+FX_LEN(384, 2, 16, 24, 1, 192, 2, 3)
+FX_LEN(512, 3, 8, 8, 8, 256, 2, 2)
+FX_LEN(576, 2, 24, 24, 1, 192, 2, 3)
+FX_LEN(768, 3, 8, 8, 12, 256, 2, 2)
+FX_LEN(1152, 3, 8, 12, 12, 384, 1, 1)
 #undef FX_LEN
 
-// resident CTAs that the register file is shared by at `regs` registers a thread
-#ifndef FX_REG_S
-#define FX_REG_S 168
-#endif
-#ifndef FX_REG_Z
-#define FX_REG_Z 112
-#endif
-constexpr int min_ctas(int T, int regs) { return 65536 / (T * regs) > 0 ? 65536 / (T * regs) : 1; }
+// the three constants of a twiddle product (fx64.cuh twiddle8), each split into
+// signed 32-bit halves
+struct Tw3 {
+  const int4 *cp;  // c: hi, lo; s + c: hi, lo
+  const int2 *m;   // s - c: hi, lo
+};
+__device__ __forceinline__ Tw3 tw3_of(const longlong2 *table, int L) {
+  const int4 *cp = reinterpret_cast<const int4 *>(table + L);
+  return {cp, reinterpret_cast<const int2 *>(cp + L)};
+}
+__device__ __forceinline__ I2 twiddle8(I2 v, const Tw3 &t, int at) {
+  const int4 cp = __ldg(&t.cp[at]);
+  const int2 m = __ldg(&t.m[at]);
+  const long long k = mulq(v.x + v.y, cp.x, cp.y);
+  return {k - mulq(v.y, cp.z, cp.w), k + mulq(v.x, m.x, m.y)};
+}
 
-template <int L> struct Fft {
+// conversion of a pencil: largest exponent em -> right shift of to_fixed_p.
+// A pencil whose values all lie below 2^-959 counts as zero.
+__device__ __forceinline__ int shift_of(int em, int B) { return em < 64 ? 8192 : em + 63 - B; }
+__device__ __forceinline__ long long to_fixed_p(long long b, int sh) {
+  const int d = min(sh - (int(b >> 52) & 0x7ff), 63);
+  const long long m = (long long)(((unsigned long long)((b & 0xfffffffffffffLL) | 0x10000000000000LL) << 10) >> d);
+  const long long sg = b >> 63;
+  return (m ^ sg) - sg;
+}
+// back: values times 2^S; where the exponents leave the range of a double, or
+// the input was not finite, every value of the pencil is alt (high word)
+struct OutScale {
+  int k;     // high word of 2^(S + 62), minus the implicit bit
+  int alt;
+  bool use_alt;
+};
+__device__ __forceinline__ OutScale out_scale(int em, int S) {
+  const bool high = em == 2047 || S + 1086 >= 2047;
+  return {(S + 1085) << 20, high ? 0x7ff80000 : 0, high || S + 1086 - 63 <= 0};
+}
+__device__ __forceinline__ double to_double_p(long long v, const OutScale &o) {
+  const long long sg = v >> 63;
+  const unsigned long long a = (unsigned long long)((v ^ sg) - sg);
+  const int lz = __clzll((long long)a);
+  const unsigned long long q = ((a << ((lz - 1) & 63)) + 0x200) >> 10;
+  int hi = int(q >> 32) + o.k - (lz << 20);
+  hi = a == 0 ? 0 : hi;
+  hi |= int(sg >> 32) & 0x80000000;
+  hi = o.use_alt ? o.alt : hi;
+  return __hiloint2double(hi, int(q));
+}
+
+// REV: the radices backwards
+template <int L, bool REV> struct Fft {
   using D = Len<L>;
-  static constexpr int P = 8, lgP = 3, T = D::T, steps = D::steps, items_max = P * L;
-  static FX_HD constexpr int NS(int q) { return q == 0 ? 1 : NS(q - 1) * D::R(q - 1); }
+  static constexpr int P = 8, lgP = 3, T = D::T, steps = D::steps, W = T / 32;
+  static FX_HD constexpr int R(int q) { return D::R(REV ? steps - 1 - q : q); }
+  static FX_HD constexpr int NS(int q) { return q == 0 ? 1 : NS(q - 1) * R(q - 1); }
   // butterflies of step q a thread holds
-  static FX_HD constexpr int MU(int q) { return (P * (L / D::R(q)) + T - 1) / T; }
-  static constexpr int smem = L * P * 16 + P * 8;
+  static FX_HD constexpr int MU(int q) { return (P * (L / R(q)) + T - 1) / T; }
+  static constexpr int last = D::steps - 1;
+  // pencils, two sets of per-warp maxima
+  static constexpr int smem = L * P * 16 + 2 * W * 8 * 4;
 
   static __device__ __forceinline__ int slot(int e, int pen) { return (e << lgP) + (pen ^ (e & (P - 1))); }
 
-  // registers of one step
   template <int Q> struct Regs {
-    I2 v[MU(Q)][D::R(Q)];
+    I2 v[MU(Q)][R(Q)];
   };
   template <int Q> static __device__ __forceinline__ bool live(int m) {
-    constexpr int items = P * (L / D::R(Q));
+    constexpr int items = P * (L / R(Q));
     return items % T == 0 || int(threadIdx.x) + m * T < items;
   }
   template <int Q> static __device__ __forceinline__ int jof(int m) { return (int(threadIdx.x) + m * T) >> lgP; }
-  // element index of input r / output r of butterfly j
-  template <int Q> static __device__ __forceinline__ int in_of(int j, int r) { return j + r * (L / D::R(Q)); }
+  // element of input r / output r of butterfly j
+  template <int Q> static __device__ __forceinline__ int in_of(int j, int r) { return j + r * (L / R(Q)); }
   template <int Q> static __device__ __forceinline__ int out_of(int j, int r) {
-    constexpr int ns = NS(Q), R = D::R(Q);
-    return (j / ns) * (ns * R) + j % ns + r * ns;
+    constexpr int ns = NS(Q);
+    return (j / ns) * (ns * R(Q)) + j % ns + r * ns;
   }
   template <int Q> static __device__ __forceinline__ void load(Regs<Q> &g, const longlong2 *s, int pen) {
 #pragma unroll
@@ -79,53 +136,73 @@ template <int L> struct Fft {
       if (live<Q>(m)) {
         const int j = jof<Q>(m);
 #pragma unroll
-        for (int r = 0; r < D::R(Q); ++r) {
+        for (int r = 0; r < R(Q); ++r) {
           const longlong2 w = s[slot(in_of<Q>(j, r), pen)];
           g.v[m][r] = {w.x, w.y};
         }
       }
   }
-  template <int Q> static __device__ __forceinline__ void store(const Regs<Q> &g, longlong2 *s, int pen) {
+  // FROM, TO: outputs r of FROM < r < TO (both exclusive) are left out
+  template <int Q, int FROM = 0, int TO = 0>
+  static __device__ __forceinline__ void store(const Regs<Q> &g, longlong2 *s, int pen) {
 #pragma unroll
     for (int m = 0; m < MU(Q); ++m)
       if (live<Q>(m)) {
         const int j = jof<Q>(m);
 #pragma unroll
-        for (int r = 0; r < D::R(Q); ++r) s[slot(out_of<Q>(j, r), pen)] = make_longlong2(g.v[m][r].x, g.v[m][r].y);
+        for (int r = 0; r < R(Q); ++r)
+          if (!(r > FROM && r < TO)) s[slot(out_of<Q>(j, r), pen)] = make_longlong2(g.v[m][r].x, g.v[m][r].y);
       }
   }
-  template <int Q> static __device__ __forceinline__ void butterfly(Regs<Q> &g, const longlong2 *tw) {
-    constexpr int R = D::R(Q), ns = NS(Q);
+  template <int Q> static __device__ __forceinline__ void butterfly(Regs<Q> &g, const Tw3 &tw) {
+    constexpr int ns = NS(Q);
 #pragma unroll
     for (int m = 0; m < MU(Q); ++m)
       if (live<Q>(m)) {
         if constexpr (Q > 0) {
-          const longlong2 *w = tw;
-          const int inc = (jof<Q>(m) % ns) * (L / (ns * R));
+          const int inc = (jof<Q>(m) % ns) * (L / (ns * R(Q)));
           g.v[m][0] = eighth(g.v[m][0]);
 #pragma unroll
-          for (int r = 1; r < R; ++r) g.v[m][r] = twiddle8(g.v[m][r], __ldg(&w[r * inc]));
+          for (int r = 1; r < R(Q); ++r) g.v[m][r] = twiddle8(g.v[m][r], tw, r * inc);
         }
-        Dft<R>::run(g.v[m]);
+        Dft<R(Q)>::run(g.v[m]);
       }
   }
-  // steps Q0 .. last, the last one's outputs left in registers
-  template <int Q0, class F> static __device__ __forceinline__ void rest(longlong2 *s, int pen, const longlong2 *tw,
-                                                                        F &&out) {
-    Regs<Q0> g;
-    load<Q0>(g, s, pen);
-    butterfly<Q0>(g, tw);
-    if constexpr (Q0 + 1 < steps) {
+  // steps Q .. last, the last one's outputs left to `out` in registers
+  template <int Q, class F> static __device__ __forceinline__ void rest(longlong2 *s, int pen, const Tw3 &tw, F &&out) {
+    Regs<Q> g;
+    load<Q>(g, s, pen);
+    butterfly<Q>(g, tw);
+    if constexpr (Q + 1 < steps) {
       __syncthreads();
-      store<Q0>(g, s, pen);
+      store<Q>(g, s, pen);
       __syncthreads();
-      rest<Q0 + 1>(s, pen, tw, out);
+      rest<Q + 1>(s, pen, tw, out);
     } else {
       out(g);
     }
   }
-  static constexpr int last = D::steps - 1;
+  // largest value over the CTA per pencil (lanes of equal low three bits)
+  static __device__ __forceinline__ int pencil_max(int v, int *wm) {
+    v = max(v, __shfl_xor_sync(0xffffffffu, v, 8));
+    v = max(v, __shfl_xor_sync(0xffffffffu, v, 16));
+    const int t = threadIdx.x;
+    if ((t & 31) < 8) wm[(t >> 5) * 8 + (t & 7)] = v;
+    __syncthreads();
+    v = wm[t & 7];
+#pragma unroll
+    for (int w = 1; w < W; ++w) v = max(v, wm[w * 8 + (t & 7)]);
+    return v;
+  }
 };
+
+// Where output or input r of the N-grid-side step of a padded length lies:
+// rows below N/2, the Nyquist row (butterfly 0 only), the padding, the first
+// row above it (not for butterfly 0, which is the padding's last), rows above
+enum Zone { Z_LOW, Z_NYQ, Z_PAD, Z_EDGE, Z_HIGH };
+template <int R> FX_HD constexpr Zone zone(int r) {
+  return r < R / 3 ? Z_LOW : (r == R / 3 ? Z_NYQ : (r < 2 * R / 3 ? Z_PAD : (r == 2 * R / 3 ? Z_EDGE : Z_HIGH)));
+}
 
 struct LArgs {
   const longlong2 *tw;
@@ -138,192 +215,309 @@ struct LRows {
   Rows r;
 };
 
-template <int L, bool TRUNC> __global__ void __launch_bounds__(Len<L>::T, min_ctas(Len<L>::T, FX_REG_S)) k_fx_strided_l(const __grid_constant__ LArgs a) {
-  using F = Fft<L>;
+// high word without the sign: its maximum has the largest exponent
+__device__ __forceinline__ int mag(long long b) { return int(b >> 32) & 0x7fffffff; }
+
+// inverse transform along x or y; PAD: N rows in, placed at the padded positions
+template <int L, bool PAD>
+__global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_inv(const __grid_constant__ LArgs a) {
+  using F = Fft<L, true>;
   extern __shared__ __align__(16) longlong2 sm[];
   const Strided &d = a.s;
+  constexpr int R0 = F::R(0), nb = L / R0, nh = L / 3, n = 2 * nh;
   const int t = threadIdx.x, pen = t & 7;
-  int *emax = reinterpret_cast<int *>(sm + L * F::P);
+  int *wm = reinterpret_cast<int *>(sm + L * 8);
+  const Tw3 tw = tw3_of(a.tw, L);
   const int kblocks = (d.kc + 7) >> 3;
-  const int o = blockIdx.x / kblocks, kz0 = (blockIdx.x - o * kblocks) << 3, kz = kz0 + pen;
+  const int o = blockIdx.x / kblocks, kz = ((blockIdx.x - o * kblocks) << 3) + pen;
   const bool lv = kz < d.kc;
-  const int n = d.n, nh = n >> 1;
   for (int op = d.first[blockIdx.y]; op < d.first[blockIdx.y + 1]; ++op) {
-    if (t < 8) emax[t] = 0;
     const double2 *src = d.src[op] + (long long)o * d.in_outer + kz;
-    const int pr = d.pr[op], pk = d.pk[op];
     typename F::template Regs<0> g;
-    int em = 0;
 #pragma unroll
     for (int m = 0; m < F::MU(0); ++m)
       if (F::template live<0>(m)) {
         const int j = F::template jof<0>(m);
+        const double2 *p = src + (long long)j * d.in_row;
+        const long long stride = (long long)nb * d.in_row, back = PAD ? (long long)nh * d.in_row : 0;
 #pragma unroll
-        for (int r = 0; r < F::D::R(0); ++r) {
-          const int l = F::template in_of<0>(j, r);
-          const int i = !d.pad_in ? l : (l <= nh ? l : (l > n ? l - nh : -1));
-          double2 v = make_double2(0.0, 0.0);
-          if (lv && i >= 0) v = src[(long long)i * d.in_row];
-          g.v[m][r] = {__double_as_longlong(v.x), __double_as_longlong(v.y)};
+        for (int r = 0; r < R0; ++r) {
+          const Zone z = PAD ? zone<R0>(r) : Z_LOW;
+          g.v[m][r] = {0, 0};
+          if (z == Z_PAD) continue;
+          if (lv && (z == Z_NYQ ? j == 0 : (z == Z_EDGE ? j > 0 : true))) {
+            const double2 v = *(p + r * stride - (z >= Z_EDGE ? back : 0));
+            g.v[m][r] = {__double_as_longlong(v.x), __double_as_longlong(v.y)};
+          }
         }
       }
-    if ((pr | pk) != 0) {
-      const double kf = pk == 0 ? 1.0 : (kz == nh ? 0.0 : (pk == 1 ? double(kz) : double(kz) * double(kz)));
+    if (PAD && (d.pr[op] | d.pk[op]) != 0) {
+      const int pr = d.pr[op], pk = d.pk[op];
+      const double kk = kz == nh ? 0.0 : double(kz), kf = pk == 2 ? kk * kk : kk;
+      const double *mode = d.mode + (pr == 2 ? n : 0);
 #pragma unroll
       for (int m = 0; m < F::MU(0); ++m)
         if (F::template live<0>(m)) {
           const int j = F::template jof<0>(m);
 #pragma unroll
-          for (int r = 0; r < F::D::R(0); ++r) {
-            const int l = F::template in_of<0>(j, r);
-            const int i = !d.pad_in ? l : (l <= nh ? l : (l > n ? l - nh : -1));
-            if (i >= 0) {
-              const double f = (pr ? __ldg(&d.mode[(pr - 1) * n + i]) : 1.0) * kf;
-              g.v[m][r].x = __double_as_longlong(__longlong_as_double(g.v[m][r].x) * f);
-              g.v[m][r].y = __double_as_longlong(__longlong_as_double(g.v[m][r].y) * f);
-            }
+          for (int r = 0; r < R0; ++r) {
+            const Zone z = zone<R0>(r);
+            if (z == Z_PAD) continue;
+            // padded positions of other butterflies hold zeros: any factor
+            const int i = z == Z_NYQ ? nh : j + r * nb - (z >= Z_EDGE ? nh : 0);
+            double f = pr ? __ldg(&mode[z == Z_EDGE && j == 0 ? 0 : i]) : kf;
+            if (pr && pk) f *= kf;
+            g.v[m][r].x = __double_as_longlong(__longlong_as_double(g.v[m][r].x) * f);
+            g.v[m][r].y = __double_as_longlong(__longlong_as_double(g.v[m][r].y) * f);
           }
         }
     }
+    int em = 0;
 #pragma unroll
     for (int m = 0; m < F::MU(0); ++m)
       if (F::template live<0>(m)) {
 #pragma unroll
-        for (int r = 0; r < F::D::R(0); ++r)
-          em = max(em, max(dbl_exponent(__longlong_as_double(g.v[m][r].x)), dbl_exponent(__longlong_as_double(g.v[m][r].y))));
+        for (int r = 0; r < R0; ++r)
+          if (!PAD || zone<R0>(r) != Z_PAD) em = max(em, max(mag(g.v[m][r].x), mag(g.v[m][r].y)));
       }
-    em = max(em, __shfl_xor_sync(0xffffffffu, em, 8));
-    em = max(em, __shfl_xor_sync(0xffffffffu, em, 16));
-    __syncthreads();
-    if ((t & 31) < 8) atomicMax(&emax[pen], em);
-    __syncthreads();
-    em = emax[pen];
-    const bool bad = em == 2047;
-    int S = em - 1022 - a.B + 3 * (F::steps - 1);
-    const bool inv = d.inverse;
-    const int sh = em + 63 - a.B;
+    em = F::pencil_max(em, wm) >> 20;
+    const int sh = shift_of(em, a.B);
+    // inverse transform: real and imaginary part exchanged, here and at the end
 #pragma unroll
     for (int m = 0; m < F::MU(0); ++m)
       if (F::template live<0>(m)) {
 #pragma unroll
-        for (int r = 0; r < F::D::R(0); ++r) {
-          const double x = __longlong_as_double(g.v[m][r].x), y = __longlong_as_double(g.v[m][r].y);
-          g.v[m][r] = {to_fixed(inv ? y : x, sh), to_fixed(inv ? x : y, sh)};
-        }
+        for (int r = 0; r < R0; ++r)
+          if (!PAD || zone<R0>(r) != Z_PAD)
+            g.v[m][r] = {to_fixed_p(g.v[m][r].y, sh), to_fixed_p(g.v[m][r].x, sh)};
       }
-    F::template butterfly<0>(g, a.tw);
+    F::template butterfly<0>(g, tw);
     F::template store<0>(g, sm, pen);
     __syncthreads();
-    auto put = [&](auto &h) {
-      double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
-      const int so = o > nh ? o - n : o;
-      const bool swap = TRUNC || inv;
+    const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1));
+    double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
+    F::template rest<1>(sm, pen, tw, [&](auto &h) {
+      constexpr int Q = F::last;
 #pragma unroll
-      for (int m = 0; m < F::MU(F::last); ++m)
-        if (F::template live<F::last>(m)) {
-          const int j = F::template jof<F::last>(m);
+      for (int m = 0; m < F::MU(Q); ++m)
+        if (F::template live<Q>(m) && lv) {
+          double2 *p = dst + (long long)F::template jof<Q>(m) * d.out_row;
+          const long long stride = (long long)F::NS(Q) * d.out_row;
 #pragma unroll
-          for (int r = 0; r < F::D::R(F::last); ++r) {
-            const int l = F::template out_of<F::last>(j, r);
-            const int i = !d.cut_out ? l : (l <= nh ? l : (l > n ? l - nh : -1));
-            if (i >= 0 && lv) {
-              double2 v = make_double2(to_double(swap ? h.v[m][r].y : h.v[m][r].x, S),
-                                       to_double(swap ? h.v[m][r].x : h.v[m][r].y, S));
-              if (bad) v = make_double2(nan_of(), nan_of());
-              if (TRUNC) {
-                v.x *= d.fac;
-                v.y *= d.fac;
-              } else if (d.cut_out) {
-                if (i == nh || (d.inv_lap && (o == nh || (o | i | kz) == 0))) {
-                  v = make_double2(0.0, 0.0);
-                } else if (d.inv_lap) {
-                  const int si = i > nh ? i - n : i;
-                  const double f = -d.fac * __ldg(&d.rinv[so * so + si * si + kz * kz]);
-                  v.x *= f;
-                  v.y *= f;
-                }
-              }
-              dst[(long long)i * d.out_row] = v;
-            }
-          }
+          for (int r = 0; r < F::R(Q); ++r)
+            p[r * stride] = make_double2(to_double_p(h.v[m][r].y, os), to_double_p(h.v[m][r].x, os));
         }
-    };
-    if constexpr (!TRUNC) {
-      F::template rest<1>(sm, pen, a.tw, put);
-    } else {
-      // forward transform, the N-grid modes kept, the largest brought back
-      // below 2^B, transformed back (inverse = exchange, forward, exchange)
-      if (t < 8) emax[t] = 0;
-      int bits = 0;
-      F::template rest<1>(sm, pen, a.tw, [&](auto &h) {
-#pragma unroll
-        for (int m = 0; m < F::MU(F::last); ++m)
-          if (F::template live<F::last>(m)) {
-            const int j = F::template jof<F::last>(m);
-#pragma unroll
-            for (int r = 0; r < F::D::R(F::last); ++r) {
-              const int l = F::template out_of<F::last>(j, r);
-              const bool keep = l < nh || l > n;
-              const I2 v = h.v[m][r];
-              h.v[m][r] = keep ? I2{v.y, v.x} : I2{0, 0};
-              if (keep) bits = max(bits, 64 - min(__clzll(v.x ^ (v.x >> 63)), __clzll(v.y ^ (v.y >> 63))));
-            }
-          }
-        bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, 8));
-        bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, 16));
-        __syncthreads();
-        if ((t & 31) < 8) atomicMax(&emax[pen], bits);
-        F::template store<F::last>(h, sm, pen);
-        __syncthreads();
-      });
-      const int down = emax[pen] - a.B;
-      const int dn = max(down, 0), up = max(-down, 0);
-      const long long half = dn ? 1LL << (dn - 1) : 0;
-      F::template load<0>(g, sm, pen);
-#pragma unroll
-      for (int m = 0; m < F::MU(0); ++m)
-        if (F::template live<0>(m)) {
-#pragma unroll
-          for (int r = 0; r < F::D::R(0); ++r)
-            g.v[m][r] = {((g.v[m][r].x + half) >> dn) << up, ((g.v[m][r].y + half) >> dn) << up};
-        }
-      S += down + 3 * (F::steps - 1);
-      F::template butterfly<0>(g, a.tw);
-      __syncthreads();
-      F::template store<0>(g, sm, pen);
-      __syncthreads();
-      F::template rest<1>(sm, pen, a.tw, put);
-    }
-    if (!TRUNC && d.inv_lap && kz0 + 8 >= d.kc) {
-      double2 *z = d.dst[op] + (long long)o * d.out_outer + d.kc;  // the kz Nyquist column
-      for (int i = t; i < n; i += F::T) z[(long long)i * d.out_row] = make_double2(0.0, 0.0);
-    }
-    __syncthreads();
+    });
+    if (op + 1 < d.first[blockIdx.y + 1]) __syncthreads();
   }
 }
 
-// spectra -> real rows (fx64.cu k_fx_c2r)
-template <int L> __global__ void __launch_bounds__(Len<L>::T, min_ctas(Len<L>::T, FX_REG_Z)) k_fx_c2r_l(const __grid_constant__ LRows a) {
-  using F = Fft<L>;
+// forward transform along x or y, the N-grid rows kept (the Nyquist row zero);
+// inv_lap: times -fac / k^2
+template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_cut(const __grid_constant__ LArgs a) {
+  using F = Fft<L, false>;
+  extern __shared__ __align__(16) longlong2 sm[];
+  const Strided &d = a.s;
+  constexpr int R0 = F::R(0), nb = L / R0, nh = L / 3, n = 2 * nh;
+  const int t = threadIdx.x, pen = t & 7;
+  int *wm = reinterpret_cast<int *>(sm + L * 8);
+  const Tw3 tw = tw3_of(a.tw, L);
+  const int kblocks = (d.kc + 7) >> 3;
+  const int o = blockIdx.x / kblocks, kz0 = (blockIdx.x - o * kblocks) << 3, kz = kz0 + pen;
+  const bool lv = kz < d.kc;
+  const int op = blockIdx.y;
+  const double2 *src = d.src[op] + (long long)o * d.in_outer + kz;
+  typename F::template Regs<0> g;
+#pragma unroll
+  for (int m = 0; m < F::MU(0); ++m)
+    if (F::template live<0>(m)) {
+      const double2 *p = src + (long long)F::template jof<0>(m) * d.in_row;
+      const long long stride = (long long)nb * d.in_row;
+#pragma unroll
+      for (int r = 0; r < R0; ++r) {
+        double2 v = make_double2(0.0, 0.0);
+        if (lv) v = p[r * stride];
+        g.v[m][r] = {__double_as_longlong(v.x), __double_as_longlong(v.y)};
+      }
+    }
+  int em = 0;
+#pragma unroll
+  for (int m = 0; m < F::MU(0); ++m)
+    if (F::template live<0>(m)) {
+#pragma unroll
+      for (int r = 0; r < R0; ++r) em = max(em, max(mag(g.v[m][r].x), mag(g.v[m][r].y)));
+    }
+  em = F::pencil_max(em, wm) >> 20;
+  const int sh = shift_of(em, a.B);
+#pragma unroll
+  for (int m = 0; m < F::MU(0); ++m)
+    if (F::template live<0>(m)) {
+#pragma unroll
+      for (int r = 0; r < R0; ++r) g.v[m][r] = {to_fixed_p(g.v[m][r].x, sh), to_fixed_p(g.v[m][r].y, sh)};
+    }
+  F::template butterfly<0>(g, tw);
+  F::template store<0>(g, sm, pen);
+  __syncthreads();
+  const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1));
+  double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
+  F::template rest<1>(sm, pen, tw, [&](auto &h) {
+    constexpr int Q = F::last, RL = F::R(Q);
+    const bool lap = d.inv_lap;
+    const int so = o > nh ? o - n : o, q0 = so * so + kz * kz;
+#pragma unroll
+    for (int m = 0; m < F::MU(Q); ++m)
+      if (F::template live<Q>(m) && lv) {
+        const int j = F::template jof<Q>(m);
+        double2 *p = dst + (long long)j * d.out_row;
+        const long long stride = (long long)F::NS(Q) * d.out_row, back = (long long)nh * d.out_row;
+#pragma unroll
+        for (int r = 0; r < RL; ++r) {
+          const Zone z = zone<RL>(r);
+          if (z == Z_PAD || (z == Z_NYQ && j != 0) || (z == Z_EDGE && j == 0)) continue;
+          double2 v = make_double2(0.0, 0.0);
+          if (z != Z_NYQ) {
+            v = make_double2(to_double_p(h.v[m][r].x, os), to_double_p(h.v[m][r].y, os));
+            if (lap) {
+              const int si = j + r * (L / RL) - (z >= Z_EDGE ? L : 0);  // signed mode index
+              const int q = q0 + si * si;
+              const double f = o == nh ? 0.0 : -d.fac * __ldg(&d.rinv[q]);  // rinv[0] = 0
+              v.x *= f;
+              v.y *= f;
+            }
+          }
+          *(p + r * stride - (z >= Z_EDGE ? back : 0)) = v;
+        }
+      }
+  });
+  if (d.inv_lap && kz0 + 8 >= d.kc) {
+    double2 *z = d.dst[op] + (long long)o * d.out_outer + d.kc;  // the kz Nyquist column
+    for (int i = t; i < n; i += F::T) z[(long long)i * d.out_row] = make_double2(0.0, 0.0);
+  }
+}
+
+// forward, the N-grid rows kept times fac, and back (in place)
+template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_trunc(const __grid_constant__ LArgs a) {
+  using F = Fft<L, false>;
+  using I = Fft<L, true>;
+  extern __shared__ __align__(16) longlong2 sm[];
+  const Strided &d = a.s;
+  constexpr int R0 = F::R(0), nb = L / R0, RL = F::R(F::last);
+  static_assert(RL == I::R(0), "the forward transform's last radix is the inverse one's first");
+  const int t = threadIdx.x, pen = t & 7;
+  int *wm = reinterpret_cast<int *>(sm + L * 8);
+  const Tw3 tw = tw3_of(a.tw, L);
+  const int kblocks = (d.kc + 7) >> 3;
+  const int o = blockIdx.x / kblocks, kz = ((blockIdx.x - o * kblocks) << 3) + pen;
+  const bool lv = kz < d.kc;
+  const int op = blockIdx.y;
+  typename I::template Regs<0> h;
+  int em, S;
+  {
+    const double2 *src = d.src[op] + (long long)o * d.in_outer + kz;
+    typename F::template Regs<0> g;
+#pragma unroll
+    for (int m = 0; m < F::MU(0); ++m)
+      if (F::template live<0>(m)) {
+        const double2 *p = src + (long long)F::template jof<0>(m) * d.in_row;
+        const long long stride = (long long)nb * d.in_row;
+#pragma unroll
+        for (int r = 0; r < R0; ++r) {
+          double2 v = make_double2(0.0, 0.0);
+          if (lv) v = p[r * stride];
+          g.v[m][r] = {__double_as_longlong(v.x), __double_as_longlong(v.y)};
+        }
+      }
+    em = 0;
+#pragma unroll
+    for (int m = 0; m < F::MU(0); ++m)
+      if (F::template live<0>(m)) {
+#pragma unroll
+        for (int r = 0; r < R0; ++r) em = max(em, max(mag(g.v[m][r].x), mag(g.v[m][r].y)));
+      }
+    em = F::pencil_max(em, wm) >> 20;
+    const int sh = shift_of(em, a.B);
+#pragma unroll
+    for (int m = 0; m < F::MU(0); ++m)
+      if (F::template live<0>(m)) {
+#pragma unroll
+        for (int r = 0; r < R0; ++r) g.v[m][r] = {to_fixed_p(g.v[m][r].x, sh), to_fixed_p(g.v[m][r].y, sh)};
+      }
+    F::template butterfly<0>(g, tw);
+    F::template store<0>(g, sm, pen);
+    __syncthreads();
+  }
+  // the modes outside the N-grid and on its Nyquist row fall away; real and
+  // imaginary part are exchanged for the inverse transform
+  int bits = 0;
+  F::template rest<1>(sm, pen, tw, [&](auto &g) {
+#pragma unroll
+    for (int m = 0; m < F::MU(F::last); ++m)
+      if (F::template live<F::last>(m)) {
+        const int j = F::template jof<F::last>(m);
+#pragma unroll
+        for (int r = 0; r < RL; ++r) {
+          const Zone z = zone<RL>(r);
+          I2 v = g.v[m][r];
+          if (z == Z_NYQ || z == Z_PAD || (z == Z_EDGE && j == 0)) v = {0, 0};
+          bits |= int((v.x ^ (v.x >> 63)) >> 32) | int((v.y ^ (v.y >> 63)) >> 32);
+          h.v[m][r] = {v.y, v.x};
+        }
+      }
+  });
+  // bring the largest back below 2^B.  Its high word decides: a pencil whose
+  // values all lie below 2^32 is far below the rounding of the first transform
+  bits = 32 - __clz(I::pencil_max(bits, wm + F::W * 8)) + 32;
+  const int down = bits - a.B, dn = max(down, 0), up = max(-down, 0);
+  const long long half = dn ? 1LL << (dn - 1) : 0;
+#pragma unroll
+  for (int m = 0; m < I::MU(0); ++m)
+    if (I::template live<0>(m)) {
+#pragma unroll
+      for (int r = 0; r < RL; ++r)
+        if (zone<RL>(r) != Z_NYQ && zone<RL>(r) != Z_PAD)
+          h.v[m][r] = {((h.v[m][r].x + half) >> dn) << up, ((h.v[m][r].y + half) >> dn) << up};
+    }
+  I::template butterfly<0>(h, tw);
+  I::template store<0>(h, sm, pen);
+  __syncthreads();
+  S = em - 1022 - a.B + down + 6 * (F::steps - 1);
+  const OutScale os = out_scale(em, S);
+  double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
+  I::template rest<1>(sm, pen, tw, [&](auto &g) {
+    constexpr int Q = I::last;
+#pragma unroll
+    for (int m = 0; m < I::MU(Q); ++m)
+      if (I::template live<Q>(m) && lv) {
+        double2 *p = dst + (long long)I::template jof<Q>(m) * d.out_row;
+        const long long stride = (long long)I::NS(Q) * d.out_row;
+#pragma unroll
+        for (int r = 0; r < I::R(Q); ++r)
+          p[r * stride] = make_double2(to_double_p(g.v[m][r].y, os) * d.fac, to_double_p(g.v[m][r].x, os) * d.fac);
+      }
+  });
+}
+
+// spectra -> real rows (fx64.cu k_fx_c2r); PAD: at most L/3 + 1 kz values
+template <int L, bool PAD>
+__global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_c2r_l(const __grid_constant__ LRows a) {
+  using F = Fft<L, true>;
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
-  constexpr int h = L / 2, W = F::T / 32;
+  constexpr int h = L / 2, kmax = PAD ? L / 3 + 1 : h, NL = (kmax + 31) / 32;
   const int t = threadIdx.x, lane = t & 31, pen = t & 7;
-  int *emax = reinterpret_cast<int *>(sm + L * F::P);
+  int *rmax = reinterpret_cast<int *>(sm + L * 8);  // per row
+  const Tw3 tw = tw3_of(a.tw, L);
   double *base = d.field[blockIdx.y];
   const long long row0 = (long long)blockIdx.x * 16;
-  const int kc = min(d.kc, h);
-  const bool nyq = d.kc > h;
-  if (t < 8) emax[t] = 0;
-  for (int e = t; e < (L - 2 * kc + 1) * 8; e += F::T) sm[F::slot(kc + (e >> 3), e & 7)] = make_longlong2(0, 0);
-  __syncthreads();
-  for (int q = t >> 5; q < 16; q += W) {
+  const int kc = min(d.kc, kmax);
+  const bool nyq = !PAD && d.kc > h;
+#pragma unroll 1
+  for (int q = t >> 5; q < 16; q += F::W) {
     const long long row = row0 + q;
     const bool lv = row < d.rows;
     const double2 *src = reinterpret_cast<const double2 *>(base + row * d.pitch);
     const int p = q >> 1, second = q & 1;
     int em = 0;
-    constexpr int NL = (h + 31) / 32;
     double2 v[NL];
 #pragma unroll
     for (int c = 0; c < NL; ++c) {
@@ -331,89 +525,110 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, min_ctas(Len<L>::T
       v[c] = make_double2(0.0, 0.0);
       if (lv && k < kc) v[c] = src[k];
     }
+    if (lane == 0) v[0].y = 0.0;  // only the real part of the k = 0 value is used
 #pragma unroll
     for (int c = 0; c < NL; ++c) {
       const int k = lane + 32 * c;
-      if (k >= kc) continue;
-      if (k == 0) {
-        em = max(em, dbl_exponent(v[c].x));
-        reinterpret_cast<double *>(&sm[F::slot(0, p)])[second] = v[c].x;
-      } else {
-        em = max(em, max(dbl_exponent(v[c].x), dbl_exponent(v[c].y)));
-        sm[F::slot(second ? L - k : k, p)] = make_longlong2(__double_as_longlong(v[c].x), __double_as_longlong(v[c].y));
-      }
+      if (k >= (PAD ? kmax : h)) continue;
+      const longlong2 b = make_longlong2(__double_as_longlong(v[c].x), __double_as_longlong(v[c].y));
+      em = max(em, max(mag(b.x), mag(b.y)));
+      if (k == 0) reinterpret_cast<long long *>(&sm[F::slot(0, p)])[second] = b.x;
+      else sm[F::slot(second ? L - k : k, p)] = b;
     }
-    if (nyq && lane == 0) {
-      const double x = lv ? src[h].x : 0.0;
-      em = max(em, dbl_exponent(x));
+    if (!PAD && lane == 0) {
+      // the Nyquist value (zero where the spectrum ends before it)
+      const double x = nyq && lv ? src[h].x : 0.0;
+      em = max(em, mag(__double_as_longlong(x)));
       reinterpret_cast<double *>(&sm[F::slot(h, p)])[second] = x;
     }
     em = int(__reduce_max_sync(0xffffffffu, unsigned(em)));
-    if (lane == 0) atomicMax(&emax[p], em);
+    if (lane == 0) rmax[q] = em;
   }
   __syncthreads();
+  const int em8 = max(rmax[2 * pen], rmax[2 * pen + 1]) >> 20;
   {
-    const int sh = emax[pen] + 63 - a.B;
-    for (int k = t >> 3; k < kc; k += F::T / 8) {
+    const int sh = shift_of(em8, a.B);
+    constexpr int kend = PAD ? kmax : h;
+    for (int k = t >> 3; k < kend; k += F::T / 8) {
       longlong2 &wa = sm[F::slot(k, pen)];
       const longlong2 va = wa;
-      const long long ax = to_fixed(__longlong_as_double(va.x), sh), ay = to_fixed(__longlong_as_double(va.y), sh);
+      const long long ax = to_fixed_p(va.x, sh), ay = to_fixed_p(va.y, sh);
       if (k == 0) {
         wa = make_longlong2(ay, ax);
         continue;
       }
       longlong2 &wb = sm[F::slot(L - k, pen)];
       const longlong2 vb = wb;
-      const long long bx = to_fixed(__longlong_as_double(vb.x), sh), by = to_fixed(__longlong_as_double(vb.y), sh);
+      const long long bx = to_fixed_p(vb.x, sh), by = to_fixed_p(vb.y, sh);
       wa = make_longlong2(ay + bx, ax - by);
       wb = make_longlong2(bx - ay, ax + by);
     }
-    if (nyq && t < 8) {
+    if (!PAD && t < 8) {
       longlong2 &w = sm[F::slot(h, t)];
       const longlong2 v = w;
-      w = make_longlong2(to_fixed(__longlong_as_double(v.y), sh), to_fixed(__longlong_as_double(v.x), sh));
+      w = make_longlong2(to_fixed_p(v.y, sh), to_fixed_p(v.x, sh));
     }
   }
   __syncthreads();
-  F::template rest<0>(sm, pen, a.tw, [&](auto &g) {
+  {
+    // the first step knows the padding (elements L/3 < e < 2L/3) to be zero
+    typename F::template Regs<0> g;
+    constexpr int R0 = F::R(0);
+#pragma unroll
+    for (int m = 0; m < F::MU(0); ++m)
+      if (F::template live<0>(m)) {
+        const int j = F::template jof<0>(m);
+#pragma unroll
+        for (int r = 0; r < R0; ++r) {
+          const Zone z = PAD ? zone<R0>(r) : Z_LOW;
+          g.v[m][r] = {0, 0};
+          if (z == Z_PAD || (z == Z_NYQ && j != 0)) continue;
+          const longlong2 w = sm[F::slot(F::template in_of<0>(j, r), pen)];
+          g.v[m][r] = {w.x, w.y};
+        }
+      }
+    F::template butterfly<0>(g, tw);
+    __syncthreads();
+    F::template store<0>(g, sm, pen);
+    __syncthreads();
+  }
+  F::template rest<1>(sm, pen, tw, [&](auto &g) {
     __syncthreads();
     F::template store<F::last>(g, sm, pen);
     __syncthreads();
   });
-  for (int q = t >> 5; q < 16; q += W) {
+#pragma unroll 1
+  for (int q = t >> 5; q < 16; q += F::W) {
     const long long row = row0 + q;
     if (row >= d.rows) break;
     double *dst = base + row * d.pitch;
     const int p = q >> 1, second = q & 1;
-    const int S = emax[p] - 1022 - a.B + 3 * (F::steps - 1);
-    const bool bad = emax[p] == 2047;
+    const int em = max(rmax[2 * p], rmax[2 * p + 1]) >> 20;
+    const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1));
 #pragma unroll 4
-    for (int e = lane; e < L; e += 32) {
-      const long long v = reinterpret_cast<const long long *>(&sm[F::slot(e, p)])[1 - second];
-      dst[e] = bad ? nan_of() : to_double(v, S);
-    }
+    for (int e = lane; e < L; e += 32)  // exchanged again: the first row is the imaginary part
+      dst[e] = to_double_p(reinterpret_cast<const long long *>(&sm[F::slot(e, p)])[1 - second], os);
   }
 }
 
-// real rows -> spectra (fx64.cu k_fx_r2c)
-template <int L> __global__ void __launch_bounds__(Len<L>::T, min_ctas(Len<L>::T, FX_REG_Z)) k_fx_r2c_l(const __grid_constant__ LRows a) {
-  using F = Fft<L>;
+// real rows -> spectra of kz < kc <= L/3 (fx64.cu k_fx_r2c)
+template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_r2c_l(const __grid_constant__ LRows a) {
+  using F = Fft<L, false>;
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
-  constexpr int W = F::T / 32;
+  constexpr int NL = (L + 31) / 32;
   const int t = threadIdx.x, lane = t & 31, pen = t & 7;
-  int *emax = reinterpret_cast<int *>(sm + L * F::P);
+  int *rmax = reinterpret_cast<int *>(sm + L * 8);
+  const Tw3 tw = tw3_of(a.tw, L);
   double *base = d.field[blockIdx.y];
   const long long row0 = (long long)blockIdx.x * 16;
-  if (t < 8) emax[t] = 0;
-  __syncthreads();
-  for (int q = t >> 5; q < 16; q += W) {
+#pragma unroll 1
+  for (int q = t >> 5; q < 16; q += F::W) {
     const long long row = row0 + q;
     const bool lv = row < d.rows;
     const double *src = base + row * d.pitch;
     const int p = q >> 1, second = q & 1;
     int em = 0;
-    constexpr int NL = (L + 31) / 32;
     double v[NL];
 #pragma unroll
     for (int c = 0; c < NL; ++c) {
@@ -425,71 +640,101 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, min_ctas(Len<L>::T
     for (int c = 0; c < NL; ++c) {
       const int e = lane + 32 * c;
       if (L % 32 == 0 || e < L) {
-        em = max(em, dbl_exponent(v[c]));
+        em = max(em, mag(__double_as_longlong(v[c])));
         reinterpret_cast<double *>(&sm[F::slot(e, p)])[second] = v[c];
       }
     }
     em = int(__reduce_max_sync(0xffffffffu, unsigned(em)));
-    if (lane == 0) atomicMax(&emax[p], em);
+    if (lane == 0) rmax[q] = em;
   }
   __syncthreads();
   {
-    const int sh = emax[pen] + 63 - a.B;
+    const int sh = shift_of(max(rmax[2 * pen], rmax[2 * pen + 1]) >> 20, a.B);
     typename F::template Regs<0> g;
     F::template load<0>(g, sm, pen);
 #pragma unroll
     for (int m = 0; m < F::MU(0); ++m)
       if (F::template live<0>(m)) {
 #pragma unroll
-        for (int r = 0; r < F::D::R(0); ++r)
-          g.v[m][r] = {to_fixed(__longlong_as_double(g.v[m][r].x), sh), to_fixed(__longlong_as_double(g.v[m][r].y), sh)};
+        for (int r = 0; r < F::R(0); ++r) g.v[m][r] = {to_fixed_p(g.v[m][r].x, sh), to_fixed_p(g.v[m][r].y, sh)};
       }
-    F::template butterfly<0>(g, a.tw);
+    F::template butterfly<0>(g, tw);
     __syncthreads();
     F::template store<0>(g, sm, pen);
     __syncthreads();
   }
-  F::template rest<1>(sm, pen, a.tw, [&](auto &g) {
+  F::template rest<1>(sm, pen, tw, [&](auto &g) {
+    constexpr int RL = F::R(F::last);
     __syncthreads();
-    F::template store<F::last>(g, sm, pen);
+    F::template store<F::last, RL / 3 - 1, 2 * RL / 3>(g, sm, pen);
     __syncthreads();
   });
   const int kc = d.kc;
-  for (int q = t >> 5; q < 16; q += W) {
+#pragma unroll 1
+  for (int q = t >> 5; q < 16; q += F::W) {
     const long long row = row0 + q;
     if (row >= d.rows) break;
     double2 *dst = reinterpret_cast<double2 *>(base + row * d.pitch);
     const int p = q >> 1, second = q & 1;
-    const int S = emax[p] - 1022 - a.B + 3 * (F::steps - 1) - 1;
-    const bool bad = emax[p] == 2047;
+    const int em = max(rmax[2 * p], rmax[2 * p + 1]) >> 20;
+    // the sums below are twice the spectra
+    const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1) - 1);
 #pragma unroll 2
     for (int k = lane; k < kc; k += 32) {
       const longlong2 u = sm[F::slot(k, p)], w = sm[F::slot(k ? L - k : 0, p)];
+      // A = (Z[k] + conj Z[L-k]) / 2, B = (Z[k] - conj Z[L-k]) / 2i
       const long long x = second ? u.y + w.y : u.x + w.x, y = second ? w.x - u.x : u.y - w.y;
-      dst[k] = bad ? make_double2(nan_of(), nan_of()) : make_double2(to_double(x, S), to_double(y, S));
+      dst[k] = make_double2(to_double_p(x, os), to_double_p(y, os));
     }
   }
 }
 
-// what of a length is launched
-enum FxOp { FX_OP_PREPARE = 0, FX_OP_STRIDED, FX_OP_TRUNCATE, FX_OP_C2R, FX_OP_R2C };
+// what of a length is launched; a length serves as padded length (multiples of
+// three), as grid length, or both
+enum FxOp { FX_OP_PREPARE = 0, FX_OP_INV_PAD, FX_OP_CUT, FX_OP_TRUNC, FX_OP_C2R_PAD, FX_OP_R2C, FX_OP_INV, FX_OP_C2R };
 
-template <int L> cudaError_t launch_len(FxOp op, const void *args, dim3 grid, cudaStream_t st) {
-  using F = Fft<L>;
-  switch (op) {
-    case FX_OP_PREPARE: {
-      cudaError_t e = cudaSuccess;
-      for (const void *f : {(const void *)k_fx_strided_l<L, false>, (const void *)k_fx_strided_l<L, true>,
-                            (const void *)k_fx_c2r_l<L>, (const void *)k_fx_r2c_l<L>})
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem);
-      return e;
+template <int L, bool PADDED, bool GRID> struct Launch {
+  static cudaError_t run(FxOp op, const void *args, dim3 grid, cudaStream_t st) {
+    using F = Fft<L, false>;
+    const LArgs *s = static_cast<const LArgs *>(args);
+    const LRows *r = static_cast<const LRows *>(args);
+    cudaError_t e = cudaSuccess;
+    auto limit = [&](const void *f) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem);
+    };
+    bool done = op == FX_OP_PREPARE;
+    if constexpr (PADDED) {
+      if (op == FX_OP_PREPARE) {
+        limit((const void *)k_fx_inv<L, true>);
+        limit((const void *)k_fx_cut<L>);
+        limit((const void *)k_fx_trunc<L>);
+        limit((const void *)k_fx_c2r_l<L, true>);
+        limit((const void *)k_fx_r2c_l<L>);
+      }
+      done = true;
+      if (op == FX_OP_INV_PAD) k_fx_inv<L, true><<<grid, F::T, F::smem, st>>>(*s);
+      else if (op == FX_OP_CUT) k_fx_cut<L><<<grid, F::T, F::smem, st>>>(*s);
+      else if (op == FX_OP_TRUNC) k_fx_trunc<L><<<grid, F::T, F::smem, st>>>(*s);
+      else if (op == FX_OP_C2R_PAD) k_fx_c2r_l<L, true><<<grid, F::T, F::smem, st>>>(*r);
+      else if (op == FX_OP_R2C) k_fx_r2c_l<L><<<grid, F::T, F::smem, st>>>(*r);
+      else done = op == FX_OP_PREPARE;
     }
-    case FX_OP_STRIDED: k_fx_strided_l<L, false><<<grid, F::T, F::smem, st>>>(*static_cast<const LArgs *>(args)); break;
-    case FX_OP_TRUNCATE: k_fx_strided_l<L, true><<<grid, F::T, F::smem, st>>>(*static_cast<const LArgs *>(args)); break;
-    case FX_OP_C2R: k_fx_c2r_l<L><<<grid, F::T, F::smem, st>>>(*static_cast<const LRows *>(args)); break;
-    case FX_OP_R2C: k_fx_r2c_l<L><<<grid, F::T, F::smem, st>>>(*static_cast<const LRows *>(args)); break;
+    if constexpr (GRID) {
+      if (op == FX_OP_PREPARE) {
+        limit((const void *)k_fx_inv<L, false>);
+        limit((const void *)k_fx_c2r_l<L, false>);
+      }
+      if (op == FX_OP_INV) {
+        k_fx_inv<L, false><<<grid, F::T, F::smem, st>>>(*s);
+        done = true;
+      } else if (op == FX_OP_C2R) {
+        k_fx_c2r_l<L, false><<<grid, F::T, F::smem, st>>>(*r);
+        done = true;
+      }
+    }
+    if (!done) return cudaErrorInvalidValue;
+    return e == cudaSuccess ? cudaGetLastError() : e;
   }
-  return cudaGetLastError();
-}
+};
 
 }  // namespace fx

@@ -3,11 +3,11 @@
 #include "fx64_len.cuh"
 
 namespace fx {
-template cudaError_t launch_len<16>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<24>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<32>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<48>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<64>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<72>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<96>(FxOp, const void *, dim3, cudaStream_t);
+template struct Launch<16, false, true>;
+template struct Launch<24, true, true>;
+template struct Launch<32, false, true>;
+template struct Launch<48, true, true>;
+template struct Launch<64, false, true>;
+template struct Launch<72, true, false>;
+template struct Launch<96, true, true>;
 }  // namespace fx

@@ -3,8 +3,8 @@
 #include "fx64_len.cuh"
 
 namespace fx {
-template cudaError_t launch_len<128>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<144>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<192>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<256>(FxOp, const void *, dim3, cudaStream_t);
+template struct Launch<128, false, true>;
+template struct Launch<144, true, false>;
+template struct Launch<192, true, true>;
+template struct Launch<256, false, true>;
 }  // namespace fx

@@ -3,7 +3,7 @@
 #include "fx64_len.cuh"
 
 namespace fx {
-template cudaError_t launch_len<288>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<384>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<512>(FxOp, const void *, dim3, cudaStream_t);
+template struct Launch<288, true, false>;
+template struct Launch<384, true, true>;
+template struct Launch<512, false, true>;
 }  // namespace fx

@@ -1,9 +1,8 @@
-// Fixed-point transforms of the lengths 576, 768, 1152 (one translation unit per group of
+// Fixed-point transforms of the lengths 576, 768 (one translation unit per group of
 // lengths, compiled in parallel).
 #include "fx64_len.cuh"
 
 namespace fx {
-template cudaError_t launch_len<576>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<768>(FxOp, const void *, dim3, cudaStream_t);
-template cudaError_t launch_len<1152>(FxOp, const void *, dim3, cudaStream_t);
+template struct Launch<576, true, false>;
+template struct Launch<768, true, true>;
 }  // namespace fx
