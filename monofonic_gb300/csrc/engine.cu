@@ -151,7 +151,8 @@ struct mfx_job {
   // plain FP64 form: transforms in 64-bit fixed point (fx64.h) and their tables
   bool fx = false;
   longlong2 *fx_twm = nullptr, *fx_twn = nullptr;  // twiddles of M and N
-  double *fx_mode = nullptr, *fx_rinv = nullptr;   // fx::Strided::mode, rinv
+  // of every plain FP64 job (fx::fill_tables)
+  double *fx_mode = nullptr, *fx_rinv = nullptr, *fx_root = nullptr;
   int *dstatus = nullptr;      // device status word: nonzero when a kernel's bounded wait ran out
   size_t rsize = 8;
   cudaStream_t stream = nullptr;
@@ -436,9 +437,9 @@ static Layout plan_layout(const mfx_job_desc *d, size_t work_bytes, bool group_a
     L.ff_tw = align_up(size_t(M) * 8) + align_up(size_t(N) * 8);
     L.status = align_up(sizeof(int));
   }
-  if (fx_supported(d))
-    L.fx = align_up(fx::twiddle_bytes(M)) + align_up(fx::twiddle_bytes(N)) +
-           align_up(2 * size_t(N) * 8) + align_up(fx::rinv_len(N) * 8);
+  if (d->precision == MFX_FP64)
+    L.fx = align_up(fx::twiddle_bytes(M)) + align_up(fx::twiddle_bytes(N)) + align_up(5 * size_t(N) * 8) +
+           2 * align_up(fx::rinv_len(N) * 8);
   const size_t np = size_t(ns) * N * N * N;
   L.part_bytes = 0;
   if (d->want_particles) {
@@ -1438,12 +1439,20 @@ template <typename R> static int assemble_stage(mfx_job *j, int mask) {
   a.in_scale2 = 1.0 / j->scale2;
   a.in_scale3 = 1.0 / j->scale3;
   asm_float_coefficients(a);
+  a.rinv = j->fx_rinv;
+  a.root = j->fx_root;
+  a.frac = j->fx_mode ? j->fx_mode + 2 * size_t(N) : nullptr;
+  a.sidx = a.frac ? a.frac + N : nullptr;
+  a.node = reinterpret_cast<const int *>(a.frac ? a.frac + 2 * size_t(N) : nullptr);
   if (j->qvbc && (mask & 1)) {
     a.qvbc = j->qvbc;
     a.qvbc32 = j->qvbc32;
     a.qvbc_len = j->sp_len;
   }
   a.nyq = nyq_steps(j);
+  for (int s = 0; s < j->ns; ++s)
+    for (int ax = 0; ax < 3; ++ax)
+      if (kShifts[j->d.lattice][s][ax] + j->lat_off[ax] != 0.0) a.shifted |= 1u << s;
   if (j->fused) {
     TRY(assemble_fused(j, a));
     return j->want_masses ? mass_stage<R>(j) : MFX_OK;
@@ -1455,8 +1464,16 @@ template <typename R> static int assemble_stage(mfx_job *j, int mask) {
     a.nshift = g;
     for (int q = 0; q < 6 * g; ++q) a.out[q] = j->asmbuf[q];
     KBEGIN(j);
-    if (a.plt) k_assemble<R, true><<<grid_for(total, 256, nsm), 256, 0, j->stream>>>(a);
-    else k_assemble<R, false><<<grid_for(total, 256, nsm), 256, 0, j->stream>>>(a);
+    if constexpr (sizeof(R) == 8) {
+      // one warp per row (i, j), eight of them a CTA
+      const unsigned gr = unsigned(std::min<size_t>((size_t(N) * N + 7) / 8, size_t(nsm) * 16));
+      if (a.plt) k_assemble_rows<true><<<gr, 256, 0, j->stream>>>(a);
+      else k_assemble_rows<false><<<gr, 256, 0, j->stream>>>(a);
+    } else if (a.plt) {
+      k_assemble<R, true><<<grid_for(total, 256, nsm), 256, 0, j->stream>>>(a);
+    } else {
+      k_assemble<R, false><<<grid_for(total, 256, nsm), 256, 0, j->stream>>>(a);
+    }
     KEND(j, "assemble", ((order == 1 ? 1.0 : (order == 2 ? 2.0 : 6.0)) + 6.0 * g) * j->n_field_bytes);
     for (int s = 0; s < g; ++s) {
       // the six components (batched)
@@ -2024,21 +2041,22 @@ static int create_job(mfx_engine *eng, const mfx_job_desc *d, mfx_job **out, int
   p += L.ff_tw;
   j->dstatus = L.status ? reinterpret_cast<int *>(p) : nullptr;
   p += L.status;
-  if (j->fx) {
+  if (j->fp64) {
     char *f = p;
     j->fx_twm = reinterpret_cast<longlong2 *>(f);
     f += align_up(fx::twiddle_bytes(j->M));
     j->fx_twn = reinterpret_cast<longlong2 *>(f);
     f += align_up(fx::twiddle_bytes(j->N));
     j->fx_mode = reinterpret_cast<double *>(f);
-    f += align_up(2 * size_t(j->N) * 8);
+    f += align_up(5 * size_t(j->N) * 8);
     j->fx_rinv = reinterpret_cast<double *>(f);
-    cudaError_t fe = fx::prepare_device(eng->device);
+    j->fx_root = reinterpret_cast<double *>(f + align_up(fx::rinv_len(j->N) * 8));
+    cudaError_t fe = j->fx ? fx::prepare_device(eng->device) : cudaSuccess;
     for (const int len : {j->M, j->N})
-      if (fe == cudaSuccess && (len == j->N || d->lpt_order >= 2))
+      if (fe == cudaSuccess && j->fx && (len == j->N || d->lpt_order >= 2))
         fe = cudaMemcpyAsync(len == j->M ? j->fx_twm : j->fx_twn, fx::twiddles(len), fx::twiddle_bytes(len),
                              cudaMemcpyHostToDevice, j->stream);
-    if (fe == cudaSuccess) fe = fx::fill_tables(j->N, j->fx_mode, j->fx_rinv, j->stream);
+    if (fe == cudaSuccess) fe = fx::fill_tables(j->N, j->fx_mode, j->fx_rinv, j->fx_root, j->stream);
     if (fe != cudaSuccess) return fail(set_error(MFX_ECUDA, "fixed-point transform set-up: %s", cudaGetErrorString(fe)));
   }
   p += L.fx;

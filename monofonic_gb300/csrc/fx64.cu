@@ -545,19 +545,24 @@ static int len_bits(const LenEntry &l, FxKind kind, bool forward, bool inverse) 
   return b;
 }
 
-static __global__ void k_fx_tables(int n, double *mode, double *rinv, int len) {
+static __global__ void k_fx_tables(int n, double *mode, double *rinv, double *root, int len) {
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < len; q += gridDim.x * blockDim.x) {
     rinv[q] = q ? 1.0 / double(q) : 0.0;
+    root[q] = sqrt(double(q));
     if (q < n) {
       const int i = q == n / 2 ? 0 : (q > n / 2 ? q - n : q);
       mode[q] = double(i);
       mode[n + q] = double(i) * double(i);
+      const double ratio = 64.0 / double(n), x = double(q) * ratio, f = floor(x);
+      mode[2 * n + q] = x - f;
+      mode[3 * n + q] = (x - (x > 32.0 ? 64.0 : 0.0)) / ratio;
+      reinterpret_cast<int *>(mode + 4 * n)[q] = int(f);
     }
   }
 }
-cudaError_t fill_tables(int n, double *mode, double *rinv, cudaStream_t st) {
+cudaError_t fill_tables(int n, double *mode, double *rinv, double *root, cudaStream_t st) {
   const int len = int(rinv_len(n));
-  k_fx_tables<<<unsigned(std::min((len + 255) / 256, 608)), 256, 0, st>>>(n, mode, rinv, len);
+  k_fx_tables<<<unsigned(std::min((len + 255) / 256, 608)), 256, 0, st>>>(n, mode, rinv, root, len);
   return cudaGetLastError();
 }
 

@@ -13,9 +13,13 @@ bool length_supported(int L);
 // each length that was asked for)
 const longlong2 *twiddles(int L);
 inline size_t twiddle_bytes(int L) { return (size_t(L) * 40 + 15) / 16 * 16; }
-// device tables of a grid: mode[2][n] (Strided::mode) and rinv[q] = 1 / q,
-// q = 1 .. 3 (n/2)^2 (rinv[0] = 0)
-cudaError_t fill_tables(int n, double *mode, double *rinv, cudaStream_t st);
+// device tables of a grid: mode[0..1][n] (Strided::mode), mode[2][n] the
+// fractional part and mode[4][n] (as int) the integer part of the PLT table
+// coordinate x = i * (64 / n), mode[3][n] the signed mode index that x stands for,
+// (x - 64 (x > 32)) / (64 / n), all evaluated in double as particle_plt.hh:551-585
+// does (where 64 / n is rounded, so are the small negative indices); rinv[q] = 1 / q and root[q] = sqrt(q) for
+// q = 1 .. 3 (n/2)^2 (zero at q = 0)
+cudaError_t fill_tables(int n, double *mode, double *rinv, double *root, cudaStream_t st);
 inline size_t rinv_len(int n) { return 3 * size_t(n / 2) * (n / 2) + 1; }
 // the kernels' shared memory limits on the current device `dev`, once (before
 // any capture)

@@ -477,8 +477,14 @@ struct AsmArgs {
   // weight, n = |k|^2 / kf^2 (null: no term)
   const double *qvbc;
   const float *qvbc32;
+  // plain FP64 form: 1 / q and sqrt(q) per |k|^2 index; per axis index the
+  // fractional part of the PLT table coordinate, the signed index and the
+  // integer part (fx64.h fill_tables)
+  const double *rinv, *root, *frac, *sidx;
+  const int *node;
   size_t qvbc_len;
   NyqSteps nyq;
+  unsigned shifted;  // bit s: sub-lattice s lies off the grid points
 };
 
 // the float coefficients of an AsmArgs from its FP64 ones
@@ -493,26 +499,6 @@ inline void asm_float_coefficients(AsmArgs &a) {
   a.fv3 = float(a.vfac3);
   a.fpfac = float(a.pfac);
   a.fvfac = float(a.vfac);
-}
-
-// get_cic_kspace (grid_fft.hh:347-373) on a 64 x 64 x 33 real table
-__device__ __forceinline__ double plt_cic(const double *T, double x, double y, double z) {
-  const int ix = int(floor(x)), iy = int(floor(y)), iz = int(floor(z));
-  const double dx = x - double(ix), tx = 1.0 - dx;
-  const double dy = y - double(iy), ty = 1.0 - dy;
-  const double dz = z - double(iz), tz = 1.0 - dz;
-  const int ix1 = (ix + 1) % 64, iy1 = (iy + 1) % 64, iz1 = min(iz + 1, 32);
-  auto e = [T](int a, int b, int c) { return T[(size_t(a) * 64 + b) * 33 + c]; };
-  double v = 0.0;
-  v += e(ix, iy, iz) * tx * ty * tz;
-  v += e(ix, iy, iz1) * tx * ty * dz;
-  v += e(ix, iy1, iz) * tx * dy * tz;
-  v += e(ix, iy1, iz1) * tx * dy * dz;
-  v += e(ix1, iy, iz) * dx * ty * tz;
-  v += e(ix1, iy, iz1) * dx * ty * dz;
-  v += e(ix1, iy1, iz) * dx * dy * tz;
-  v += e(ix1, iy1, iz1) * dx * dy * dz;
-  return v;
 }
 
 // FP32 form of the PLT gradient: the interpolation point x = i * 64/N is
@@ -575,44 +561,6 @@ __device__ __forceinline__ void plt_grad_f32(const TA &e, int i, int j, int k, i
   vcorr = al;
 }
 
-// particle::lattice_gradient::gradient / vfac_corr (particle_plt.hh:551-585):
-// the plain form evaluates the reference's FP64 expressions (interpolation
-// point i * 64/N in double, get_cic_kspace on the double tables); the FP32
-// form uses plt_grad_f32.
-template <typename R>
-__device__ __forceinline__ void plt_grad(const AsmArgs &a, int i, int j, int k, int N, R G[3], R &vcorr) {
-  if constexpr (sizeof(R) == 4) {
-    plt_grad_f32(PltGlobal{a.plt4}, i, j, k, N, a.fkfac, G, vcorr);
-  } else {
-    const double x = double(i) * a.mapratio, y = double(j) * a.mapratio, z = double(k) * a.mapratio;
-    const double twopi = 2.0 * 3.141592653589793;
-    const double kx = (x - double(x > 32.0) * 64.0) * twopi;
-    const double ky = (y - double(y > 32.0) * 64.0) * twopi;
-    const double kz = (z - double(z > 32.0) * 64.0) * twopi;
-    const double kr = sqrt(kx * kx + ky * ky + kz * kz);
-    const double kmod = kr / a.mapratio / a.boxlen;
-    const size_t TS = size_t(64) * 64 * 33;
-    const double Dr = plt_cic(a.plt, x, y, z);
-    const double Dt = plt_cic(a.plt + TS, x, y, z);
-    const double Dp = plt_cic(a.plt + 2 * TS, x, y, z);
-    const double al = plt_cic(a.plt + 3 * TS, x, y, z);
-    double st = 0.0, ct = 1.0, sp = 0.0, cp = 1.0;
-    if (kr > 0.0) {
-      const double kperp = sqrt(kx * kx + ky * ky);
-      st = kperp / kr;
-      ct = kz / kr;
-      if (kperp > 0.0) {
-        cp = kx / kperp;
-        sp = ky / kperp;
-      }
-    }
-    G[0] = R(kmod * (Dr * st * cp + Dt * ct * cp - Dp * sp));
-    G[1] = R(kmod * (Dr * st * sp + Dt * ct * sp + Dp * cp));
-    G[2] = R(kmod * (Dr * ct - Dt * st));
-    vcorr = R(1.0 / (1.0 / al));
-  }
-}
-
 // One k-space mode of the displacement (P) and velocity (V) components before
 // the sub-lattice phase (ic_generator.cc:929-1053): idx = (i N + j)(N/2+1) + k.
 // TAB: the FP32 form's PLT table accessor for the mode's own gradient (the
@@ -626,13 +574,10 @@ __device__ __forceinline__ void asm_mode(const AsmArgs &a, int i, int j, int k, 
   // Gp: gradient applied to the displacement, Gv: gradient times vfac_corr
   // applied to the velocity
   R Gp[3], Gv[3];
-  // the coefficients in R (the FP32 form's were rounded on the host)
-  constexpr bool F32 = sizeof(R) == 4;
-  const R c_kf = F32 ? R(a.fkfac) : R(a.kfac);
-  const R c_s1 = F32 ? R(a.fs1) : R(a.g1 * a.in_scale1), c_s2 = F32 ? R(a.fs2) : R(a.g2 * a.in_scale2);
-  const R c_s3 = F32 ? R(a.fs3) : R(a.g3 * a.in_scale3), c_sa = F32 ? R(a.fsa) : R(a.g3c * a.in_scale3);
-  const R c_v1 = F32 ? R(a.fv1) : R(a.vfac1), c_v2 = F32 ? R(a.fv2) : R(a.vfac2), c_v3 = F32 ? R(a.fv3) : R(a.vfac3);
-  const R c_pf = F32 ? R(a.fpfac) : R(a.pfac), c_vf = F32 ? R(a.fvfac) : R(a.vfac);
+  // the coefficients were rounded on the host
+  static_assert(sizeof(R) == 4, "the plain FP64 form assembles by rows (k_assemble_rows)");
+  const R c_kf = a.fkfac, c_s1 = a.fs1, c_s2 = a.fs2, c_s3 = a.fs3, c_sa = a.fsa;
+  const R c_v1 = a.fv1, c_v2 = a.fv2, c_v3 = a.fv3, c_pf = a.fpfac, c_vf = a.fvfac;
   if (!PLT) {
     // op::fourier_gradient (operators.hh:46-56): Nyquist index zeroed, exactly odd in k
     const R kf = c_kf;
@@ -643,10 +588,10 @@ __device__ __forceinline__ void asm_mode(const AsmArgs &a, int i, int j, int k, 
     for (int d = 0; d < 3; ++d) Gv[d] = Gp[d];
   } else {
     R G[3], vc;
-    if constexpr (!std::is_void<TAB>::value && sizeof(R) == 4)
+    if constexpr (!std::is_void<TAB>::value)
       plt_grad_f32(*tab, i, j, k, N, a.fkfac, G, vc);
     else
-      plt_grad<R>(a, i, j, k, N, G, vc);
+      plt_grad_f32(PltGlobal{a.plt4}, i, j, k, N, a.fkfac, G, vc);
     if (k == 0 || k == nh) {
       // On the kz = 0 and kz = N/2 planes the c2r sees both k and -k.  The
       // interpolated PLT gradient is not exactly odd where the CIC stencil
@@ -658,7 +603,7 @@ __device__ __forceinline__ void asm_mode(const AsmArgs &a, int i, int j, int k, 
       // the Nyquist planes, MUSIC1's.)
       const int im = i ? N - i : 0, jm = j ? N - j : 0;
       R Gm[3], vcm;
-      plt_grad<R>(a, im, jm, k, N, Gm, vcm);
+      plt_grad_f32(PltGlobal{a.plt4}, im, jm, k, N, a.fkfac, Gm, vcm);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         Gp[d] = R(0.5) * (G[d] - Gm[d]);
@@ -682,7 +627,7 @@ __device__ __forceinline__ void asm_mode(const AsmArgs &a, int i, int j, int k, 
     // weight times 1 + C A_theta_bc / (A k^2 g1)
     const int si = signed_idx(i, N), sj = signed_idx(j, N);
     const size_t n = size_t(si * si + sj * sj + k * k);
-    const R q = n < a.qvbc_len ? (F32 ? R(a.qvbc32[n]) : R(a.qvbc[n])) : R(0);
+    const R q = n < a.qvbc_len ? R(a.qvbc32[n]) : R(0);
     vs_re += q * vs_re;
     vs_im += q * vs_im;
   }
@@ -777,6 +722,207 @@ __global__ void __launch_bounds__(256) k_assemble(AsmArgs a) {
             mkc<R>(V[d].x * er - V[d].y * ei, V[d].x * ei + V[d].y * er);
       }
     }
+  }
+}
+
+// The assembly of the plain FP64 form: the same sums as asm_mode (the oracle's
+// expressions, particle_plt.hh:551-585 and ic_generator.cc:929-1053) with as few
+// FP64 operations as they can be written in, one warp per row (i, j).  GB300's
+// FP64 pipe bounds it (1.9 operations per SM and clock): evaluated mode by mode
+// the PLT gradient and the sums took about 460 operations, 6.5 ms at 256^3 BCC
+// and 23.9 ms at 384^3 FCC.
+//  * The CIC interpolation of the four tables is taken along x and y once per row,
+//    at the table's 33 kz nodes (shared memory); a mode interpolates along z only:
+//    two operations a table instead of 40.
+//  * k times the unit vectors of the spherical basis needs no angles: k e_r = k,
+//    k e_theta = (kz kx / rho, kz ky / rho, -rho), k e_phi = |k| (-ky, kx, 0) / rho,
+//    rho and |k| from a table of square roots by integer |k|^2.
+//  * The curl term is formed once for displacement and velocity; constant factors
+//    are multiplied on the host; a sub-lattice without a shift has no phase.
+struct AsmRow {
+  double wxy[4];   // CIC weights of the row's four (x, y) corners
+  int o[4];        // and their table offsets
+};
+__device__ __forceinline__ void asm_row_cic(const AsmArgs &a, int i, int j, AsmRow &r) {
+  const int ix = __ldg(&a.node[i]), iy = __ldg(&a.node[j]);
+  const double dx = __ldg(&a.frac[i]), dy = __ldg(&a.frac[j]), tx = 1.0 - dx, ty = 1.0 - dy;
+  const int x1 = (ix + 1) & 63, y1 = (iy + 1) & 63;
+  r.wxy[0] = tx * ty;
+  r.wxy[1] = tx * dy;
+  r.wxy[2] = dx * ty;
+  r.wxy[3] = dx * dy;
+  r.o[0] = (ix * 64 + iy) * 33;
+  r.o[1] = (ix * 64 + y1) * 33;
+  r.o[2] = (x1 * 64 + iy) * 33;
+  r.o[3] = (x1 * 64 + y1) * 33;
+}
+__device__ __forceinline__ double asm_row_at(const AsmRow &r, const double *T, int z) {
+  double v = __ldg(&T[r.o[0] + z]) * r.wxy[0];
+  v += __ldg(&T[r.o[1] + z]) * r.wxy[1];
+  v += __ldg(&T[r.o[2] + z]) * r.wxy[2];
+  return v + __ldg(&T[r.o[3] + z]) * r.wxy[3];
+}
+// (D_r, D_theta, D_phi) -> gradient over 2 pi / L; cp, sp = kx / rho, ky / rho
+__device__ __forceinline__ void asm_gradient(double Dr, double Dt, double Dp, double sx, double sy, double sz,
+                                             double rho, double R, double cp, double sp, double G[3]) {
+  const double u = Dt * sz, w = Dp * R;
+  G[0] = Dr * sx + u * cp - w * sp;
+  G[1] = Dr * sy + u * sp + w * cp;
+  G[2] = Dr * sz - Dt * rho;
+}
+
+template <bool PLT> __global__ void __launch_bounds__(256) k_assemble_rows(const __grid_constant__ AsmArgs a) {
+  __shared__ double tab[PLT ? 8 : 1][PLT ? 4 : 1][PLT ? 34 : 1];
+  const int N = a.N, nh = N >> 1, nk = nh + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const size_t TS = size_t(64) * 64 * 33;
+  const double kf = a.kfac;
+  // weights of the potentials in the displacement and in the velocity
+  const double s1 = a.g1 * a.in_scale1, s2 = a.g2 * a.in_scale2, s3 = a.g3 * a.in_scale3, sa = a.g3c * a.in_scale3;
+  const double pf = a.pfac * kf, vf = a.vfac * kf;
+  const double p1 = s1 * pf, p2 = s2 * pf, p3 = s3 * pf, pa = sa * pf;
+  const double v1 = a.vfac1 * s1 * vf, v2 = a.vfac2 * s2 * vf, v3 = a.vfac3 * s3 * vf, va = a.vfac3 * sa * vf;
+  // NGenIC's potentials vanish on every Nyquist index
+  const int kend = a.nyq.active ? nk : nh;
+  const size_t rows = size_t(N) * N;
+  for (size_t row = size_t(blockIdx.x) * 8 + wid; row < rows; row += size_t(gridDim.x) * 8) {
+    const int i = int(row / N), j = int(row - size_t(i) * N);
+    const int si = signed_idx(i, N), sj = signed_idx(j, N);
+    const double sx = PLT ? __ldg(&a.sidx[i]) : double(si), sy = PLT ? __ldg(&a.sidx[j]) : double(sj);
+    double rho = 0.0, cp = 1.0, sp = 0.0;
+    if constexpr (PLT) {
+      AsmRow r;
+      asm_row_cic(a, i, j, r);
+      __syncwarp();
+      for (int z = lane; z < 33; z += 32)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tab[wid][q][z] = asm_row_at(r, a.plt + q * TS, z);
+      __syncwarp();
+      const int q2 = si * si + sj * sj;
+      if (q2) {
+        rho = __ldg(&a.root[q2]);
+        const double ir = rho * __ldg(&a.rinv[q2]);
+        cp = sx * ir;
+        sp = sy * ir;
+      }
+    }
+    for (int k = lane; k < kend; k += 32) {
+      const size_t idx = row * nk + k;
+      double P[6], V[6];  // re, im of the three components over i
+      const double2 f1 = reinterpret_cast<const double2 *>(a.phi[0])[idx];
+      double w1 = v1;
+      if (a.qvbc) {
+        const size_t n = size_t(si * si + sj * sj + k * k);
+        w1 += w1 * (n < a.qvbc_len ? a.qvbc[n] : 0.0);
+      }
+      double pr = p1 * f1.x, pi = p1 * f1.y, vr = w1 * f1.x, vi = w1 * f1.y;
+      double2 A[3];
+      if (a.order > 1) {
+        const double2 f = reinterpret_cast<const double2 *>(a.phi[1])[idx];
+        pr += p2 * f.x;
+        pi += p2 * f.y;
+        vr += v2 * f.x;
+        vi += v2 * f.y;
+      }
+      if (a.order > 2) {
+        const double2 f = reinterpret_cast<const double2 *>(a.phi[2])[idx];
+        pr += p3 * f.x;
+        pi += p3 * f.y;
+        vr += v3 * f.x;
+        vi += v3 * f.y;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) A[d] = reinterpret_cast<const double2 *>(a.A3[d])[idx];
+      }
+      double G[3], vc = 1.0;
+      const double sz = PLT ? __ldg(&a.sidx[k]) : double(k);
+      if constexpr (!PLT) {
+        // op::fourier_gradient (operators.hh:46-56): Nyquist index zeroed
+        G[0] = i != nh ? sx : 0.0;
+        G[1] = j != nh ? sy : 0.0;
+        G[2] = k != nh ? sz : 0.0;
+      } else {
+        const int z0 = __ldg(&a.node[k]), z1 = min(z0 + 1, 32);
+        const double dz = __ldg(&a.frac[k]);
+        double D[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const double t0 = tab[wid][q][z0];
+          D[q] = t0 + dz * (tab[wid][q][z1] - t0);
+        }
+        vc = D[3];
+        const double R = __ldg(&a.root[si * si + sj * sj + k * k]);
+        asm_gradient(D[0], D[1], D[2], sx, sy, sz, rho, R, cp, sp, G);
+      }
+      auto combine = [&](const double *g, double fr, double fi, double c, double *o) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
+          double re = g[d] * fr, im = g[d] * fi;
+          if (a.order > 2) {
+            re += c * (g[d1] * A[d2].x - g[d2] * A[d1].x);
+            im += c * (g[d1] * A[d2].y - g[d2] * A[d1].y);
+          }
+          o[2 * d] = re;
+          o[2 * d + 1] = im;
+        }
+      };
+      if (PLT && (k == 0 || k == nh)) {
+        // odd part of the gradient on the planes that the c2r sees twice (asm_mode)
+        const int im = i ? N - i : 0, jm = j ? N - j : 0, z = k == 0 ? 0 : 32;
+        const int mi = signed_idx(im, N), mj = signed_idx(jm, N), q2 = mi * mi + mj * mj;
+        AsmRow r;
+        asm_row_cic(a, im, jm, r);
+        const double mx = __ldg(&a.sidx[im]), my = __ldg(&a.sidx[jm]), mrho = __ldg(&a.root[q2]);
+        const double ir = mrho * __ldg(&a.rinv[q2]);
+        double M[3], Gp[3], Gv[3];
+        const double vm = asm_row_at(r, a.plt + 3 * TS, z);
+        asm_gradient(asm_row_at(r, a.plt, z), asm_row_at(r, a.plt + TS, z), asm_row_at(r, a.plt + 2 * TS, z), mx, my, sz,
+                     mrho, __ldg(&a.root[q2 + k * k]), q2 ? mx * ir : 1.0, q2 ? my * ir : 0.0, M);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          Gp[d] = 0.5 * (G[d] - M[d]);
+          Gv[d] = 0.5 * (G[d] * vc - M[d] * vm);
+        }
+        combine(Gp, pr, pi, pa, P);
+        combine(Gv, vr, vi, va, V);
+      } else {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
+          P[2 * d] = G[d] * pr;
+          P[2 * d + 1] = G[d] * pi;
+          V[2 * d] = G[d] * vr;
+          V[2 * d + 1] = G[d] * vi;
+          if (a.order > 2) {
+            const double cr = G[d1] * A[d2].x - G[d2] * A[d1].x, ci = G[d1] * A[d2].y - G[d2] * A[d1].y;
+            P[2 * d] += pa * cr;
+            P[2 * d + 1] += pa * ci;
+            V[2 * d] += va * cr;
+            V[2 * d + 1] += va * ci;
+          }
+          if (PLT) {
+            V[2 * d] *= vc;
+            V[2 * d + 1] *= vc;
+          }
+        }
+      }
+      const bool dc = idx == 0;
+      for (int s = 0; s < a.nshift; ++s) {
+        double er = 1.0, ei = 0.0;
+        const bool phase = (a.shifted >> (a.shift0 + s)) & 1;
+        if (phase) lattice_phase<double>(a, a.shift0 + s, i, j, k, er, ei);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          // times i and the phase
+          const double re = c < 3 ? P[2 * c] : V[2 * c - 6], im = c < 3 ? P[2 * c + 1] : V[2 * c - 5];
+          double2 v = phase ? make_double2(-im * er - re * ei, re * er - im * ei) : make_double2(-im, re);
+          if (dc) v = make_double2(0.0, 0.0);
+          reinterpret_cast<double2 *>(a.out[s * 6 + c])[idx] = v;
+        }
+      }
+    }
+    if (kend < nk && lane < 6)
+      for (int s = 0; s < a.nshift; ++s)
+        reinterpret_cast<double2 *>(a.out[s * 6 + lane])[row * nk + nh] = make_double2(0.0, 0.0);
   }
 }
 
