@@ -1279,9 +1279,17 @@ static int assemble_fused(mfx_job *j, const AsmArgs &as) {
   // 57 -> 44 ms; 256^3 BCC: 0.63 -> 0.93 ms, so not there), and wherever the
   // 4-pencil form does not fit; MFX_FA_HALVES = 0 / 1 in the environment
   // forces it off / on where both fit (for comparisons)
+  // A simple cubic lattice (one sub-lattice) has nothing to share, but from the
+  // same sizes up the repeated assembly of the component groups (three times at
+  // 768) and the row pieces cost more than the memory the other forms take:
+  // 2LPT / 3LPT x pass at 384^3 1.26 / 2.14 ms by groups, 1.09 / 1.59 kept, 1.47 /
+  // 1.95 in halves; 768^3 15.4 / 29.7, 15.2 / 19.7, 11.9 / 19.3; 256^3 0.23 by
+  // groups, 0.25 kept
   const char *envh = getenv("MFX_FA_HALVES");
-  const bool halves = nsub > 1 && ff::fa_halves(j->M) &&
-                      (!ff::fa_keep(j->M) || (envh ? envh[0] == '1' : N >= 384));
+  const int halves_from = ns > 1 ? 384 : 768;
+  const bool halves = (nsub > 1 || ns == 1) && ff::fa_halves(j->M) &&
+                      ((nsub > 1 && !ff::fa_keep(j->M)) || (envh ? envh[0] == '1' : N >= halves_from));
+  const bool kept = nsub > 1 || (ns == 1 && N >= 384 && ff::fa_keep(j->M));
   const bool plt = as.plt != nullptr;
   ff::FAArgs fa{};
   fa.as = as;
@@ -1299,7 +1307,7 @@ static int assemble_fused(mfx_job *j, const AsmArgs &as) {
   fa.vscale = vscale;
   fa.vunscale = 1.0 / double(vscale);
   fa.vunscale_f = float(fa.vunscale);
-  fa.halves = halves ? 1 : 0;
+  fa.form = halves ? ff::FA_HALVES : (kept ? ff::FA_KEPT : ff::FA_GROUPS);
   auto pass = [&](int op, const char *name, double bytes) -> int {
     KBEGIN(j);
     const cudaError_t e = ff::fa_launch(j->M, op, plt, fa, j->stream);
@@ -1311,7 +1319,10 @@ static int assemble_fused(mfx_job *j, const AsmArgs &as) {
   // sub-lattices with equal x-shifts (FCC: 0, 0, 1/2, 1/2) share one x pass
   // output: the x pass applies only the x factor of the phase and the y pass
   // the y and z factors; each shared output is read out of place by the other
-  // sub-lattices first and in place by its own last.  MFX_FA_XONLY=0 in the
+  // sub-lattices first and in place by its own last.  The one sub-lattice of a
+  // simple cubic lattice goes the same way: without a secondary shift it has no
+  // y and z factors, and the x pass no product of three table entries per mode
+  // (768^3 in halves: 34.9 -> 11.9 ms).  MFX_FA_XONLY=0 in the
   // environment turns this off (for comparisons)
   int xrep[4] = {0, 0, 0, 0}, xvar[4] = {0, 0, 0, 0}, nxv = 0;
   for (int s = 0; s < ns; ++s) {
@@ -1321,7 +1332,7 @@ static int assemble_fused(mfx_job *j, const AsmArgs &as) {
     xvar[s] = v;
   }
   const char *envx = getenv("MFX_FA_XONLY");
-  if (nsub == ns && nxv < ns && !(envx && envx[0] == '0')) {
+  if (nsub == ns && (nxv < ns || ns == 1) && !(envx && envx[0] == '0')) {
     fa.shift = 0;
     fa.nsub = nxv;
     fa.xonly = 1;
@@ -1331,7 +1342,7 @@ static int assemble_fused(mfx_job *j, const AsmArgs &as) {
     }
     TRY(pass(ff::FA_X, "fa_x", in_b + 6 * nxv * qf));
     fa.xonly = 0;
-    fa.yzphase = 1;
+    fa.yzphase = ns > 1 || (as.shifted & 1) ? 1 : 0;
     for (int v = 0; v < nxv; ++v)
       for (int pass_rep = 0; pass_rep < 2; ++pass_rep)
         for (int s = 0; s < ns; ++s) {

@@ -24,6 +24,10 @@
 namespace mfx {
 namespace ff {
 
+// ASM1: the assembly repeated for each group of components (one sub-lattice),
+// kept in shared memory (FA::keep), or in halves with tiles of 8 pencils (FA::halves)
+enum FAForm { FA_GROUPS = 0, FA_KEPT, FA_HALVES };
+
 struct FAArgs {
   AsmArgs as;             // potentials, PLT tables, phases, coefficients
   float2 *q[6];           // component fields [N][N][N/2] of sub-lattice `shift` (ASM2 in place, ASM3 input)
@@ -37,7 +41,7 @@ struct FAArgs {
   int xonly, xsub[4];
   int yzphase;
   const float2 *qin[6];   // ASM2 input when not in place (null: q)
-  int halves;             // ASM1 in halves (tiles of 8 pencils; FA::halves), with nsub > 1
+  int form;               // ASM1 form (FAForm)
   const float2 *tw;       // W_N^t, t < N
   int *status;            // set when a bounded wait ran out
   int shift;              // sub-lattice

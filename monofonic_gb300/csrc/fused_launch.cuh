@@ -217,14 +217,14 @@ template <int M> cudaError_t fa_launch_m(int op, bool plt, const FAArgs &a, cuda
     constexpr size_t units1 = size_t(N) * (F::Kh / F::P);
     switch (op) {
       case FA_X:
-        if (a.nsub > 1 && a.halves) {
+        if (a.form == FA_HALVES) {
           if constexpr (F::halves) {
             if (plt) MFX_FF_PERSISTENT((k_fa_x_halves<N, true>), F::t1h, F::s1h + (F::halves_xs ? F::s1h_x : 0), size_t(N) * (F::Kh / F::P8), s, a);
             else MFX_FF_PERSISTENT((k_fa_x_halves<N, false>), F::t1h, F::s1h + (F::halves_xs ? F::s1h_x : 0), size_t(N) * (F::Kh / F::P8), s, a);
           } else {
             return cudaErrorInvalidValue;
           }
-        } else if (a.nsub > 1) {
+        } else if (a.form == FA_KEPT) {
           if constexpr (F::keep) {
             if (plt) MFX_FF_PERSISTENT((k_fa_x<N, true, true>), F::t1k, F::s1k, units1, s, a);
             else MFX_FF_PERSISTENT((k_fa_x<N, false, true>), F::t1k, F::s1k, units1, s, a);
