@@ -550,10 +550,11 @@ class Job:
 
 
 class _JobView(Job):
-    """A job owned by a Batch (not destroyed by this wrapper)."""
+    """A job owned by a Batch or a Server (not destroyed by this wrapper)."""
 
-    def __init__(self, handle, num_particles, pos64, vel64, id64, n):
+    def __init__(self, handle, num_particles, pos64, vel64, id64, n, owner):
         self._h = handle
+        self._owner = owner  # the batch or server keeps the job's device memory
         self.num_particles = num_particles
         self.pos64, self.vel64, self.id64 = pos64, vel64, id64
         self.n = n
@@ -610,7 +611,7 @@ class Batch:
     def job(self, q: int) -> Job:
         h = C.c_void_p()
         check(load().mfx_batch_job(self._h, q, C.byref(h)))
-        return _JobView(h, *self._meta[q])
+        return _JobView(h, *self._meta[q], self)
 
     def close(self):
         if self._h and self._h.value:
@@ -731,7 +732,7 @@ class Server:
     def job(self, ticket: int) -> Job:
         h = C.c_void_p()
         check(load().mfx_server_job(self._h, ticket, C.byref(h)))
-        return _JobView(h, *self._meta[ticket])
+        return _JobView(h, *self._meta[ticket], self)
 
     def release(self, ticket: int):
         check(load().mfx_server_release(self._h, ticket))
