@@ -636,8 +636,9 @@ template <typename R> static int launch_noise(mfx_job *j, int mode, void *out) {
   a.norm = (j->d.inversion ? -1.0 : 1.0) / volfac;
   a.out_scale = j->scale1;
   const int cols = j->N * j->N;
+  a.split = noise_split(j->N, num_sm());
   KBEGIN(j);
-  k_noise_phi1<R><<<(cols + 127) / 128, 128, 0, j->stream>>>(a, (typename Cplx<R>::T *)out);
+  k_noise_phi1<R><<<noise_grid(j->N, a.split), 128, 0, j->stream>>>(a, (typename Cplx<R>::T *)out);
   KEND(j, "noise_phi1", j->n_field_bytes + 4.0 * cols + 8.0 * j->d.amp_table_len);
   return MFX_OK;
 }

@@ -135,11 +135,14 @@ extern "C" int mfx_noise_fill_noalloc(mfx_engine *eng, uint32_t ngrid, double bo
   const double volfac = std::pow(boxlen / ngrid / 2.0 / M_PI, 1.5);
   a.norm = (inversion ? -1.0 : 1.0) / volfac;
   a.out_scale = 1.0;
-  const int cols = int(ngrid * ngrid);
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+  a.split = noise_split(a.N, sms);
+  const unsigned grid = noise_grid(a.N, a.split);
   if (precision == MFX_FP64)
-    k_noise_phi1<double><<<(cols + 127) / 128, 128, 0, st>>>(a, static_cast<double2 *>(out_device));
+    k_noise_phi1<double><<<grid, 128, 0, st>>>(a, static_cast<double2 *>(out_device));
   else
-    k_noise_phi1<float><<<(cols + 127) / 128, 128, 0, st>>>(a, static_cast<float2 *>(out_device));
+    k_noise_phi1<float><<<grid, 128, 0, st>>>(a, static_cast<float2 *>(out_device));
   e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(MFX_ECUDA, "noise kernel launch: %s", cudaGetErrorString(e));
   return MFX_OK;
