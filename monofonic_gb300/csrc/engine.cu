@@ -148,9 +148,9 @@ struct mfx_job {
   void *ffC[17] = {};          // C-space [M][M][N/2] complex
   float2 *ff_tw = nullptr;     // W_M^t, t < M
   float2 *ff_twn = nullptr;    // W_N^t, t < N (fused assembly)
-  // plain FP64 form: transforms in 64-bit fixed point (fx64.h) and their tables
+  // pruned transforms (fx64.h; FP64 in 64-bit fixed point) and their tables
   bool fx = false;
-  longlong2 *fx_twm = nullptr, *fx_twn = nullptr;  // twiddles of M and N
+  void *fx_twm = nullptr, *fx_twn = nullptr;  // twiddles of M and N
   // of every plain FP64 job (fx::fill_tables)
   double *fx_mode = nullptr, *fx_rinv = nullptr, *fx_root = nullptr;
   int *dstatus = nullptr;      // device status word: nonzero when a kernel's bounded wait ran out
@@ -392,13 +392,15 @@ static bool fused_supported(const mfx_job_desc *d) {
   return (N / 2) % 8 == 0 && ff::ff_length_supported(M);
 }
 
-// The plain FP64 form runs its transforms in 64-bit fixed point (fx64.cuh) for
-// grids whose length and padded length have no prime factor above 7; other
-// grids use cuFFT.  MFX_FUSED=0 sends this form through cuFFT as well.  One
-// padded D2Z at 384^3 took cuFFT 7.15 ms, the three fixed-point passes 1.6 ms
-// without any pruning; at 96^3 0.11 and 0.04 ms: no size favours cuFFT.
+// Grids whose length and padded length have no prime factor above 7 take the
+// pruned pencil transforms of fx64.h: the plain FP64 form in 64-bit fixed point,
+// the FP32 form, where it has no fused transforms, in single precision; other
+// grids use cuFFT.  MFX_FUSED=0 sends all of them through cuFFT.  One padded D2Z
+// at 384^3 took cuFFT 7.15 ms, the three fixed-point passes 1.6 ms without any
+// pruning, at 96^3 0.11 and 0.04 ms; a single-precision 3LPT job's transforms at
+// 256^3 took it 13.4 ms, the pruned passes 6.3 ms: no size favours cuFFT.
 static bool fx_supported(const mfx_job_desc *d) {
-  if (d->precision != MFX_FP64) return false;
+  if (fused_supported(d)) return false;
   const char *env = getenv("MFX_FUSED");
   if (env && env[0] == '0') return false;
   const int N = d->ngrid;
@@ -437,6 +439,7 @@ static Layout plan_layout(const mfx_job_desc *d, size_t work_bytes, bool group_a
     L.ff_tw = align_up(size_t(M) * 8) + align_up(size_t(N) * 8);
     L.status = align_up(sizeof(int));
   }
+  if (d->precision == MFX_FP32C && fx_supported(d)) L.fx = align_up(size_t(M) * 8) + align_up(size_t(N) * 8);
   if (d->precision == MFX_FP64)
     L.fx = align_up(fx::twiddle_bytes(M)) + align_up(fx::twiddle_bytes(N)) + align_up(5 * size_t(N) * 8) +
            2 * align_up(fx::rinv_len(N) * 8);
@@ -909,7 +912,8 @@ static int run_potentials_fused(mfx_job *j) {
 }
 
 // ---------------------------------------------------------------------------
-// pruned transforms of the plain FP64 form in fixed point (fx64.h)
+// pruned transforms (fx64.h): of the plain FP64 form in fixed point, of the FP32
+// form's grids without fused transforms in single precision
 // ---------------------------------------------------------------------------
 // The padded fields stay in their M-grid slots throughout: a slot holds rows
 // (x, y) of M + 2 reals or their kz < M/2 + 1 spectra; after the y pass of an
@@ -917,12 +921,12 @@ static int run_potentials_fused(mfx_job *j) {
 // kz >= N/2 (+ 1 where the noise fills the Nyquist planes) are never touched.
 static int fx_pass(mfx_job *j, const fx::Strided &s, const char *name, double bytes) {
   KBEGIN(j);
-  const cudaError_t e = fx::run_strided(s, j->stream);
+  const cudaError_t e = j->fp64 ? fx::run_strided(s, j->stream) : fx::run_strided32(s, j->stream);
   if (e != cudaSuccess) return set_error(MFX_ECUDA, "%s (length %d): %s", name, s.L, cudaGetErrorString(e));
-  KEND(j, name, bytes);
+  KEND(j, name, bytes * j->rsize / 8.0);
   return MFX_OK;
 }
-static int fx_rows(mfx_job *j, int L, const longlong2 *tw, int kc, void *const *f, int count, bool inverse,
+static int fx_rows(mfx_job *j, int L, const void *tw, int kc, void *const *f, int count, bool inverse,
                    const char *name) {
   fx::Rows r{};
   r.L = L;
@@ -931,11 +935,12 @@ static int fx_rows(mfx_job *j, int L, const longlong2 *tw, int kc, void *const *
   r.rows = (long long)L * L;
   r.pitch = L + 2;
   r.count = count;
-  for (int c = 0; c < count; ++c) r.field[c] = static_cast<double *>(f[c]);
+  for (int c = 0; c < count; ++c) r.field[c] = f[c];
   KBEGIN(j);
-  const cudaError_t e = inverse ? fx::run_c2r(r, j->stream) : fx::run_r2c(r, j->stream);
+  const cudaError_t e = j->fp64 ? (inverse ? fx::run_c2r(r, j->stream) : fx::run_r2c(r, j->stream))
+                                : (inverse ? fx::run_c2r32(r, j->stream) : fx::run_r2c32(r, j->stream));
   if (e != cudaSuccess) return set_error(MFX_ECUDA, "%s (length %d): %s", name, L, cudaGetErrorString(e));
-  KEND(j, name, double(count) * L * L * (16.0 * kc + 8.0 * L));
+  KEND(j, name, double(count) * L * L * (2.0 * kc + L) * j->rsize);
   return MFX_OK;
 }
 // one op per field in its own group
@@ -943,8 +948,8 @@ static void fx_ops(fx::Strided &s, int count, void *const *src, void *const *dst
   s.ops = s.groups = count;
   for (int c = 0; c < count; ++c) {
     s.first[c] = c;
-    s.src[c] = static_cast<const double2 *>(src[c]);
-    s.dst[c] = static_cast<double2 *>(dst[c]);
+    s.src[c] = src[c];
+    s.dst[c] = dst[c];
   }
   s.first[count] = count;
 }
@@ -974,8 +979,9 @@ static void fx_slot_x(const mfx_job *j, fx::Strided &s) {
 // functor of convolution.hh:136-157 without its factor -(2 pi / L)^2 and the
 // pad factor, which the later passes put in): along y, phi, ky phi and ky^2 phi
 // go to the slots of zz, yz and yy; along x, each of these makes its group's
-// outputs with kx and kz factors, the one in its own slot last
-static int fx_hessians(mfx_job *j, const void *phi, void **H, int kc) {
+// outputs with kx and kz factors, the one in its own slot last.  fac: factor of
+// the single-precision form's Hessians, which keeps them at the size of delta
+static int fx_hessians(mfx_job *j, const void *phi, void **H, int kc, double fac) {
   const double N = j->N, M = j->M, by = 16.0 * kc;
   fx::Strided y = fx_base(j, kc);
   y.inverse = true;
@@ -987,6 +993,7 @@ static int fx_hessians(mfx_job *j, const void *phi, void **H, int kc) {
   void *dst[3] = {H[2], H[5], H[1]};
   fx_ops(y, 3, src, dst);
   for (int o = 0; o < 3; ++o) y.pr[o] = o;
+  y.in_fac = fac;
   TRY(fx_pass(j, y, "fx_y3", (N * N + 3 * N * M) * by));
   fx::Strided x = fx_base(j, kc);
   x.inverse = true;
@@ -1001,8 +1008,8 @@ static int fx_hessians(mfx_job *j, const void *phi, void **H, int kc) {
   x.first[2] = 5;
   x.first[3] = 6;
   for (int o = 0; o < 6; ++o) {
-    x.src[o] = static_cast<const double2 *>(H[in[o]]);
-    x.dst[o] = static_cast<double2 *>(H[out[o]]);
+    x.src[o] = H[in[o]];
+    x.dst[o] = H[out[o]];
     x.pr[o] = pr[o];
     x.pk[o] = pk[o];
   }
@@ -1073,9 +1080,10 @@ static int fx_c2r_n(mfx_job *j, void *const *f, int count) {
   return fx_rows(j, j->N, j->fx_twn, kc, f, count, true, "fx_n_c2r");
 }
 
-// LPT potentials of the plain FP64 form.  Slots as in the cuFFT route: 0..5 the
-// phi1 Hessians, 6..10 sources and pair products, 11..16 the phi2 Hessians.
-static int run_potentials_fx(mfx_job *j) {
+// LPT potentials through the pruned transforms.  Slots as in the cuFFT route:
+// 0..5 the phi1 Hessians, 6..10 sources and pair products, 11..16 the phi2
+// Hessians.
+template <typename R> static int run_potentials_fx(mfx_job *j) {
   const int nsm = num_sm();
   const double M3 = double(j->M) * j->M * j->M, N3 = double(j->N) * j->N * j->N;
   const double kf = 2.0 * M_PI / j->d.boxlen;
@@ -1084,31 +1092,35 @@ static int run_potentials_fx(mfx_job *j) {
   // h = kf^2 / sqrt(N^3); an unpadded product of two carries h^2 sqrt(N^3) / M^3,
   // over kf^2 for the inverse Laplacian; a truncated pair 1 / M^3 and the -h of
   // the third Hessian.  Evaluated with the fewest roundings: they scale a field.
-  const double ufac = kf * kf / (M3 * std::sqrt(N3)), tfac = -ufac;
+  // In single precision the Hessians carry h themselves (their exponents' range
+  // is the smaller one): ufac and tfac over h^2 and h.
+  const bool f32 = sizeof(R) == 4;
+  const double h = kf * kf / std::sqrt(N3), u = kf * kf / (M3 * std::sqrt(N3));
+  const double hfac = f32 ? h : 0.0, ufac = f32 ? u / (h * h) : u, tfac = f32 ? -u / h : -u;
   const size_t mreal = size_t(j->M) * j->M * (j->M + 2);
   const unsigned grid = grid_for(mreal, 256, nsm);
   void **H1 = &j->mslot[0], **T = &j->mslot[6], **H2 = &j->mslot[11];
   SrcArgs s{};
-  TRY(fx_hessians(j, j->nf[0], H1, j->d.noise_generator == MFX_NOISE_NGENIC ? j->nh : j->nk));
+  TRY(fx_hessians(j, j->nf[0], H1, j->d.noise_generator == MFX_NOISE_NGENIC ? j->nh : j->nk, hfac));
   for (int c = 0; c < 6; ++c) s.h1[c] = H1[c];
   s.count = mreal;
   s.out[0] = T[0];
   KBEGIN(j);
-  k_src2<double><<<grid, 256, 0, j->stream>>>(s);
+  k_src2<R><<<grid, 256, 0, j->stream>>>(s);
   KEND(j, "src2", 7.0 * j->m_field_bytes);
   TRY(fx_unpad(j, T, &j->nf[1], 1, ufac));
   if (j->timed) CU(cudaEventRecord(j->ev[2], j->stream));
   if (j->d.lpt_order < 3) return MFX_OK;
   for (int t = 0; t < 5; ++t) s.out[t] = T[t];
   KBEGIN(j);
-  k_pairs3a<double><<<grid, 256, 0, j->stream>>>(s);
+  k_pairs3a<R><<<grid, 256, 0, j->stream>>>(s);
   KEND(j, "pairs3a", 10.0 * j->m_field_bytes);
   TRY(fx_truncate(j, T, 5, tfac));
-  TRY(fx_hessians(j, j->nf[1], H2, j->nh));
+  TRY(fx_hessians(j, j->nf[1], H2, j->nh, hfac));
   for (int c = 0; c < 6; ++c) s.h2[c] = H2[c];
   for (int t = 0; t < 5; ++t) s.t[t] = T[t];
   KBEGIN(j);
-  k_src3<double><<<grid, 256, 0, j->stream>>>(s);
+  k_src3<R><<<grid, 256, 0, j->stream>>>(s);
   KEND(j, "src3", 21.0 * j->m_field_bytes);
   return fx_unpad(j, T, &j->nf[2], 4, ufac);
 }
@@ -1553,7 +1565,7 @@ template <typename R> static int run_pipeline(mfx_job *j) {
   if (j->fused) {
     TRY(run_potentials_fused(j));
   } else if (j->fx && order >= 2) {
-    TRY(run_potentials_fx(j));
+    TRY(run_potentials_fx<R>(j));
   } else {
   if (order >= 2) {
     TRY(hessians<R>(j, j->nf[0], H1));
@@ -2055,9 +2067,9 @@ static int create_job(mfx_engine *eng, const mfx_job_desc *d, mfx_job **out, int
   p += L.status;
   if (j->fp64) {
     char *f = p;
-    j->fx_twm = reinterpret_cast<longlong2 *>(f);
+    j->fx_twm = f;
     f += align_up(fx::twiddle_bytes(j->M));
-    j->fx_twn = reinterpret_cast<longlong2 *>(f);
+    j->fx_twn = f;
     f += align_up(fx::twiddle_bytes(j->N));
     j->fx_mode = reinterpret_cast<double *>(f);
     f += align_up(5 * size_t(j->N) * 8);
@@ -2070,6 +2082,16 @@ static int create_job(mfx_engine *eng, const mfx_job_desc *d, mfx_job **out, int
                              cudaMemcpyHostToDevice, j->stream);
     if (fe == cudaSuccess) fe = fx::fill_tables(j->N, j->fx_mode, j->fx_rinv, j->fx_root, j->stream);
     if (fe != cudaSuccess) return fail(set_error(MFX_ECUDA, "fixed-point transform set-up: %s", cudaGetErrorString(fe)));
+  }
+  if (j->fx && !j->fp64) {
+    j->fx_twm = p;
+    j->fx_twn = p + align_up(size_t(j->M) * 8);
+    cudaError_t fe = fx::prepare_device32(eng->device);
+    for (const int len : {j->M, j->N})
+      if (fe == cudaSuccess && (len == j->N || d->lpt_order >= 2))
+        fe = cudaMemcpyAsync(len == j->M ? j->fx_twm : j->fx_twn, fx::twiddles32(len), size_t(len) * 8,
+                             cudaMemcpyHostToDevice, j->stream);
+    if (fe != cudaSuccess) return fail(set_error(MFX_ECUDA, "pruned transform set-up: %s", cudaGetErrorString(fe)));
   }
   p += L.fx;
   if (j->dstatus && (cudaMemsetAsync(j->dstatus, 0, sizeof(int), j->stream) != cudaSuccess))

@@ -136,6 +136,19 @@ static void make_twiddles(int L, longlong2 *out) {
 }
 
 bool length_supported(int L) { return fx_supported(L); }
+const float2 *twiddles32(int L) {
+  static std::mutex mu;
+  static std::map<int, std::vector<float2>> tables;
+  std::lock_guard<std::mutex> lk(mu);
+  std::vector<float2> &t = tables[L];
+  if (t.empty())
+    for (int q = 0; q < L; ++q) {
+      const CS w = q62_turn(q, L);
+      t.push_back(make_float2(float(std::ldexp(double((long long)w.c), -62)), float(std::ldexp(double((long long)-w.s), -62))));
+    }
+  return t.data();
+}
+
 const longlong2 *twiddles(int L) {
   static std::mutex mu;
   static std::map<int, std::vector<longlong2>> tables;
@@ -255,7 +268,7 @@ __global__ void __launch_bounds__(384) k_fx_strided(const __grid_constant__ SArg
     if (t < P) emax[t] = 0;
     __syncthreads();
     // load
-    const double2 *src = d.src[op] + (long long)o * d.in_outer + kz;
+    const double2 *src = static_cast<const double2 *>(d.src[op]) + (long long)o * d.in_outer + kz;
     const int pr = d.pr[op], pk = d.pk[op];
     const bool scaled = (pr | pk) != 0;
     const double kf = pk == 0 ? 1.0 : ((d.inverse && kz == nh) ? 0.0 : (pk == 1 ? double(kz) : double(kz) * double(kz)));
@@ -316,7 +329,7 @@ __global__ void __launch_bounds__(384) k_fx_strided(const __grid_constant__ SArg
       inverse = true;
     }
     // store
-    double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
+    double2 *dst = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + kz;
     const int so = o > nh ? o - n : o;
     for (int l = t >> lgP; l < L; l += step_l) {
       const int i = !d.cut_out ? l : (l <= nh ? l : (l > n ? l - nh : -1));
@@ -342,7 +355,7 @@ __global__ void __launch_bounds__(384) k_fx_strided(const __grid_constant__ SArg
     }
     if (d.inv_lap && kz0 + P >= d.kc) {
       // the kz Nyquist column
-      double2 *z = d.dst[op] + (long long)o * d.out_outer + d.kc;
+      double2 *z = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + d.kc;
       for (int i = t; i < n; i += T) z[(long long)i * d.out_row] = make_double2(0.0, 0.0);
     }
     __syncthreads();
@@ -361,7 +374,7 @@ __global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a)
   const Rows &d = a.r;
   const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
   int *emax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));
-  double *base = d.field[blockIdx.y];
+  double *base = static_cast<double *>(d.field[blockIdx.y]);
   const long long row0 = (long long)blockIdx.x * 2 * P;
   const int h = L >> 1, kc = min(d.kc, h);  // the Nyquist value, if any, is handled apart
   const bool nyq = d.kc > h;
@@ -443,7 +456,7 @@ __global__ void __launch_bounds__(384) k_fx_r2c(const __grid_constant__ RArgs a)
   const Rows &d = a.r;
   const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
   int *emax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));
-  double *base = d.field[blockIdx.y];
+  double *base = static_cast<double *>(d.field[blockIdx.y]);
   const long long row0 = (long long)blockIdx.x * 2 * P;
   if (t < P) emax[t] = 0;
   __syncthreads();
@@ -592,13 +605,13 @@ cudaError_t run_strided(const Strided &s, cudaStream_t st) {
     if (s.inverse && !s.cut_out && !s.truncate) op = s.pad_in ? (p ? FX_OP_INV_PAD : op) : (l->grid ? FX_OP_INV : op);
     else if (!s.inverse && !s.pad_in && single) op = !p ? op : (s.truncate ? FX_OP_TRUNC : (s.cut_out ? FX_OP_CUT : op));
     if (op != FX_OP_PREPARE) {
-      const LArgs a{s.tw, len_bits(*l, FX_STRIDED, !s.inverse, s.inverse || s.truncate), s};
+      const LArgs a{static_cast<const longlong2 *>(s.tw), len_bits(*l, FX_STRIDED, !s.inverse, s.inverse || s.truncate), s};
       return l->fn(op, &a, dim3(unsigned(s.outer * ((s.kc + 7) / 8)), unsigned(s.groups)), st);
     }
   }
   SArgs a;
   if (!fx_plan(s.L, FX_STRIDED, &a.c.p)) return cudaErrorInvalidValue;
-  a.c.tw = s.tw;
+  a.c.tw = static_cast<const longlong2 *>(s.tw);
   a.s = s;
   const int kb = (s.kc + a.c.p.P - 1) / a.c.p.P;
   k_fx_strided<<<dim3(unsigned(s.outer * kb), unsigned(s.groups)), a.c.p.T, a.c.p.smem, st>>>(a);
@@ -611,13 +624,13 @@ static cudaError_t run_rows(const Rows &r, FxKind kind, cudaStream_t st) {
     if (kind == FX_C2R) op = l->padded && r.kc <= r.L / 3 + 1 ? FX_OP_C2R_PAD : (l->grid ? FX_OP_C2R : op);
     else if (l->padded && r.kc <= r.L / 3) op = FX_OP_R2C;
     if (op != FX_OP_PREPARE) {
-      const LRows a{r.tw, len_bits(*l, kind, kind == FX_R2C, kind == FX_C2R), r};
+      const LRows a{static_cast<const longlong2 *>(r.tw), len_bits(*l, kind, kind == FX_R2C, kind == FX_C2R), r};
       return l->fn(op, &a, dim3(unsigned((r.rows + 15) / 16), unsigned(r.count)), st);
     }
   }
   RArgs a;
   if (!fx_plan(r.L, kind, &a.c.p)) return cudaErrorInvalidValue;
-  a.c.tw = r.tw;
+  a.c.tw = static_cast<const longlong2 *>(r.tw);
   a.r = r;
   const long long per = 2 * a.c.p.P;
   const dim3 grid(unsigned((r.rows + per - 1) / per), unsigned(r.count));

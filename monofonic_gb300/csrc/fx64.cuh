@@ -118,6 +118,21 @@ template <long long W> FX_HD long long mulk(long long a) {
   return mulq(a + a, wh, wl);
 }
 template <long long W> FX_HD I2 mulk(I2 a) { return {mulk<W>(a.x), mulk<W>(a.y)}; }
+FX_HD I2 minus_half(I2 a, I2 b) { return {a.x - (b.x >> 1), a.y - (b.y >> 1)}; }
+FX_HD I2 minus_quarter(I2 a, I2 b) { return {a.x - (b.x >> 2), a.y - (b.y >> 2)}; }
+
+// the same DFTs in single precision (fs32.cuh)
+struct F2 {
+  float x, y;
+};
+FX_HD F2 operator+(F2 a, F2 b) { return {a.x + b.x, a.y + b.y}; }
+FX_HD F2 operator-(F2 a, F2 b) { return {a.x - b.x, a.y - b.y}; }
+template <long long W> FX_HD F2 mulk(F2 a) {
+  constexpr float w = float(double(W) * 1.0842021724855044e-19);  // 2^-63
+  return {a.x * w, a.y * w};
+}
+FX_HD F2 minus_half(F2 a, F2 b) { return {a.x - 0.5f * b.x, a.y - 0.5f * b.y}; }
+FX_HD F2 minus_quarter(F2 a, F2 b) { return {a.x - 0.25f * b.x, a.y - 0.25f * b.y}; }
 
 // v exp(-2 pi i NUM / DEN): quarter turns by exchange, an eighth by one
 // constant, the rest by three lifting steps (tan, sin, tan of an angle of at
@@ -142,6 +157,20 @@ template <int NUM, int DEN> FX_HD I2 rotc(I2 v) {
     const long long x = q.x + mulk<t>(q.y);
     const long long y = q.y - mulk<s>(x);
     return {x + mulk<t>(y), y};
+  }
+}
+
+template <int NUM, int DEN> FX_HD F2 rotc(F2 v) {
+  constexpr int n = ((NUM % DEN) + DEN) % DEN;
+  if constexpr (n == 0) return v;
+  else if constexpr (4 * n == DEN) return {v.y, -v.x};
+  else if constexpr (2 * n == DEN) return {-v.x, -v.y};
+  else if constexpr (4 * n == 3 * DEN) return {-v.y, v.x};
+  else {
+    constexpr CS w = q62_turn(n, DEN);
+    constexpr float c = float(double((long long)w.c) * 2.168404344971009e-19),  // 2^-62
+        s = float(double((long long)w.s) * 2.168404344971009e-19);
+    return {v.x * c + v.y * s, v.y * c - v.x * s};
   }
 }
 
@@ -178,13 +207,13 @@ constexpr int radix_split(int R) {
 
 // X[k] = sum_n v[n] exp(-2 pi i n k / R), in place
 template <int R> struct Dft {
-  static FX_HD void run(I2 *v) {
+  template <class V> static FX_HD void run(V *v) {
     constexpr int A = radix_split(R), B = R / A;
-    I2 t[R];
+    V t[R];
     if constexpr (gcd_(A, B) == 1) {
       constexpr int ea = B * inv_mod(B % A, A), eb = A * inv_mod(A % B, B);  // CRT idempotents
       sfor<B>([&](auto b) {
-        I2 c[A];
+        V c[A];
         sfor<A>([&](auto a) { c[a] = v[(B * decltype(a)::value + A * decltype(b)::value) % R]; });
         Dft<A>::run(c);
         sfor<A>([&](auto a) { t[decltype(a)::value * B + decltype(b)::value] = c[a]; });
@@ -197,7 +226,7 @@ template <int R> struct Dft {
       });
     } else {
       sfor<B>([&](auto b) {
-        I2 c[A];
+        V c[A];
         sfor<A>([&](auto a) { c[a] = v[B * decltype(a)::value + decltype(b)::value]; });
         Dft<A>::run(c);
         sfor<A>([&](auto a) {
@@ -212,35 +241,35 @@ template <int R> struct Dft {
   }
 };
 template <> struct Dft<1> {
-  static FX_HD void run(I2 *) {}
+  template <class V> static FX_HD void run(V *) {}
 };
 template <> struct Dft<2> {
-  static FX_HD void run(I2 *v) {
-    const I2 a = v[0], b = v[1];
+  template <class V> static FX_HD void run(V *v) {
+    const V a = v[0], b = v[1];
     v[0] = a + b;
     v[1] = a - b;
   }
 };
 template <> struct Dft<3> {
-  static FX_HD void run(I2 *v) {
+  template <class V> static FX_HD void run(V *v) {
     constexpr long long s = 7987674492471257551LL;  // sin(pi/3) 2^63
-    const I2 t = v[1] + v[2], d = mulk<s>(v[1] - v[2]);
-    const I2 m = {v[0].x - (t.x >> 1), v[0].y - (t.y >> 1)};
+    const V t = v[1] + v[2], d = mulk<s>(v[1] - v[2]);
+    const V m = minus_half(v[0], t);
     v[0] = v[0] + t;
     v[1] = {m.x + d.y, m.y - d.x};
     v[2] = {m.x - d.y, m.y + d.x};
   }
 };
 template <> struct Dft<5> {
-  static FX_HD void run(I2 *v) {
+  template <class V> static FX_HD void run(V *v) {
     constexpr long long c = 5156021714044493573LL;   // sqrt(5)/4 2^63
     constexpr long long s1 = 8771948077865237882LL;  // sin(2 pi/5) 2^63
     constexpr long long s2 = 5421362059670026167LL;  // sin(pi/5) 2^63
-    const I2 t1 = v[1] + v[4], t2 = v[2] + v[3], d1 = v[1] - v[4], d2 = v[2] - v[3];
-    const I2 t = t1 + t2, b = mulk<c>(t1 - t2);
-    const I2 a = {v[0].x - (t.x >> 2), v[0].y - (t.y >> 2)};
-    const I2 m1 = a + b, m2 = a - b;
-    const I2 e1 = mulk<s1>(d1) + mulk<s2>(d2), e2 = mulk<s2>(d1) - mulk<s1>(d2);
+    const V t1 = v[1] + v[4], t2 = v[2] + v[3], d1 = v[1] - v[4], d2 = v[2] - v[3];
+    const V t = t1 + t2, b = mulk<c>(t1 - t2);
+    const V a = minus_quarter(v[0], t);
+    const V m1 = a + b, m2 = a - b;
+    const V e1 = mulk<s1>(d1) + mulk<s2>(d2), e2 = mulk<s2>(d1) - mulk<s1>(d2);
     v[0] = v[0] + t;
     v[1] = {m1.x + e1.y, m1.y - e1.x};
     v[4] = {m1.x - e1.y, m1.y + e1.x};
@@ -249,18 +278,18 @@ template <> struct Dft<5> {
   }
 };
 template <> struct Dft<7> {
-  static FX_HD void run(I2 *v) {
+  template <class V> static FX_HD void run(V *v) {
     // cos and sin of 2 pi j / 7 in Q63, j = 1, 2, 3
     constexpr long long c1 = 5750678403727967667LL, c2 = -2052393359867478633LL, c3 = -8309971062287876938LL;
     constexpr long long s1 = 7211122632928341039LL, s2 = 8992122843167040398LL, s3 = 4001871146622878209LL;
-    const I2 t1 = v[1] + v[6], t2 = v[2] + v[5], t3 = v[3] + v[4];
-    const I2 d1 = v[1] - v[6], d2 = v[2] - v[5], d3 = v[3] - v[4];
-    const I2 m1 = v[0] + mulk<c1>(t1) + mulk<c2>(t2) + mulk<c3>(t3);
-    const I2 m2 = v[0] + mulk<c2>(t1) + mulk<c3>(t2) + mulk<c1>(t3);
-    const I2 m3 = v[0] + mulk<c3>(t1) + mulk<c1>(t2) + mulk<c2>(t3);
-    const I2 e1 = mulk<s1>(d1) + mulk<s2>(d2) + mulk<s3>(d3);
-    const I2 e2 = mulk<s2>(d1) - mulk<s3>(d2) - mulk<s1>(d3);
-    const I2 e3 = mulk<s3>(d1) - mulk<s1>(d2) + mulk<s2>(d3);
+    const V t1 = v[1] + v[6], t2 = v[2] + v[5], t3 = v[3] + v[4];
+    const V d1 = v[1] - v[6], d2 = v[2] - v[5], d3 = v[3] - v[4];
+    const V m1 = v[0] + mulk<c1>(t1) + mulk<c2>(t2) + mulk<c3>(t3);
+    const V m2 = v[0] + mulk<c2>(t1) + mulk<c3>(t2) + mulk<c1>(t3);
+    const V m3 = v[0] + mulk<c3>(t1) + mulk<c1>(t2) + mulk<c2>(t3);
+    const V e1 = mulk<s1>(d1) + mulk<s2>(d2) + mulk<s3>(d3);
+    const V e2 = mulk<s2>(d1) - mulk<s3>(d2) - mulk<s1>(d3);
+    const V e3 = mulk<s3>(d1) - mulk<s1>(d2) + mulk<s2>(d3);
     v[0] = v[0] + t1 + t2 + t3;
     v[1] = {m1.x + e1.y, m1.y - e1.x};
     v[6] = {m1.x - e1.y, m1.y + e1.x};

@@ -30,7 +30,7 @@ cudaError_t prepare_device(int dev);
 // row + kz (complex elements).
 struct Strided {
   int L;                  // transform length
-  const longlong2 *tw;    // its twiddles
+  const void *tw;         // its twiddles on the device (twiddles / twiddles32)
   bool inverse;
   int n;                  // N (the unpadded grid) for padded or cut rows
   bool pad_in;            // rows r < n go to the padded positions of a length-L pencil (else r < L)
@@ -40,8 +40,8 @@ struct Strided {
   // up to 6 outputs in `groups` groups of consecutive ones: a CTA makes the
   // outputs of one group in turn, so that the last may overwrite their source
   int ops, groups, first[7];
-  const double2 *src[6];
-  double2 *dst[6];
+  const void *src[6];
+  void *dst[6];
   // factors of an output's input: (row index)^pr (kz)^pk, signed mode indices
   // with the Nyquist index n / 2 zero where the power is positive
   int pr[6], pk[6];
@@ -52,6 +52,7 @@ struct Strided {
   bool inv_lap;
   const double *rinv;
   double fac;
+  double in_fac;          // single precision: factor of the inputs (0: one); mode and rinv are not read
   // forward transform, rows cut to n (Nyquist zero), factor fac, transformed
   // back: convolve3's truncation between its two products
   bool truncate;
@@ -62,13 +63,22 @@ cudaError_t run_strided(const Strided &s, cudaStream_t st);
 // with their spectra (kz < kc complex values); two rows share a transform.
 struct Rows {
   int L;
-  const longlong2 *tw;
+  const void *tw;
   int kc;                 // kz values of the spectrum (read or written); 2 (kc - 1) == L: with the Nyquist one
   long long rows, pitch;
   int count;              // fields
-  double *field[6];
+  void *field[6];
 };
 cudaError_t run_c2r(const Rows &r, cudaStream_t st);
 cudaError_t run_r2c(const Rows &r, cudaStream_t st);
+
+// The same passes on single-precision fields (fs32.cu), for the lengths that
+// length_supported names
+cudaError_t run_strided32(const Strided &s, cudaStream_t st);
+cudaError_t run_c2r32(const Rows &r, cudaStream_t st);
+cudaError_t run_r2c32(const Rows &r, cudaStream_t st);
+// float2 (cos, -sin)(2 pi t / L), t < L (host memory, kept for the process)
+const float2 *twiddles32(int L);
+cudaError_t prepare_device32(int dev);
 
 }  // namespace fx

@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_inv(const __grid
   const int o = blockIdx.x / kblocks, kz = ((blockIdx.x - o * kblocks) << 3) + pen;
   const bool lv = kz < d.kc;
   for (int op = d.first[blockIdx.y]; op < d.first[blockIdx.y + 1]; ++op) {
-    const double2 *src = d.src[op] + (long long)o * d.in_outer + kz;
+    const double2 *src = static_cast<const double2 *>(d.src[op]) + (long long)o * d.in_outer + kz;
     typename F::template Regs<0> g;
 #pragma unroll
     for (int m = 0; m < F::MU(0); ++m)
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_inv(const __grid
     F::template store<0>(g, sm, pen);
     __syncthreads();
     const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1));
-    double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
+    double2 *dst = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + kz;
     F::template rest<1>(sm, pen, tw, [&](auto &h) {
       constexpr int Q = F::last;
 #pragma unroll
@@ -326,7 +326,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   const int o = blockIdx.x / kblocks, kz0 = (blockIdx.x - o * kblocks) << 3, kz = kz0 + pen;
   const bool lv = kz < d.kc;
   const int op = blockIdx.y;
-  const double2 *src = d.src[op] + (long long)o * d.in_outer + kz;
+  const double2 *src = static_cast<const double2 *>(d.src[op]) + (long long)o * d.in_outer + kz;
   typename F::template Regs<0> g;
 #pragma unroll
   for (int m = 0; m < F::MU(0); ++m)
@@ -359,7 +359,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   F::template store<0>(g, sm, pen);
   __syncthreads();
   const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1));
-  double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
+  double2 *dst = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + kz;
   F::template rest<1>(sm, pen, tw, [&](auto &h) {
     constexpr int Q = F::last, RL = F::R(Q);
     const bool lap = d.inv_lap;
@@ -390,7 +390,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
       }
   });
   if (d.inv_lap && kz0 + 8 >= d.kc) {
-    double2 *z = d.dst[op] + (long long)o * d.out_outer + d.kc;  // the kz Nyquist column
+    double2 *z = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + d.kc;  // the kz Nyquist column
     for (int i = t; i < n; i += F::T) z[(long long)i * d.out_row] = make_double2(0.0, 0.0);
   }
 }
@@ -413,7 +413,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   typename I::template Regs<0> h;
   int em, S;
   {
-    const double2 *src = d.src[op] + (long long)o * d.in_outer + kz;
+    const double2 *src = static_cast<const double2 *>(d.src[op]) + (long long)o * d.in_outer + kz;
     typename F::template Regs<0> g;
 #pragma unroll
     for (int m = 0; m < F::MU(0); ++m)
@@ -482,7 +482,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   __syncthreads();
   S = em - 1022 - a.B + down + 6 * (F::steps - 1);
   const OutScale os = out_scale(em, S);
-  double2 *dst = d.dst[op] + (long long)o * d.out_outer + kz;
+  double2 *dst = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + kz;
   I::template rest<1>(sm, pen, tw, [&](auto &g) {
     constexpr int Q = I::last;
 #pragma unroll
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_c2r_l(const __g
   const int t = threadIdx.x, lane = t & 31, pen = t & 7;
   int *rmax = reinterpret_cast<int *>(sm + L * 8);  // per row
   const Tw3 tw = tw3_of(a.tw, L);
-  double *base = d.field[blockIdx.y];
+  double *base = static_cast<double *>(d.field[blockIdx.y]);
   const long long row0 = (long long)blockIdx.x * 16;
   const int kc = min(d.kc, kmax);
   const bool nyq = !PAD && d.kc > h;
@@ -620,7 +620,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_f
   const int t = threadIdx.x, lane = t & 31, pen = t & 7;
   int *rmax = reinterpret_cast<int *>(sm + L * 8);
   const Tw3 tw = tw3_of(a.tw, L);
-  double *base = d.field[blockIdx.y];
+  double *base = static_cast<double *>(d.field[blockIdx.y]);
   const long long row0 = (long long)blockIdx.x * 16;
 #pragma unroll 1
   for (int q = t >> 5; q < 16; q += F::W) {
