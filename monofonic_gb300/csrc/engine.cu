@@ -18,6 +18,7 @@
 #include <cufft.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -131,7 +132,35 @@ struct mfx_engine {
     int pk[6];
   };
   std::map<int, FFTiles> ff_tuned;  // per grid size: x/y tile, ZSRC3 and ZSRC2 shapes
+  // Status words of the jobs with bounded waits, in page-locked memory that the
+  // device writes on a time-out and the host reads after the stream is idle: a
+  // device word took every wait a blocking copy of its own (7.5 us, a tenth of a
+  // 32^3 pass).  One 64-byte line a job; a job that finds none free has its word
+  // in its arena.
+  static constexpr int kStatusLines = 1024;
+  std::atomic<int> running{0};  // jobs with a run that has not been waited for
+  int *status_host = nullptr;
+  std::vector<int> status_free;
 };
+
+// a free status line, or -1
+static int acquire_status(mfx_engine *eng) {
+  std::lock_guard<std::mutex> lk(eng->mu);
+  if (!eng->status_host) {
+    if (cudaHostAlloc(reinterpret_cast<void **>(&eng->status_host), size_t(mfx_engine::kStatusLines) * 64,
+                      cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      eng->status_host = nullptr;
+      return -1;
+    }
+    for (int q = mfx_engine::kStatusLines - 1; q >= 0; --q) eng->status_free.push_back(q);
+  }
+  if (eng->status_free.empty()) return -1;
+  const int q = eng->status_free.back();
+  eng->status_free.pop_back();
+  return q;
+}
+
 
 struct mfx_job {
   mfx_engine *eng = nullptr;
@@ -153,7 +182,10 @@ struct mfx_job {
   void *fx_twm = nullptr, *fx_twn = nullptr;  // twiddles of M and N
   // of every plain FP64 job (fx::fill_tables)
   double *fx_mode = nullptr, *fx_rinv = nullptr, *fx_root = nullptr;
-  int *dstatus = nullptr;      // device status word: nonzero when a kernel's bounded wait ran out
+  int *dstatus = nullptr;      // status word (device address): nonzero when a kernel's bounded wait ran out
+  bool running = false;        // counted in the engine's running jobs
+  bool shared_gpu = false;     // a server's job: others run beside it
+  int status_line = -1;        // its line of the engine's page-locked words, -1: in the arena
   size_t rsize = 8;
   cudaStream_t stream = nullptr;
   cudaStream_t xfer[4] = {};  // particle downloads, split across copy streams
@@ -537,6 +569,7 @@ static void engine_retain(mfx_engine *eng) {
 
 static void engine_free(mfx_engine *eng) {
   for (auto &p : eng->plan_pool) destroy_plan(p);
+  if (eng->status_host) cudaFreeHost(eng->status_host);
   delete eng;
 }
 
@@ -641,7 +674,7 @@ template <typename R> static int launch_noise(mfx_job *j, int mode, void *out) {
   const int cols = j->N * j->N;
   a.split = noise_split(j->N, num_sm());
   KBEGIN(j);
-  k_noise_phi1<R><<<noise_grid(j->N, a.split), 128, 0, j->stream>>>(a, (typename Cplx<R>::T *)out);
+  launch_pdl(k_noise_phi1<R>, noise_grid(j->N, a.split), 128, 0, j->stream, a, (typename Cplx<R>::T *)out);
   KEND(j, "noise_phi1", j->n_field_bytes + 4.0 * cols + 8.0 * j->d.amp_table_len);
   return MFX_OK;
 }
@@ -770,7 +803,7 @@ template <typename R> static int hessians(mfx_job *j, const void *phi, void **ou
   a.fac = std::pow(1.5, 1.5) / std::sqrt(M3);
   const size_t total = size_t(j->M) * j->M * j->mk;
   KBEGIN(j);
-  k_pad_hessian<R><<<grid_for(total, 256, num_sm()), 256, 0, j->stream>>>(a);
+  launch_pdl(k_pad_hessian<R>, grid_for(total, 256, num_sm()), 256, 0, j->stream, a);
   KEND(j, "pad_hessian", j->n_field_bytes + 6.0 * j->m_field_bytes);
   for (int c = 0; c < 6; ++c) TRY(exec_fft(j, j->m_c2r, out[c], false));
   return MFX_OK;
@@ -789,7 +822,7 @@ template <typename R> static int unpad_invlap(mfx_job *j, void *F, void *out) {
   a.fac = 1.0 / std::sqrt(M3) / rfac_u;
   const size_t total = size_t(j->N) * j->N * j->nk;
   KBEGIN(j);
-  k_unpad_invlap<R><<<grid_for(total, 256, num_sm()), 256, 0, j->stream>>>(a);
+  launch_pdl(k_unpad_invlap<R>, grid_for(total, 256, num_sm()), 256, 0, j->stream, a);
   KEND(j, "unpad_invlap", 2.0 * j->n_field_bytes);
   return MFX_OK;
 }
@@ -892,7 +925,7 @@ static int run_potentials_fused(mfx_job *j) {
     TRY(ff_run(j, ff::FF_ZSRC2, j->ff_pz2, z, "ff_zsrc2", 6 * bC + nout * bC));
   }
   TRY(ff_finish(j, D[0], j->nf[1], 0));
-  if (j->timed) CU(cudaEventRecord(j->ev[2], j->stream));
+  if (j->timed && j->d.lpt_order >= 3) CU(cudaEventRecord(j->ev[2], j->stream));
   if (order >= 3) {
     void *const *CT = &j->ffC[12];
     for (int t = 0; t < 5; ++t) TRY(ff_finish(j, D[1 + t], CT[t], 1));
@@ -1106,21 +1139,21 @@ template <typename R> static int run_potentials_fx(mfx_job *j) {
   s.count = mreal;
   s.out[0] = T[0];
   KBEGIN(j);
-  k_src2<R><<<grid, 256, 0, j->stream>>>(s);
+  launch_pdl(k_src2<R>, grid, 256, 0, j->stream, s);
   KEND(j, "src2", 7.0 * j->m_field_bytes);
   TRY(fx_unpad(j, T, &j->nf[1], 1, ufac));
-  if (j->timed) CU(cudaEventRecord(j->ev[2], j->stream));
+  if (j->timed && j->d.lpt_order >= 3) CU(cudaEventRecord(j->ev[2], j->stream));
   if (j->d.lpt_order < 3) return MFX_OK;
   for (int t = 0; t < 5; ++t) s.out[t] = T[t];
   KBEGIN(j);
-  k_pairs3a<R><<<grid, 256, 0, j->stream>>>(s);
+  launch_pdl(k_pairs3a<R>, grid, 256, 0, j->stream, s);
   KEND(j, "pairs3a", 10.0 * j->m_field_bytes);
   TRY(fx_truncate(j, T, 5, tfac));
   TRY(fx_hessians(j, j->nf[1], H2, j->nh, hfac));
   for (int c = 0; c < 6; ++c) s.h2[c] = H2[c];
   for (int t = 0; t < 5; ++t) s.t[t] = T[t];
   KBEGIN(j);
-  k_src3<R><<<grid, 256, 0, j->stream>>>(s);
+  launch_pdl(k_src3<R>, grid, 256, 0, j->stream, s);
   KEND(j, "src3", 21.0 * j->m_field_bytes);
   return fx_unpad(j, T, &j->nf[2], 4, ufac);
 }
@@ -1152,6 +1185,7 @@ static void tune_fused(mfx_job *j) {
 // Times the fused passes for every admissible pencil-tile shape on the job's
 // own buffers and keeps the fastest per size class (engine-wide cache).
 static int autotune_fused(mfx_job *j) {
+  pdl_enabled() = false;  // launches are timed one by one
   const int N = j->N, M = j->M;
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
@@ -1491,12 +1525,12 @@ template <typename R> static int assemble_stage(mfx_job *j, int mask) {
     if constexpr (sizeof(R) == 8) {
       // one warp per row (i, j), eight of them a CTA
       const unsigned gr = unsigned(std::min<size_t>((size_t(N) * N + 7) / 8, size_t(nsm) * 16));
-      if (a.plt) k_assemble_rows<true><<<gr, 256, 0, j->stream>>>(a);
-      else k_assemble_rows<false><<<gr, 256, 0, j->stream>>>(a);
+      if (a.plt) launch_pdl(k_assemble_rows<true>, gr, 256, 0, j->stream, a);
+      else launch_pdl(k_assemble_rows<false>, gr, 256, 0, j->stream, a);
     } else if (a.plt) {
-      k_assemble<R, true><<<grid_for(total, 256, nsm), 256, 0, j->stream>>>(a);
+      launch_pdl(k_assemble<R, true>, grid_for(total, 256, nsm), 256, 0, j->stream, a);
     } else {
-      k_assemble<R, false><<<grid_for(total, 256, nsm), 256, 0, j->stream>>>(a);
+      launch_pdl(k_assemble<R, false>, grid_for(total, 256, nsm), 256, 0, j->stream, a);
     }
     KEND(j, "assemble", ((order == 1 ? 1.0 : (order == 2 ? 2.0 : 6.0)) + 6.0 * g) * j->n_field_bytes);
     for (int s = 0; s < g; ++s) {
@@ -1522,10 +1556,10 @@ template <typename R> static int assemble_stage(mfx_job *j, int mask) {
       p.id_offset = j->d.id_offset * uint64_t(j->ns) * uint64_t(N3);
       KBEGIN(j);
       const unsigned pg = grid_for(size_t(N) * N * N / 4, 256, nsm);
-      if (p.pos64 && p.vel64) k_particles<R, double, double><<<pg, 256, 0, j->stream>>>(p);
-      else if (p.pos64) k_particles<R, double, float><<<pg, 256, 0, j->stream>>>(p);
-      else if (p.vel64) k_particles<R, float, double><<<pg, 256, 0, j->stream>>>(p);
-      else k_particles<R, float, float><<<pg, 256, 0, j->stream>>>(p);
+      if (p.pos64 && p.vel64) launch_pdl(k_particles<R, double, double>, pg, 256, 0, j->stream, p);
+      else if (p.pos64) launch_pdl(k_particles<R, double, float>, pg, 256, 0, j->stream, p);
+      else if (p.vel64) launch_pdl(k_particles<R, float, double>, pg, 256, 0, j->stream, p);
+      else launch_pdl(k_particles<R, float, float>, pg, 256, 0, j->stream, p);
       KEND(j, "particles", N3 * (6.0 * j->rsize + 3.0 * (p.pos64 ? 8 : 4) + 3.0 * (p.vel64 ? 8 : 4) + (p.id64 ? 8 : 4)));
     }
   }
@@ -1543,7 +1577,24 @@ static void ring_point(mfx_job *j, int s) {
   j->ids = (j->host_q || j->fused) ? nullptr : a;  // the fused read-out writes no device ids
 }
 
+// A run's launches overlap their predecessors' ends (pdl.cuh) while the job has
+// the GPU to itself: its next kernel's waiting CTAs then take only what the
+// current one leaves.  Beside other jobs that room is theirs: a server's burst of
+// requests took 7.1 instead of 6.5 ms with it, three 128^3 jobs in turn 2.73
+// instead of 2.60 ms a round; alone, 32^3 2LPT goes from 77 to 59 us, 64^3 3LPT
+// from 308 to 226 us.
+static void job_idle(mfx_job *j) {
+  if (j->running) j->eng->running.fetch_sub(1, std::memory_order_relaxed);
+  j->running = false;
+}
+static void pdl_rule(mfx_job *j) {
+  if (!j->running) j->eng->running.fetch_add(1, std::memory_order_relaxed);
+  j->running = true;
+  pdl_enabled() = !j->shared_gpu && j->eng->running.load(std::memory_order_relaxed) == 1;
+}
+
 template <typename R> static int run_pipeline(mfx_job *j) {
+  pdl_rule(j);
   const int order = j->d.lpt_order;
   const size_t mreal = size_t(j->M) * j->M * (j->M + 2);
   const int nsm = num_sm();
@@ -1574,11 +1625,11 @@ template <typename R> static int run_pipeline(mfx_job *j) {
     s.out[0] = j->mslot[6];
     s.count = mreal;
     KBEGIN(j);
-    k_src2<R><<<grid_for(mreal, 256, nsm), 256, 0, j->stream>>>(s);
+    launch_pdl(k_src2<R>, grid_for(mreal, 256, nsm), 256, 0, j->stream, s);
     KEND(j, "src2", 7.0 * j->m_field_bytes);
     TRY(unpad_invlap<R>(j, j->mslot[6], j->nf[1]));
   }
-  if (j->timed) CU(cudaEventRecord(j->ev[2], j->stream));
+  if (j->timed && j->d.lpt_order >= 3) CU(cudaEventRecord(j->ev[2], j->stream));
   if (order >= 3) {
     // phi3a: pairwise dealiased triple products (ic_generator.cc:577-586).
     // The five first-pair products are formed in one pass, each is truncated to
@@ -1594,7 +1645,7 @@ template <typename R> static int run_pipeline(mfx_job *j) {
       for (int t = 0; t < 5; ++t) s.out[t] = T[t];
       s.count = mreal;
       KBEGIN(j);
-      k_pairs3a<R><<<grid_for(mreal, 256, nsm), 256, 0, j->stream>>>(s);
+      launch_pdl(k_pairs3a<R>, grid_for(mreal, 256, nsm), 256, 0, j->stream, s);
       KEND(j, "pairs3a", 10.0 * j->m_field_bytes);
     }
     for (int t = 0; t < 5; ++t) {
@@ -1605,7 +1656,7 @@ template <typename R> static int run_pipeline(mfx_job *j) {
       ta.M = j->M;
       ta.fac = (1.0 / std::sqrt(M3) / rfac_u) * rfac_p / std::sqrt(M3);
       KBEGIN(j);
-      k_trunc_repad<R><<<grid_for(size_t(j->M) * j->M * j->mk, 256, nsm), 256, 0, j->stream>>>(ta);
+      launch_pdl(k_trunc_repad<R>, grid_for(size_t(j->M) * j->M * j->mk, 256, nsm), 256, 0, j->stream, ta);
       KEND(j, "trunc_repad", 2.0 * j->m_field_bytes);
       TRY(exec_fft(j, j->m_c2r, T[t], false));
     }
@@ -1619,7 +1670,7 @@ template <typename R> static int run_pipeline(mfx_job *j) {
     for (int q = 0; q < 4; ++q) s.out[q] = T[q];  // phi3 source, A3x, A3y, A3z
     s.count = mreal;
     KBEGIN(j);
-    k_src3<R><<<grid_for(mreal, 256, nsm), 256, 0, j->stream>>>(s);
+    launch_pdl(k_src3<R>, grid_for(mreal, 256, nsm), 256, 0, j->stream, s);
     KEND(j, "src3", 21.0 * j->m_field_bytes);
     TRY(unpad_invlap<R>(j, T[0], j->nf[2]));
     for (int d = 0; d < 3; ++d) TRY(unpad_invlap<R>(j, T[1 + d], j->nf[3 + d]));
@@ -1813,6 +1864,7 @@ static void free_job(mfx_job *j) {
   if (!j) return;
   join_id_fill(j);
   if (j->stream) cudaStreamSynchronize(j->stream);
+  if (j->eng && j->running) j->eng->running.fetch_sub(1, std::memory_order_relaxed);
   if (j->gexec) cudaGraphExecDestroy(j->gexec);
   if (j->graph) cudaGraphDestroy(j->graph);
   if (j->eng) {
@@ -1867,6 +1919,7 @@ static void free_job(mfx_job *j) {
   if (eng) {
     std::lock_guard<std::mutex> lk(eng->mu);
     eng->in_use -= std::min(eng->in_use, j->arena_bytes + size_t(j->ring_sets) * j->ring_set_bytes + j->sp_bytes);
+    if (j->status_line >= 0) eng->status_free.push_back(j->status_line);
   }
   delete j;
   if (eng) engine_release(eng);
@@ -2094,8 +2147,16 @@ static int create_job(mfx_engine *eng, const mfx_job_desc *d, mfx_job **out, int
     if (fe != cudaSuccess) return fail(set_error(MFX_ECUDA, "pruned transform set-up: %s", cudaGetErrorString(fe)));
   }
   p += L.fx;
-  if (j->dstatus && (cudaMemsetAsync(j->dstatus, 0, sizeof(int), j->stream) != cudaSuccess))
-    return fail(set_error(MFX_ECUDA, "status word reset failed"));
+  if (j->dstatus) {
+    j->status_line = acquire_status(eng);
+    if (j->status_line >= 0) {
+      // unified addressing: the mapped word has one address on both sides
+      j->dstatus = eng->status_host + 16 * j->status_line;
+      *static_cast<volatile int *>(j->dstatus) = 0;
+    } else if (cudaMemsetAsync(j->dstatus, 0, sizeof(int), j->stream) != cudaSuccess) {
+      return fail(set_error(MFX_ECUDA, "status word reset failed"));
+    }
+  }
   const int nfield = d->lpt_order == 1 ? 1 : (d->lpt_order == 2 ? 2 : 6);
   j->n_field_bytes = L.n_field;
   j->m_field_bytes = L.m_field;
@@ -2368,8 +2429,10 @@ int mfx_job_assemble(mfx_job *job, int orders_mask) {
   job->ev_next = 0;
   job->prof_recs.clear();
   if (job->fetched) CU(cudaStreamWaitEvent(job->stream, job->fetched, 0));  // downloads of these particles
+  pdl_rule(job);
   TRY(job->fp64 ? assemble_stage<double>(job, orders_mask) : assemble_stage<float>(job, orders_mask));
   CU(cudaStreamSynchronize(job->stream));
+  job_idle(job);
   return MFX_OK;
   GUARD_END
 }
@@ -2561,6 +2624,7 @@ int mfx_job_run_noise(mfx_job *job, int raw) {
   if (!job) return set_error(MFX_EINVAL, "null job");
   CU(cudaSetDevice(job->eng->device));
   job->own_launches = 0;
+  pdl_rule(job);
   int rc = job->fp64 ? make_noise<double>(job, raw ? 0 : 1, job->nf[0])
                      : make_noise<float>(job, raw ? 0 : 1, job->nf[0]);
   if (rc == MFX_OK) {
@@ -2576,7 +2640,8 @@ int mfx_job_run_noise(mfx_job *job, int raw) {
 static int check_status(mfx_job *job) {
   if (!job->dstatus) return MFX_OK;
   int st = 0;
-  CU(cudaMemcpy(&st, job->dstatus, sizeof(int), cudaMemcpyDeviceToHost));
+  if (job->status_line >= 0) st = *static_cast<volatile int *>(job->eng->status_host + 16 * job->status_line);
+  else CU(cudaMemcpy(&st, job->dstatus, sizeof(int), cudaMemcpyDeviceToHost));
   if (st) return set_error(MFX_ETIMEOUT, "a fused-transform kernel timed out waiting for its staged inputs");
   return MFX_OK;
 }
@@ -2586,12 +2651,16 @@ int mfx_job_wait(mfx_job *job, int timeout_ms) {
   if (!job) return set_error(MFX_EINVAL, "null job");
   if (timeout_ms < 0) {
     CU(cudaStreamSynchronize(job->stream));
+    job_idle(job);
     return check_status(job);
   }
   // bounded host-side poll
   for (int waited = 0;; ++waited) {
     cudaError_t e = cudaStreamQuery(job->stream);
-    if (e == cudaSuccess) return check_status(job);
+    if (e == cudaSuccess) {
+      job_idle(job);
+      return check_status(job);
+    }
     if (e != cudaErrorNotReady) return set_error(MFX_ECUDA, "job stream: %s", cudaGetErrorString(e));
     if (waited >= timeout_ms) return set_error(MFX_ETIMEOUT, "job not finished after %d ms", timeout_ms);
     struct timespec ts = {0, 1000000};
@@ -2885,8 +2954,13 @@ int mfx_job_stage_times(mfx_job *job, double *ms, int max_stages) {
   if (cudaStreamSynchronize(job->stream) != cudaSuccess) return set_error(MFX_ECUDA, "sync failed");
   int n = 0;
   for (int s = 0; s < 4 && n < max_stages; ++s) {
+    // below third order the phi2 stage ends where the (empty) phi3 stage would:
+    // one event less between the kernels (about 2 us each)
+    const bool low = job->d.lpt_order < 3;
     float t = 0;
-    if (cudaEventElapsedTime(&t, job->ev[s], job->ev[s + 1]) != cudaSuccess) t = 0;
+    if (!(low && s == 2) &&
+        cudaEventElapsedTime(&t, job->ev[s], job->ev[low && s == 1 ? 3 : s + 1]) != cudaSuccess)
+      t = 0;
     ms[n++] = t;
   }
   return n;
@@ -3237,6 +3311,7 @@ static void setup_loop(mfx_server *s) {
     mfx_job *j = nullptr;
     int rc = create_job(s->eng, &t->d, &j, s->size_priority ? stream_priority_for(t->footprint, s->small_first) : 0);
     std::string err = rc == MFX_OK ? "" : g_last_error;
+    if (rc == MFX_OK) j->shared_gpu = true;
     if (rc == MFX_OK) rc = j->fp64 ? run_pipeline<double>(j) : run_pipeline<float>(j);
     if (rc == MFX_OK && cudaEventRecord(t->done, j->stream) != cudaSuccess) rc = MFX_ECUDA;
     if (rc != MFX_OK && err.empty()) err = g_last_error;

@@ -111,6 +111,7 @@ __device__ __forceinline__ void transform32(const FxPlan &p, const float2 *tw) {
 }
 
 __global__ void __launch_bounds__(512) k_fs_strided(const __grid_constant__ SArgs32 a) {
+  mfx::pdl_begin();
   extern __shared__ __align__(16) F2 fsm[];
   const Strided &d = a.s;
   const float2 *tw = static_cast<const float2 *>(d.tw);
@@ -177,6 +178,7 @@ __global__ void __launch_bounds__(512) k_fs_strided(const __grid_constant__ SArg
 }
 
 __global__ void __launch_bounds__(512) k_fs_c2r_g(const __grid_constant__ RArgs32 a) {
+  mfx::pdl_begin();
   extern __shared__ __align__(16) F2 fsm[];
   const Rows &d = a.r;
   const int L = a.p.L, lgP = a.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
@@ -216,6 +218,7 @@ __global__ void __launch_bounds__(512) k_fs_c2r_g(const __grid_constant__ RArgs3
 }
 
 __global__ void __launch_bounds__(512) k_fs_r2c_g(const __grid_constant__ RArgs32 a) {
+  mfx::pdl_begin();
   extern __shared__ __align__(16) F2 fsm[];
   const Rows &d = a.r;
   const int L = a.p.L, lgP = a.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
@@ -296,7 +299,7 @@ cudaError_t run_strided32(const Strided &s, cudaStream_t st) {
   if (!plan32(s.L, &a.p)) return cudaErrorInvalidValue;
   a.s = s;
   const int kb = (s.kc + a.p.P - 1) / a.p.P;
-  k_fs_strided<<<dim3(unsigned(s.outer * kb), unsigned(s.groups)), a.p.T, a.p.smem, st>>>(a);
+  mfx::launch_pdl(k_fs_strided, dim3(unsigned(s.outer * kb), unsigned(s.groups)), a.p.T, a.p.smem, st, a);
   return cudaGetLastError();
 }
 
@@ -312,8 +315,8 @@ static cudaError_t rows32(const Rows &r, bool inverse, cudaStream_t st) {
   a.r = r;
   const long long per = 2 * a.p.P;
   const dim3 grid(unsigned((r.rows + per - 1) / per), unsigned(r.count));
-  if (inverse) k_fs_c2r_g<<<grid, a.p.T, a.p.smem, st>>>(a);
-  else k_fs_r2c_g<<<grid, a.p.T, a.p.smem, st>>>(a);
+  if (inverse) mfx::launch_pdl(k_fs_c2r_g, grid, a.p.T, a.p.smem, st, a);
+  else mfx::launch_pdl(k_fs_r2c_g, grid, a.p.T, a.p.smem, st, a);
   return cudaGetLastError();
 }
 cudaError_t run_c2r32(const Rows &r, cudaStream_t st) { return rows32(r, true, st); }

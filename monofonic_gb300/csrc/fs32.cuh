@@ -133,6 +133,7 @@ __device__ __forceinline__ float kz_factor(int kz, int n, int pk, double in_fac)
 // inverse transform along x or y; PAD: N rows in, placed at the padded positions
 template <int L, bool PAD>
 __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) k_fs_inv(const __grid_constant__ Strided d) {
+  mfx::pdl_begin();
   using F = Fft32<L, true>;
   extern __shared__ __align__(16) F2 fsm[];
   constexpr int R0 = F::R(0), nb = L / R0, nh = L / 3, n = 2 * nh;
@@ -198,6 +199,7 @@ __device__ __forceinline__ float lap_factor(const Strided &d, int so, int si, in
 
 // forward transform along x or y, the N-grid rows kept (the Nyquist row zero)
 template <int L> __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) k_fs_cut(const __grid_constant__ Strided d) {
+  mfx::pdl_begin();
   using F = Fft32<L, false>;
   extern __shared__ __align__(16) F2 fsm[];
   constexpr int R0 = F::R(0), nb = L / R0, nh = L / 3, n = 2 * nh;
@@ -258,6 +260,7 @@ template <int L> __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) 
 // forward, the N-grid rows kept times fac, and back (in place)
 template <int L>
 __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) k_fs_trunc(const __grid_constant__ Strided d) {
+  mfx::pdl_begin();
   using F = Fft32<L, false>;
   using I = Fft32<L, true>;
   extern __shared__ __align__(16) F2 fsm[];
@@ -323,6 +326,7 @@ __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) k_fs_trunc(const 
 // conj A[k] + i conj B[k]; PAD: at most L/3 + 1 kz values
 template <int L, bool PAD>
 __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) k_fs_c2r(const __grid_constant__ Rows d) {
+  mfx::pdl_begin();
   using F = Fft32<L, true>;
   extern __shared__ __align__(16) F2 fsm[];
   constexpr int h = L / 2, kmax = PAD ? L / 3 + 1 : h, NL = (kmax + 31) / 32;
@@ -404,6 +408,7 @@ __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) k_fs_c2r(const __
 
 // real rows -> spectra of kz < kc <= L/3
 template <int L> __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) k_fs_r2c(const __grid_constant__ Rows d) {
+  mfx::pdl_begin();
   using F = Fft32<L, false>;
   extern __shared__ __align__(16) F2 fsm[];
   constexpr int NL = (L + 31) / 32;
@@ -482,11 +487,11 @@ template <int L, bool PADDED, bool GRID> struct Launch32 {
         limit((const void *)k_fs_r2c<L>);
       }
       done = true;
-      if (op == FS_INV_PAD) k_fs_inv<L, true><<<grid, F::T, F::smem, st>>>(*s);
-      else if (op == FS_CUT) k_fs_cut<L><<<grid, F::T, F::smem, st>>>(*s);
-      else if (op == FS_TRUNC) k_fs_trunc<L><<<grid, F::T, F::smem, st>>>(*s);
-      else if (op == FS_C2R_PAD) k_fs_c2r<L, true><<<grid, F::T, F::smem, st>>>(*r);
-      else if (op == FS_R2C) k_fs_r2c<L><<<grid, F::T, F::smem, st>>>(*r);
+      if (op == FS_INV_PAD) mfx::launch_pdl(k_fs_inv<L, true>, grid, F::T, F::smem, st, *s);
+      else if (op == FS_CUT) mfx::launch_pdl(k_fs_cut<L>, grid, F::T, F::smem, st, *s);
+      else if (op == FS_TRUNC) mfx::launch_pdl(k_fs_trunc<L>, grid, F::T, F::smem, st, *s);
+      else if (op == FS_C2R_PAD) mfx::launch_pdl(k_fs_c2r<L, true>, grid, F::T, F::smem, st, *r);
+      else if (op == FS_R2C) mfx::launch_pdl(k_fs_r2c<L>, grid, F::T, F::smem, st, *r);
       else done = op == FS_PREPARE;
     }
     if constexpr (GRID) {
@@ -495,10 +500,10 @@ template <int L, bool PADDED, bool GRID> struct Launch32 {
         limit((const void *)k_fs_c2r<L, false>);
       }
       if (op == FS_INV) {
-        k_fs_inv<L, false><<<grid, F::T, F::smem, st>>>(*s);
+        mfx::launch_pdl(k_fs_inv<L, false>, grid, F::T, F::smem, st, *s);
         done = true;
       } else if (op == FS_C2R) {
-        k_fs_c2r<L, false><<<grid, F::T, F::smem, st>>>(*r);
+        mfx::launch_pdl(k_fs_c2r<L, false>, grid, F::T, F::smem, st, *r);
         done = true;
       }
     }

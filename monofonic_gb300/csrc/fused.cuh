@@ -38,6 +38,7 @@
 // outputs straight to their destination, so the x/y passes move each element
 // through shared memory once.
 #pragma once
+#include "pdl.cuh"
 #include <stdint.h>
 
 #include <type_traits>
@@ -570,16 +571,25 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-template <int M> __device__ __forceinline__ void load_tw(float2 *tw, const float2 *g) {
+// Twiddles into shared memory, with a barrier.  Every kernel of the passes
+// begins with one of these two: the tables are constant, so they load before
+// the wait for the stream's earlier kernels (pdl.cuh).
+template <int M> __device__ __forceinline__ void load_tw_early(float2 *tw, const float2 *g) {
+  pdl_trigger();
   for (int t = threadIdx.x; t < M; t += blockDim.x) tw[t] = g[t];
   __syncthreads();
+}
+template <int M> __device__ __forceinline__ void load_tw(float2 *tw, const float2 *g) {
+  load_tw_early<M>(tw, g);
+  pdl_wait();
 }
 // the flat table and the per-step tables (TwTab<M>) of the non-PF transforms
 template <int M> __device__ __forceinline__ void load_tw_steps(float2 *tw, const float2 *g) {
   using TT = TwTab<M>;
-  load_tw<M>(tw, g);
+  load_tw_early<M>(tw, g);
   for (int e = threadIdx.x; e < TT::n2 + TT::n3; e += blockDim.x) tw[M + e] = tw[TT::src(e)];
   __syncthreads();
+  pdl_wait();
 }
 
 // ---------------------------------------------------------------------------

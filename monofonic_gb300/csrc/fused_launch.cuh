@@ -111,7 +111,7 @@ template <class K> static unsigned ff_persistent_grid(K kernel, int threads, siz
     static unsigned grid_ = 0;                                                      \
     if (!grid_) grid_ = ff_persistent_grid(kernel, threads, smem, size_t(1) << 40); \
     const unsigned g_ = grid_ < (units) ? grid_ : unsigned(units);                   \
-    kernel<<<g_, threads, smem, stream>>>(args);                                    \
+    launch_pdl(kernel, dim3(g_), unsigned(threads), smem, stream, args);             \
   } while (0)
 
 template <int M, int P> cudaError_t ff_launch_xy(int op, const FArgs &a, cudaStream_t s) {

@@ -254,6 +254,7 @@ struct SArgs {
 };
 
 __global__ void __launch_bounds__(384) k_fx_strided(const __grid_constant__ SArgs a) {
+  mfx::pdl_begin();
   extern __shared__ __align__(16) longlong2 sm[];
   const Strided &d = a.s;
   const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x;
@@ -370,6 +371,7 @@ struct RArgs {
 // spectra -> real rows: rows 2q and 2q + 1 as the real and imaginary part of
 // one pencil, Z[k] = A[k] + i B[k], Z[L - k] = conj A[k] + i conj B[k]
 __global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a) {
+  mfx::pdl_begin();
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
   const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
@@ -452,6 +454,7 @@ __global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a)
 
 // real rows -> spectra of kz < kc, two rows a pencil
 __global__ void __launch_bounds__(384) k_fx_r2c(const __grid_constant__ RArgs a) {
+  mfx::pdl_begin();
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
   const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
@@ -575,7 +578,7 @@ static __global__ void k_fx_tables(int n, double *mode, double *rinv, double *ro
 }
 cudaError_t fill_tables(int n, double *mode, double *rinv, double *root, cudaStream_t st) {
   const int len = int(rinv_len(n));
-  k_fx_tables<<<unsigned(std::min((len + 255) / 256, 608)), 256, 0, st>>>(n, mode, rinv, root, len);
+  mfx::launch_pdl(k_fx_tables, unsigned(std::min((len + 255) / 256, 608)), 256, 0, st, n, mode, rinv, root, len);
   return cudaGetLastError();
 }
 
@@ -614,7 +617,7 @@ cudaError_t run_strided(const Strided &s, cudaStream_t st) {
   a.c.tw = static_cast<const longlong2 *>(s.tw);
   a.s = s;
   const int kb = (s.kc + a.c.p.P - 1) / a.c.p.P;
-  k_fx_strided<<<dim3(unsigned(s.outer * kb), unsigned(s.groups)), a.c.p.T, a.c.p.smem, st>>>(a);
+  mfx::launch_pdl(k_fx_strided, dim3(unsigned(s.outer * kb), unsigned(s.groups)), a.c.p.T, a.c.p.smem, st, a);
   return cudaGetLastError();
 }
 
@@ -634,8 +637,8 @@ static cudaError_t run_rows(const Rows &r, FxKind kind, cudaStream_t st) {
   a.r = r;
   const long long per = 2 * a.c.p.P;
   const dim3 grid(unsigned((r.rows + per - 1) / per), unsigned(r.count));
-  if (kind == FX_C2R) k_fx_c2r<<<grid, a.c.p.T, a.c.p.smem, st>>>(a);
-  else k_fx_r2c<<<grid, a.c.p.T, a.c.p.smem, st>>>(a);
+  if (kind == FX_C2R) mfx::launch_pdl(k_fx_c2r, grid, a.c.p.T, a.c.p.smem, st, a);
+  else mfx::launch_pdl(k_fx_r2c, grid, a.c.p.T, a.c.p.smem, st, a);
   return cudaGetLastError();
 }
 cudaError_t run_c2r(const Rows &r, cudaStream_t st) { return run_rows(r, FX_C2R, st); }

@@ -5,6 +5,8 @@
 
 #include <cstddef>
 
+#include "pdl.cuh"
+
 namespace fx {
 
 // a length the transforms are built for: even, no prime factor above 7

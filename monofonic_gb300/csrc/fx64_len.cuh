@@ -221,6 +221,7 @@ __device__ __forceinline__ int mag(long long b) { return int(b >> 32) & 0x7fffff
 // inverse transform along x or y; PAD: N rows in, placed at the padded positions
 template <int L, bool PAD>
 __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_inv(const __grid_constant__ LArgs a) {
+  mfx::pdl_begin();
   using F = Fft<L, true>;
   extern __shared__ __align__(16) longlong2 sm[];
   const Strided &d = a.s;
@@ -315,6 +316,7 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_inv(const __grid
 // forward transform along x or y, the N-grid rows kept (the Nyquist row zero);
 // inv_lap: times -fac / k^2
 template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_cut(const __grid_constant__ LArgs a) {
+  mfx::pdl_begin();
   using F = Fft<L, false>;
   extern __shared__ __align__(16) longlong2 sm[];
   const Strided &d = a.s;
@@ -397,6 +399,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
 
 // forward, the N-grid rows kept times fac, and back (in place)
 template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_trunc(const __grid_constant__ LArgs a) {
+  mfx::pdl_begin();
   using F = Fft<L, false>;
   using I = Fft<L, true>;
   extern __shared__ __align__(16) longlong2 sm[];
@@ -500,6 +503,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
 // spectra -> real rows (fx64.cu k_fx_c2r); PAD: at most L/3 + 1 kz values
 template <int L, bool PAD>
 __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_c2r_l(const __grid_constant__ LRows a) {
+  mfx::pdl_begin();
   using F = Fft<L, true>;
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
@@ -613,6 +617,7 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_c2r_l(const __g
 
 // real rows -> spectra of kz < kc <= L/3 (fx64.cu k_fx_r2c)
 template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_r2c_l(const __grid_constant__ LRows a) {
+  mfx::pdl_begin();
   using F = Fft<L, false>;
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
@@ -712,11 +717,11 @@ template <int L, bool PADDED, bool GRID> struct Launch {
         limit((const void *)k_fx_r2c_l<L>);
       }
       done = true;
-      if (op == FX_OP_INV_PAD) k_fx_inv<L, true><<<grid, F::T, F::smem, st>>>(*s);
-      else if (op == FX_OP_CUT) k_fx_cut<L><<<grid, F::T, F::smem, st>>>(*s);
-      else if (op == FX_OP_TRUNC) k_fx_trunc<L><<<grid, F::T, F::smem, st>>>(*s);
-      else if (op == FX_OP_C2R_PAD) k_fx_c2r_l<L, true><<<grid, F::T, F::smem, st>>>(*r);
-      else if (op == FX_OP_R2C) k_fx_r2c_l<L><<<grid, F::T, F::smem, st>>>(*r);
+      if (op == FX_OP_INV_PAD) mfx::launch_pdl(k_fx_inv<L, true>, grid, F::T, F::smem, st, *s);
+      else if (op == FX_OP_CUT) mfx::launch_pdl(k_fx_cut<L>, grid, F::T, F::smem, st, *s);
+      else if (op == FX_OP_TRUNC) mfx::launch_pdl(k_fx_trunc<L>, grid, F::T, F::smem, st, *s);
+      else if (op == FX_OP_C2R_PAD) mfx::launch_pdl(k_fx_c2r_l<L, true>, grid, F::T, F::smem, st, *r);
+      else if (op == FX_OP_R2C) mfx::launch_pdl(k_fx_r2c_l<L>, grid, F::T, F::smem, st, *r);
       else done = op == FX_OP_PREPARE;
     }
     if constexpr (GRID) {
@@ -725,10 +730,10 @@ template <int L, bool PADDED, bool GRID> struct Launch {
         limit((const void *)k_fx_c2r_l<L, false>);
       }
       if (op == FX_OP_INV) {
-        k_fx_inv<L, false><<<grid, F::T, F::smem, st>>>(*s);
+        mfx::launch_pdl(k_fx_inv<L, false>, grid, F::T, F::smem, st, *s);
         done = true;
       } else if (op == FX_OP_C2R) {
-        k_fx_c2r_l<L, false><<<grid, F::T, F::smem, st>>>(*r);
+        mfx::launch_pdl(k_fx_c2r_l<L, false>, grid, F::T, F::smem, st, *r);
         done = true;
       }
     }

@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "noise64.cuh"
+#include "pdl.cuh"
 #include "ranlxd.cuh"
 
 namespace mfx {
@@ -219,6 +220,7 @@ __device__ __noinline__ void noise_column_redraw(const NoiseArgs &a, typename Cp
 // FP32 form 32^3 24.8 -> 10.9 us, 64^3 39.4 -> 19.3 us; 256^3 191 -> 157 us.
 template <typename R>
 __global__ void __launch_bounds__(128) k_noise_phi1(NoiseArgs a, typename Cplx<R>::T *out) {
+  pdl_begin();
   const int N = a.N, nh = N >> 1, nk = nh + 1;
   const int warp = int(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)), part = warp % a.split;
   const int col = (warp / a.split) * 32 + int(threadIdx.x & 31);
@@ -265,6 +267,7 @@ struct PadArgs {
 };
 
 template <typename R> __global__ void __launch_bounds__(256) k_pad_hessian(PadArgs a) {
+  pdl_begin();
   using C = typename Cplx<R>::T;
   const int N = a.N, nh = N >> 1, nk = nh + 1, M = a.M, mk = (M >> 1) + 1;
   const size_t total = size_t(M) * M * mk;
@@ -314,6 +317,7 @@ struct SrcArgs {
 // phi(2) source, ic_generator.cc:530-534:
 //   xx (yy + zz) + yy zz - xy^2 - xz^2 - yz^2
 template <typename R> __global__ void __launch_bounds__(256) k_src2(SrcArgs a) {
+  pdl_begin();
   const R *H[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) H[c] = reinterpret_cast<const R *>(a.h1[c]);
@@ -335,6 +339,7 @@ template <typename R> __global__ void __launch_bounds__(256) k_src2(SrcArgs a) {
 // convolve3 = convolve2(convolve2(a, b), c), convolution.hh:525-532):
 //   xx*yy, xy*xz, yz*yz, xz*xz, xy*xy   -> out[0..4]
 template <typename R> __global__ void __launch_bounds__(256) k_pairs3a(SrcArgs a) {
+  pdl_begin();
   const R *H[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) H[c] = reinterpret_cast<const R *>(a.h1[c]);
@@ -358,6 +363,7 @@ template <typename R> __global__ void __launch_bounds__(256) k_pairs3a(SrcArgs a
 // out[0] = phi3 source, out[1..3] = A3 sources.  Outputs may alias t[] slots
 // (each element is read before it is written by the same thread).
 template <typename R> __global__ void __launch_bounds__(256) k_src3(SrcArgs a) {
+  pdl_begin();
   const R c57 = R(-5.0 / 7.0), c107 = R(10.0 / 7.0);
   for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < a.count;
        q += size_t(gridDim.x) * blockDim.x) {
@@ -414,6 +420,7 @@ struct UnpadArgs {
 };
 
 template <typename R> __global__ void __launch_bounds__(256) k_unpad_invlap(UnpadArgs a) {
+  pdl_begin();
   using C = typename Cplx<R>::T;
   const int N = a.N, nh = N >> 1, nk = nh + 1, M = a.M, mk = (M >> 1) + 1;
   const size_t total = size_t(N) * N * nk;
@@ -447,6 +454,7 @@ struct TruncArgs {
 };
 
 template <typename R> __global__ void __launch_bounds__(256) k_trunc_repad(TruncArgs a) {
+  pdl_begin();
   using C = typename Cplx<R>::T;
   const int N = a.N, nh = N >> 1, M = a.M, mk = (M >> 1) + 1;
   const size_t total = size_t(M) * M * mk;
@@ -763,6 +771,7 @@ __device__ __forceinline__ void lattice_phase(const AsmArgs &a, int s, int i, in
 
 template <typename R, bool PLT>
 __global__ void __launch_bounds__(256) k_assemble(AsmArgs a) {
+  pdl_begin();
   using C = typename Cplx<R>::T;
   const int N = a.N, nh = N >> 1, nk = nh + 1;
   const size_t total = size_t(N) * N * nk;
@@ -833,6 +842,7 @@ __device__ __forceinline__ void asm_gradient(double Dr, double Dt, double Dp, do
 }
 
 template <bool PLT> __global__ void __launch_bounds__(256) k_assemble_rows(const __grid_constant__ AsmArgs a) {
+  pdl_begin();
   __shared__ double tab[PLT ? 8 : 1][PLT ? 4 : 1][PLT ? 34 : 1];
   const int N = a.N, nh = N >> 1, nk = nh + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const size_t TS = size_t(64) * 64 * 33;
@@ -1126,6 +1136,7 @@ __device__ __forceinline__ void store6(float *o, const double *v) {
 // store is a 16-byte vector store and a warp writes one contiguous run.
 template <typename R, typename PosT, typename VelT>
 __global__ void __launch_bounds__(256) k_particles(PartArgs a) {
+  pdl_begin();
   const int N = a.N;
   const size_t n3 = size_t(N) * N * N, nq = n3 / 4;
   const size_t rowp = size_t(N + 2);
