@@ -1,5 +1,5 @@
 // Single-precision pruned transforms (fs32.cuh): lengths without an instance
-// (run-time radices up to 16) and the launches.
+// (run-time radices up to 12) and the launches.
 #include "fs32.cuh"
 
 #include <algorithm>
@@ -103,9 +103,6 @@ __device__ __forceinline__ void transform32(const FxPlan &p, const float2 *tw) {
       case 9: step32<9>(tw, L, lgP, NS, mg); break;
       case 10: step32<10>(tw, L, lgP, NS, mg); break;
       case 12: step32<12>(tw, L, lgP, NS, mg); break;
-      case 14: step32<14>(tw, L, lgP, NS, mg); break;
-      case 15: step32<15>(tw, L, lgP, NS, mg); break;
-      case 16: step32<16>(tw, L, lgP, NS, mg); break;
     }
   }
 }
@@ -255,7 +252,39 @@ struct Len32Entry {
 };
 #define FS_LENGTHS(X)                                                                                              \
   X(16, false, true) X(24, true, true) X(32, false, true) X(48, true, true) X(64, false, true) X(96, true, true)    \
-  X(128, false, true) X(192, true, true) X(256, false, true) X(384, true, true) X(512, false, true) X(768, true, true)
+  X(128, false, true) X(192, true, true) X(256, false, true) X(384, true, true) X(512, false, true) X(768, true, true) \
+  X(56, false, true) \
+  X(60, false, true) \
+  X(72, true, true) \
+  X(80, false, true) \
+  X(84, true, true) \
+  X(90, true, false) \
+  X(100, false, true) \
+  X(108, true, true) \
+  X(112, false, true) \
+  X(120, true, true) \
+  X(126, true, false) \
+  X(140, false, true) \
+  X(144, true, true) \
+  X(150, true, false) \
+  X(160, false, true) \
+  X(162, true, false) \
+  X(168, true, true) \
+  X(180, true, true) \
+  X(196, false, true) \
+  X(200, false, true) \
+  X(210, true, false) \
+  X(216, true, true) \
+  X(224, false, true) \
+  X(240, true, true) \
+  X(252, true, true) \
+  X(270, true, false) \
+  X(294, true, false) \
+  X(300, true, false) \
+  X(324, true, false) \
+  X(336, true, false) \
+  X(360, true, false) \
+  X(378, true, false)
 #define FS_EXTERN(L, P, G) extern template struct Launch32<L, P, G>;
 FS_LENGTHS(FS_EXTERN)
 #define FS_ENTRY(L, P, G) {L, P, G, Launch32<L, P, G>::run},

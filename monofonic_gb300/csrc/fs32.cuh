@@ -36,6 +36,38 @@ FS_LEN(256, 2, 16, 16, 1, 256, 3)
 FS_LEN(384, 2, 16, 24, 1, 384, 2)
 FS_LEN(512, 3, 8, 8, 8, 512, 2)
 FS_LEN(768, 3, 8, 8, 12, 512, 2)
+FS_LEN(56, 2, 7, 8, 1, 128, 6)
+FS_LEN(60, 2, 10, 6, 1, 160, 5)
+FS_LEN(80, 2, 8, 10, 1, 160, 5)
+FS_LEN(84, 2, 7, 12, 1, 192, 4)
+FS_LEN(90, 2, 10, 9, 1, 160, 5)
+FS_LEN(100, 2, 10, 10, 1, 160, 5)
+FS_LEN(108, 2, 9, 12, 1, 192, 4)
+FS_LEN(112, 2, 8, 14, 1, 224, 3)
+FS_LEN(120, 2, 10, 12, 1, 192, 4)
+FS_LEN(126, 2, 14, 9, 1, 224, 3)
+FS_LEN(140, 2, 10, 14, 1, 224, 3)
+FS_LEN(150, 2, 10, 15, 1, 256, 3)
+FS_LEN(160, 2, 10, 16, 1, 256, 3)
+FS_LEN(162, 2, 9, 18, 1, 288, 2)
+FS_LEN(168, 2, 14, 12, 1, 224, 3)
+FS_LEN(180, 2, 15, 12, 1, 256, 3)
+FS_LEN(196, 2, 14, 14, 1, 224, 3)
+FS_LEN(200, 2, 10, 20, 1, 320, 2)
+FS_LEN(210, 2, 14, 15, 1, 256, 3)
+FS_LEN(216, 2, 12, 18, 1, 288, 2)
+FS_LEN(224, 2, 14, 16, 1, 256, 3)
+FS_LEN(240, 2, 16, 15, 1, 256, 3)
+FS_LEN(252, 2, 14, 18, 1, 288, 2)
+FS_LEN(270, 2, 15, 18, 1, 288, 2)
+FS_LEN(294, 2, 14, 21, 1, 352, 2)
+FS_LEN(300, 2, 20, 15, 1, 320, 2)
+FS_LEN(324, 2, 18, 18, 1, 288, 2)
+FS_LEN(336, 2, 14, 24, 1, 384, 2)
+FS_LEN(360, 2, 20, 18, 1, 320, 2)
+FS_LEN(378, 2, 18, 21, 1, 352, 2)
+FS_LEN(72, 2, 8, 9, 1, 160, 5)
+FS_LEN(144, 2, 12, 12, 1, 192, 4)
 #undef FS_LEN
 
 __device__ __forceinline__ F2 ld(const float2 *p) {

@@ -31,7 +31,7 @@ namespace fx {
 // plans
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int kRadices[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+constexpr int kRadices[] = {12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
 constexpr int kSmemMax = 220 * 1024;
 
 // rough cost of a point: real multiplications (three products each, measured
@@ -41,8 +41,7 @@ double radix_cost(int R) {
     case 2: case 4: return 0.0;
     case 3: return 0.67; case 5: return 2.0; case 6: return 0.67; case 7: return 5.1;
     case 8: return 0.5; case 9: return 2.0; case 10: return 2.0; case 12: return 0.67;
-    case 14: return 5.1; case 15: return 2.67; case 16: return 1.25; case 18: return 2.0;
-    case 20: return 2.0; default: return 1.17;  // 24
+    default: return 0.0;
   }
 }
 
@@ -180,6 +179,7 @@ __device__ __noinline__ void step(const longlong2 *tw, int L, int lgP, int NS, u
   const int T = blockDim.x, t = threadIdx.x;
   const int nb = L / R, items = nb << lgP;
   const int pen = t & ((1 << lgP) - 1);
+  const Tw3 t3 = tw3_of(tw, L);
   I2 v[MU][R];
   int jn[MU];
 #pragma unroll
@@ -198,8 +198,8 @@ __device__ __noinline__ void step(const longlong2 *tw, int L, int lgP, int NS, u
         if (raw) {
 #pragma unroll
           for (int r = 0; r < R; ++r) {
-            v[m][r].x = to_fixed(__longlong_as_double(v[m][r].x), sh);
-            v[m][r].y = to_fixed(__longlong_as_double(v[m][r].y), sh);
+            v[m][r].x = to_fixed_p(v[m][r].x, sh);
+            v[m][r].y = to_fixed_p(v[m][r].y, sh);
           }
         }
       } else {
@@ -208,7 +208,7 @@ __device__ __noinline__ void step(const longlong2 *tw, int L, int lgP, int NS, u
         const int inc = lo * (nb / NS);  // lo L / (NS R)
         v[m][0] = eighth(v[m][0]);
 #pragma unroll
-        for (int r = 1; r < R; ++r) v[m][r] = twiddle8(v[m][r], __ldg(&tw[r * inc]));
+        for (int r = 1; r < R; ++r) v[m][r] = twiddle8(v[m][r], t3, r * inc);
       }
       Dft<R>::run(v[m]);
     }
@@ -241,9 +241,6 @@ __device__ __forceinline__ void transform(const Core &c, bool raw, int sh) {
       case 9: step<9>(c.tw, L, lgP, NS, mg, rw, sh); break;
       case 10: step<10>(c.tw, L, lgP, NS, mg, rw, sh); break;
       case 12: step<12>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 14: step<14>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 15: step<15>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 16: step<16>(c.tw, L, lgP, NS, mg, rw, sh); break;
     }
   }
 }
@@ -286,17 +283,16 @@ __global__ void __launch_bounds__(384) k_fx_strided(const __grid_constant__ SArg
           v.y *= f;
         }
       }
-      em = max(em, max(dbl_exponent(v.x), dbl_exponent(v.y)));
+      em = max(em, max(mag(__double_as_longlong(v.x)), mag(__double_as_longlong(v.y))));
       sm[slot(l, pen, lgP)] = d.inverse ? make_longlong2(__double_as_longlong(v.y), __double_as_longlong(v.x))
                                         : make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
     }
     for (int off = P; off < 32; off <<= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, off));
     if ((t & 31) < P) atomicMax(&emax[pen], em);
     __syncthreads();
-    em = emax[pen];
-    bool bad = em == 2047;
+    em = emax[pen] >> 20;
     int S = em - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1);
-    transform(a.c, true, em + 63 - a.c.p.B);
+    transform(a.c, true, shift_of(em, a.c.p.B));
     bool inverse = d.inverse;
     if (d.truncate) {
       // keep the N-grid modes, bring the largest back below 2^B, swap for the
@@ -332,12 +328,12 @@ __global__ void __launch_bounds__(384) k_fx_strided(const __grid_constant__ SArg
     // store
     double2 *dst = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + kz;
     const int so = o > nh ? o - n : o;
+    const OutScale os = out_scale(em, S);
     for (int l = t >> lgP; l < L; l += step_l) {
       const int i = !d.cut_out ? l : (l <= nh ? l : (l > n ? l - nh : -1));
       if (i < 0 || !live) continue;
       const longlong2 w = sm[slot(l, pen, lgP)];
-      double2 v = make_double2(to_double(w.x, S), to_double(w.y, S));
-      if (bad) v = make_double2(nan_of(), nan_of());
+      double2 v = make_double2(to_double_p(w.x, os), to_double_p(w.y, os));
       if (inverse) v = make_double2(v.y, v.x);
       if (d.cut_out) {
         if (i == nh || (d.inv_lap && (o == nh || (o | i | kz) == 0))) {
@@ -395,16 +391,16 @@ __global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a)
       double2 v = live ? src[k] : make_double2(0.0, 0.0);
       if (k == 0) {
         // only the real part of the k = 0 (and the Nyquist) value is used
-        em = max(em, dbl_exponent(v.x));
+        em = max(em, mag(__double_as_longlong(v.x)));
         reinterpret_cast<double *>(&sm[slot(0, pen, lgP)])[second] = v.x;
       } else {
-        em = max(em, max(dbl_exponent(v.x), dbl_exponent(v.y)));
+        em = max(em, max(mag(__double_as_longlong(v.x)), mag(__double_as_longlong(v.y))));
         sm[slot(second ? L - k : k, pen, lgP)] = make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
       }
     }
     if (nyq && lane == 0) {
       const double v = live ? src[h].x : 0.0;
-      em = max(em, dbl_exponent(v));
+      em = max(em, mag(__double_as_longlong(v)));
       reinterpret_cast<double *>(&sm[slot(h, pen, lgP)])[second] = v;
     }
     em = __reduce_max_sync(0xffffffffu, unsigned(em));
@@ -414,25 +410,25 @@ __global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a)
   {
     // Z of both rows in fixed point, real and imaginary part exchanged (the
     // inverse transform)
-    const int pen = t & (P - 1), sh = emax[pen] + 63 - a.c.p.B;
+    const int pen = t & (P - 1), sh = shift_of(emax[pen] >> 20, a.c.p.B);
     for (int k = t >> lgP; k < kc; k += T >> lgP) {
       longlong2 &wa = sm[slot(k, pen, lgP)];
       const longlong2 va = wa;
-      const long long ax = to_fixed(__longlong_as_double(va.x), sh), ay = to_fixed(__longlong_as_double(va.y), sh);
+      const long long ax = to_fixed_p(va.x, sh), ay = to_fixed_p(va.y, sh);
       if (k == 0) {
         wa = make_longlong2(ay, ax);
         continue;
       }
       longlong2 &wb = sm[slot(L - k, pen, lgP)];
       const longlong2 vb = wb;
-      const long long bx = to_fixed(__longlong_as_double(vb.x), sh), by = to_fixed(__longlong_as_double(vb.y), sh);
+      const long long bx = to_fixed_p(vb.x, sh), by = to_fixed_p(vb.y, sh);
       wa = make_longlong2(ay + bx, ax - by);
       wb = make_longlong2(bx - ay, ax + by);
     }
     if (nyq && t < P) {
       longlong2 &w = sm[slot(h, t, lgP)];
       const longlong2 v = w;
-      w = make_longlong2(to_fixed(__longlong_as_double(v.y), sh), to_fixed(__longlong_as_double(v.x), sh));
+      w = make_longlong2(to_fixed_p(v.y, sh), to_fixed_p(v.x, sh));
     }
   }
   __syncthreads();
@@ -442,13 +438,10 @@ __global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a)
     if (row >= d.rows) break;
     double *dst = base + row * d.pitch;
     const int pen = q >> 1, second = q & 1;
-    const int S = emax[pen] - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1);
-    const bool bad = emax[pen] == 2047;
-    for (int e = lane; e < L; e += 32) {
-      // exchanged again: the first row is the imaginary part
-      const long long v = reinterpret_cast<const long long *>(&sm[slot(e, pen, lgP)])[1 - second];
-      dst[e] = bad ? nan_of() : to_double(v, S);
-    }
+    const int em = emax[pen] >> 20;
+    const OutScale os = out_scale(em, em - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1));
+    for (int e = lane; e < L; e += 32)  // exchanged again: the first row is the imaginary part
+      dst[e] = to_double_p(reinterpret_cast<const long long *>(&sm[slot(e, pen, lgP)])[1 - second], os);
   }
 }
 
@@ -472,14 +465,14 @@ __global__ void __launch_bounds__(384) k_fx_r2c(const __grid_constant__ RArgs a)
 #pragma unroll 8
     for (int e = lane; e < L; e += 32) {
       const double v = live ? src[e] : 0.0;
-      em = max(em, dbl_exponent(v));
+      em = max(em, mag(__double_as_longlong(v)));
       reinterpret_cast<double *>(&sm[slot(e, pen, lgP)])[second] = v;
     }
     em = __reduce_max_sync(0xffffffffu, unsigned(em));
     if (lane == 0) atomicMax(&emax[pen], em);
   }
   __syncthreads();
-  transform(a.c, true, emax[t & (P - 1)] + 63 - a.c.p.B);
+  transform(a.c, true, shift_of(emax[t & (P - 1)] >> 20, a.c.p.B));
   const int kc = d.kc;
   for (int q = t >> 5; q < 2 * P; q += T >> 5) {
     const long long row = row0 + q;
@@ -487,13 +480,13 @@ __global__ void __launch_bounds__(384) k_fx_r2c(const __grid_constant__ RArgs a)
     double2 *dst = reinterpret_cast<double2 *>(base + row * d.pitch);
     const int pen = q >> 1, second = q & 1;
     // the sums below are twice the spectra
-    const int S = emax[pen] - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1) - 1;
-    const bool bad = emax[pen] == 2047;
+    const int em = emax[pen] >> 20;
+    const OutScale os = out_scale(em, em - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1) - 1);
     for (int k = lane; k < kc; k += 32) {
       const longlong2 u = sm[slot(k, pen, lgP)], w = sm[slot(k ? L - k : 0, pen, lgP)];
       // A = (Z[k] + conj Z[L-k]) / 2, B = (Z[k] - conj Z[L-k]) / 2i
       const long long x = second ? u.y + w.y : u.x + w.x, y = second ? w.x - u.x : u.y - w.y;
-      dst[k] = bad ? make_double2(nan_of(), nan_of()) : make_double2(to_double(x, S), to_double(y, S));
+      dst[k] = make_double2(to_double_p(x, os), to_double_p(y, os));
     }
   }
 }
@@ -514,10 +507,10 @@ extern template struct Launch<24, true, true>;
 extern template struct Launch<32, false, true>;
 extern template struct Launch<48, true, true>;
 extern template struct Launch<64, false, true>;
-extern template struct Launch<72, true, false>;
+extern template struct Launch<72, true, true>;
 extern template struct Launch<96, true, true>;
 extern template struct Launch<128, false, true>;
-extern template struct Launch<144, true, false>;
+extern template struct Launch<144, true, true>;
 extern template struct Launch<192, true, true>;
 extern template struct Launch<256, false, true>;
 extern template struct Launch<288, true, false>;
@@ -526,6 +519,36 @@ extern template struct Launch<512, false, true>;
 extern template struct Launch<576, true, false>;
 extern template struct Launch<768, true, true>;
 extern template struct Launch<1152, true, false>;
+extern template struct Launch<56, false, true>;
+extern template struct Launch<60, false, true>;
+extern template struct Launch<80, false, true>;
+extern template struct Launch<84, true, true>;
+extern template struct Launch<90, true, false>;
+extern template struct Launch<100, false, true>;
+extern template struct Launch<108, true, true>;
+extern template struct Launch<112, false, true>;
+extern template struct Launch<120, true, true>;
+extern template struct Launch<126, true, false>;
+extern template struct Launch<140, false, true>;
+extern template struct Launch<150, true, false>;
+extern template struct Launch<160, false, true>;
+extern template struct Launch<162, true, false>;
+extern template struct Launch<168, true, true>;
+extern template struct Launch<180, true, true>;
+extern template struct Launch<196, false, true>;
+extern template struct Launch<200, false, true>;
+extern template struct Launch<210, true, false>;
+extern template struct Launch<216, true, true>;
+extern template struct Launch<224, false, true>;
+extern template struct Launch<240, true, true>;
+extern template struct Launch<252, true, true>;
+extern template struct Launch<270, true, false>;
+extern template struct Launch<294, true, false>;
+extern template struct Launch<300, true, false>;
+extern template struct Launch<324, true, false>;
+extern template struct Launch<336, true, false>;
+extern template struct Launch<360, true, false>;
+extern template struct Launch<378, true, false>;
 template <int L, bool PADDED, bool GRID> static LenEntry entry() {
   return {L, PADDED, GRID, Launch<L, PADDED, GRID>::run, Len<L>::steps, {Len<L>::R(0), Len<L>::R(1), Len<L>::R(2)}};
 }
@@ -534,10 +557,10 @@ static const LenEntry kLens[] = {entry<16, false, true>(),
                                  entry<32, false, true>(),
                                  entry<48, true, true>(),
                                  entry<64, false, true>(),
-                                 entry<72, true, false>(),
+                                 entry<72, true, true>(),
                                  entry<96, true, true>(),
                                  entry<128, false, true>(),
-                                 entry<144, true, false>(),
+                                 entry<144, true, true>(),
                                  entry<192, true, true>(),
                                  entry<256, false, true>(),
                                  entry<288, true, false>(),
@@ -545,7 +568,37 @@ static const LenEntry kLens[] = {entry<16, false, true>(),
                                  entry<512, false, true>(),
                                  entry<576, true, false>(),
                                  entry<768, true, true>(),
-                                 entry<1152, true, false>()};
+                                 entry<1152, true, false>(),
+                                 entry<56, false, true>(),
+                                 entry<60, false, true>(),
+                                 entry<80, false, true>(),
+                                 entry<84, true, true>(),
+                                 entry<90, true, false>(),
+                                 entry<100, false, true>(),
+                                 entry<108, true, true>(),
+                                 entry<112, false, true>(),
+                                 entry<120, true, true>(),
+                                 entry<126, true, false>(),
+                                 entry<140, false, true>(),
+                                 entry<150, true, false>(),
+                                 entry<160, false, true>(),
+                                 entry<162, true, false>(),
+                                 entry<168, true, true>(),
+                                 entry<180, true, true>(),
+                                 entry<196, false, true>(),
+                                 entry<200, false, true>(),
+                                 entry<210, true, false>(),
+                                 entry<216, true, true>(),
+                                 entry<224, false, true>(),
+                                 entry<240, true, true>(),
+                                 entry<252, true, true>(),
+                                 entry<270, true, false>(),
+                                 entry<294, true, false>(),
+                                 entry<300, true, false>(),
+                                 entry<324, true, false>(),
+                                 entry<336, true, false>(),
+                                 entry<360, true, false>(),
+                                 entry<378, true, false>()};
 static const LenEntry *find_len(int L) {
   for (const LenEntry &e : kLens)
     if (e.L == L) return &e;

@@ -200,6 +200,7 @@ constexpr int radix_split(int R) {
     case 16: return 4;
     case 18: return 2;
     case 20: return 4;
+    case 21: return 3;
     case 24: return 3;
     default: return 1;  // prime
   }
@@ -300,31 +301,9 @@ template <> struct Dft<7> {
   }
 };
 
-// v w / 8 for the table entry w = (cos, -sin) 2^61 of an angle: three products
-FX_HD I2 twiddle8(I2 v, longlong2 w) {
-  const long long k = mulq(v.x + v.y, w.x);
-  return {k - mulq(v.y, w.y + w.x), k + mulq(v.x, w.y - w.x)};
-}
 // v / 8, rounded (the element that a step's twiddles leave alone)
 FX_HD I2 eighth(I2 v) { return {(v.x + 4) >> 3, (v.y + 4) >> 3}; }
 
-// bits of a double -> fixed point; sh = e + 63 - B with e the biased exponent
-// of the pencil's largest component (subnormals count as zero)
-FX_HD long long to_fixed(double v, int sh) {
-  long long b;
-#ifdef __CUDA_ARCH__
-  b = __double_as_longlong(v);
-#else
-  __builtin_memcpy(&b, &v, 8);
-#endif
-  const int ex = int(b >> 52) & 0x7ff;
-  int d = sh - ex;
-  d = d > 63 ? 63 : d;
-  long long m = ((b & 0xfffffffffffffLL) | 0x10000000000000LL) << 10;
-  m = ex == 0 ? 0 : m >> d;
-  const long long sg = b >> 63;
-  return (m ^ sg) - sg;
-}
 // v 2^S -> double, rounded to nearest; S + 1086 is the biased exponent of bit 63
 FX_HD double to_double(long long v, int S) {
   const long long sg = v >> 63;

@@ -8,6 +8,6 @@ template struct Launch<24, true, true>;
 template struct Launch<32, false, true>;
 template struct Launch<48, true, true>;
 template struct Launch<64, false, true>;
-template struct Launch<72, true, false>;
+template struct Launch<72, true, true>;
 template struct Launch<96, true, true>;
 }  // namespace fx

@@ -4,7 +4,7 @@
 
 namespace fx {
 template struct Launch<128, false, true>;
-template struct Launch<144, true, false>;
+template struct Launch<144, true, true>;
 template struct Launch<192, true, true>;
 template struct Launch<256, false, true>;
 }  // namespace fx

@@ -117,3 +117,21 @@ def test_zero_field_gives_the_lattice(mfxlib, engine):
     want = np.stack(np.meshgrid(q, q, q, indexing="ij"), -1).reshape(-1, 3)
     assert np.array_equal(pos, want) and not vel.any()
     j.close()
+
+
+# every further instance: both forms against cuFFT, order 3 where it is quick
+@pytest.mark.parametrize("n", [56, 60, 72, 80, 84, 100, 108, 112, 120, 140, 144, 160, 168, 180, 196, 200, 216, 224,
+                               240, 252])
+def test_further_instances_match_cufft_route(mfxlib, engine, n, monkeypatch):
+    order = 3 if n <= 144 else 2
+    c = Case(mfxlib, n, 300.0, 24.0, order, 6, lattice=1)
+    for prec, tol in ((mfxlib.FP64, TOL), (mfxlib.FP32C, 5e-6)):
+        out = []
+        for env in ("1", "0"):
+            monkeypatch.setenv("MFX_FUSED", env)
+            j = c.job(mfxlib, engine, precision=prec)
+            j.run()
+            out.append(fields_of(mfxlib, j, order) + [j.particles()[1].astype(np.float64)])
+            j.close()
+        for a, b in zip(*out):
+            assert rel_l2(a, b) < tol
