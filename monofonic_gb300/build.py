@@ -57,9 +57,8 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
     inc = ["-I", str(ROOT / "include"), "-I", str(PKG / "csrc"), "-I", str(PKG / "host")]
     jobs = []
     objs = []
-    # the longest compiles first: the run-time radix kernels, the engine, the
-    # long padded lengths
-    first = ["fx64", "fs32", "engine", "ff_m1152", "ff_m1536", "fx64_len_d", "fx64_len_c"]
+    # the longest compiles first
+    first = ["fs32_len", "fs32_len2", "fs32_len3", "fx64_len_d", "fx64_len_c", "engine", "ff_m1152", "ff_m1536"]
     cu.sort(key=lambda s: first.index(s.stem) if s.stem in first else len(first))
     for s in cu:
         o = BUILD / "obj" / (s.stem + ".cu.o")

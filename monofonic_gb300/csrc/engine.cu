@@ -430,13 +430,16 @@ static bool fused_supported(const mfx_job_desc *d) {
 // grids use cuFFT.  MFX_FUSED=0 sends all of them through cuFFT.  One padded D2Z
 // at 384^3 took cuFFT 7.15 ms, the three fixed-point passes 1.6 ms without any
 // pruning, at 96^3 0.11 and 0.04 ms; a single-precision 3LPT job's transforms at
-// 256^3 took it 13.4 ms, the pruned passes 6.3 ms: no size favours cuFFT.
+// 256^3 took it 13.4 ms, the pruned passes 6.3 ms; longer lengths without an
+// instance favour cuFFT in single precision (fx::length_fast32).
 static bool fx_supported(const mfx_job_desc *d) {
   if (fused_supported(d)) return false;
   const char *env = getenv("MFX_FUSED");
   if (env && env[0] == '0') return false;
-  const int N = d->ngrid;
-  return fx::length_supported(N) && (d->lpt_order < 2 || fx::length_supported(3 * N / 2));
+  const int N = d->ngrid, M = 3 * N / 2;
+  if (d->precision == MFX_FP32C)
+    return fx::length_fast32(N, false) && (d->lpt_order < 2 || fx::length_fast32(M, true));
+  return fx::length_supported(N) && (d->lpt_order < 2 || fx::length_supported(M));
 }
 
 // group_all: hold every sub-lattice's assembled components at once even where

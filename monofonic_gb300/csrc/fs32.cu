@@ -1,5 +1,5 @@
 // Single-precision pruned transforms (fs32.cuh): lengths without an instance
-// (run-time radices up to 12) and the launches.
+// (run-time radices up to 16) and the launches.
 #include "fs32.cuh"
 
 #include <algorithm>
@@ -20,17 +20,13 @@ constexpr int kSmem32 = 220 * 1024;
 // and threads for 8-byte values
 bool plan32(int L, FxPlan *p) {
   if (!fx_plan(L, FX_STRIDED, p)) return false;
-  for (int P : {16, 8, 4}) {
-    int need = 32, most = 32;
-    for (int q = 0; q < p->steps; ++q) {
-      const int items = P * (L / p->R[q]);
-      need = std::max(need, (items + radix_mult(p->R[q]) - 1) / radix_mult(p->R[q]));
-      most = std::max(most, items);
-    }
-    const int T = (std::max(need, std::min(most, 256)) + 31) / 32 * 32;
-    if (T > 512 || L * P * 8 > kSmem32) continue;
+  for (int P : {16, 8, 4, 2}) {
+    int need = 32;
+    for (int q = 0; q < p->steps; ++q) need = std::max(need, P * (L / p->R[q]));
+    const int T = (need + 31) / 32 * 32;
+    if (T > 768 || L * P * 8 > kSmem32) continue;
     p->P = P;
-    p->lgP = P == 16 ? 4 : (P == 8 ? 3 : 2);
+    p->lgP = P == 16 ? 4 : (P == 8 ? 3 : (P == 4 ? 2 : 1));
     p->T = T;
     p->smem = L * P * 8;
     return true;
@@ -53,37 +49,28 @@ __device__ __forceinline__ int slot32(int e, int q, int lgP) { return (e << lgP)
 template <int R>
 __device__ __noinline__ void step32(const float2 *tw, int L, int lgP, int NS, unsigned magic) {
   extern __shared__ __align__(16) F2 fsm[];
-  constexpr int MU = radix_mult(R);
-  const int T = blockDim.x, t = threadIdx.x;
-  const int nb = L / R, items = nb << lgP, pen = t & ((1 << lgP) - 1);
-  F2 v[MU][R];
-  int at[MU];
+  const int t = threadIdx.x, nb = L / R, pen = t & ((1 << lgP) - 1), j = t >> lgP;
+  const bool live = t < (nb << lgP);
+  F2 v[R];
+  int at = 0;
+  if (live) {
 #pragma unroll
-  for (int m = 0; m < MU; ++m) {
-    const int it = t + m * T;
-    at[m] = -1;
-    if (it < items) {
-      const int j = it >> lgP;
+    for (int r = 0; r < R; ++r) v[r] = fsm[slot32(j + r * nb, pen, lgP)];
+    if (NS == 1) {
+      at = j * R;
+    } else {
+      const int hi = int(__umulhi(unsigned(j), magic)), lo = j - hi * NS, inc = lo * (nb / NS);
+      at = hi * NS * R + lo;
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[m][r] = fsm[slot32(j + r * nb, pen, lgP)];
-      if (NS == 1) {
-        at[m] = j * R;
-      } else {
-        const int hi = int(__umulhi(unsigned(j), magic)), lo = j - hi * NS, inc = lo * (nb / NS);
-        at[m] = hi * NS * R + lo;
-#pragma unroll
-        for (int r = 1; r < R; ++r) v[m][r] = cmul(v[m][r], __ldg(&tw[r * inc]));
-      }
-      Dft<R>::run(v[m]);
+      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], __ldg(&tw[r * inc]));
     }
+    Dft<R>::run(v);
   }
   __syncthreads();
+  if (live) {
 #pragma unroll
-  for (int m = 0; m < MU; ++m)
-    if (at[m] >= 0) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) fsm[slot32(at[m] + r * NS, pen, lgP)] = v[m][r];
-    }
+    for (int r = 0; r < R; ++r) fsm[slot32(at + r * NS, pen, lgP)] = v[r];
+  }
   __syncthreads();
 }
 
@@ -103,11 +90,14 @@ __device__ __forceinline__ void transform32(const FxPlan &p, const float2 *tw) {
       case 9: step32<9>(tw, L, lgP, NS, mg); break;
       case 10: step32<10>(tw, L, lgP, NS, mg); break;
       case 12: step32<12>(tw, L, lgP, NS, mg); break;
+      case 14: step32<14>(tw, L, lgP, NS, mg); break;
+      case 15: step32<15>(tw, L, lgP, NS, mg); break;
+      case 16: step32<16>(tw, L, lgP, NS, mg); break;
     }
   }
 }
 
-__global__ void __launch_bounds__(512) k_fs_strided(const __grid_constant__ SArgs32 a) {
+__global__ void __launch_bounds__(768) k_fs_strided(const __grid_constant__ SArgs32 a) {
   mfx::pdl_begin();
   extern __shared__ __align__(16) F2 fsm[];
   const Strided &d = a.s;
@@ -174,7 +164,7 @@ __global__ void __launch_bounds__(512) k_fs_strided(const __grid_constant__ SArg
   }
 }
 
-__global__ void __launch_bounds__(512) k_fs_c2r_g(const __grid_constant__ RArgs32 a) {
+__global__ void __launch_bounds__(768) k_fs_c2r_g(const __grid_constant__ RArgs32 a) {
   mfx::pdl_begin();
   extern __shared__ __align__(16) F2 fsm[];
   const Rows &d = a.r;
@@ -214,7 +204,7 @@ __global__ void __launch_bounds__(512) k_fs_c2r_g(const __grid_constant__ RArgs3
   }
 }
 
-__global__ void __launch_bounds__(512) k_fs_r2c_g(const __grid_constant__ RArgs32 a) {
+__global__ void __launch_bounds__(768) k_fs_r2c_g(const __grid_constant__ RArgs32 a) {
   mfx::pdl_begin();
   extern __shared__ __align__(16) F2 fsm[];
   const Rows &d = a.r;
@@ -293,6 +283,11 @@ static const Len32Entry *find32(int L) {
   for (const Len32Entry &e : kLens32)
     if (e.L == L) return &e;
   return nullptr;
+}
+
+bool length_fast32(int L, bool padded) {
+  const Len32Entry *e = find32(L);
+  return (e && (padded ? e->padded : e->grid)) || (L <= 96 && length_supported(L));
 }
 
 cudaError_t prepare_device32(int dev) {

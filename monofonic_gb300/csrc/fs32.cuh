@@ -502,46 +502,50 @@ template <int L> __global__ void __launch_bounds__(Len32<L>::T, Len32<L>::ctas) 
 
 enum FsOp { FS_PREPARE = 0, FS_INV_PAD, FS_CUT, FS_TRUNC, FS_C2R_PAD, FS_R2C, FS_INV, FS_C2R };
 
+// (defined outside the class: an inline member would be instantiated, kernels and
+// all, wherever its address is taken)
 template <int L, bool PADDED, bool GRID> struct Launch32 {
-  static cudaError_t run(FsOp op, const Strided *s, const Rows *r, dim3 grid, cudaStream_t st) {
-    using F = Fft32<L, false>;
-    cudaError_t e = cudaSuccess;
-    auto limit = [&](const void *f) {
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem);
-    };
-    bool done = op == FS_PREPARE;
-    if constexpr (PADDED) {
-      if (op == FS_PREPARE) {
-        limit((const void *)k_fs_inv<L, true>);
-        limit((const void *)k_fs_cut<L>);
-        limit((const void *)k_fs_trunc<L>);
-        limit((const void *)k_fs_c2r<L, true>);
-        limit((const void *)k_fs_r2c<L>);
-      }
-      done = true;
-      if (op == FS_INV_PAD) mfx::launch_pdl(k_fs_inv<L, true>, grid, F::T, F::smem, st, *s);
-      else if (op == FS_CUT) mfx::launch_pdl(k_fs_cut<L>, grid, F::T, F::smem, st, *s);
-      else if (op == FS_TRUNC) mfx::launch_pdl(k_fs_trunc<L>, grid, F::T, F::smem, st, *s);
-      else if (op == FS_C2R_PAD) mfx::launch_pdl(k_fs_c2r<L, true>, grid, F::T, F::smem, st, *r);
-      else if (op == FS_R2C) mfx::launch_pdl(k_fs_r2c<L>, grid, F::T, F::smem, st, *r);
-      else done = op == FS_PREPARE;
-    }
-    if constexpr (GRID) {
-      if (op == FS_PREPARE) {
-        limit((const void *)k_fs_inv<L, false>);
-        limit((const void *)k_fs_c2r<L, false>);
-      }
-      if (op == FS_INV) {
-        mfx::launch_pdl(k_fs_inv<L, false>, grid, F::T, F::smem, st, *s);
-        done = true;
-      } else if (op == FS_C2R) {
-        mfx::launch_pdl(k_fs_c2r<L, false>, grid, F::T, F::smem, st, *r);
-        done = true;
-      }
-    }
-    if (!done) return cudaErrorInvalidValue;
-    return e == cudaSuccess ? cudaGetLastError() : e;
-  }
+  static cudaError_t run(FsOp op, const Strided *s, const Rows *r, dim3 grid, cudaStream_t st);
 };
+template <int L, bool PADDED, bool GRID>
+cudaError_t Launch32<L, PADDED, GRID>::run(FsOp op, const Strided *s, const Rows *r, dim3 grid, cudaStream_t st) {
+  using F = Fft32<L, false>;
+  cudaError_t e = cudaSuccess;
+  auto limit = [&](const void *f) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem);
+  };
+  bool done = op == FS_PREPARE;
+  if constexpr (PADDED) {
+    if (op == FS_PREPARE) {
+      limit((const void *)k_fs_inv<L, true>);
+      limit((const void *)k_fs_cut<L>);
+      limit((const void *)k_fs_trunc<L>);
+      limit((const void *)k_fs_c2r<L, true>);
+      limit((const void *)k_fs_r2c<L>);
+    }
+    done = true;
+    if (op == FS_INV_PAD) mfx::launch_pdl(k_fs_inv<L, true>, grid, F::T, F::smem, st, *s);
+    else if (op == FS_CUT) mfx::launch_pdl(k_fs_cut<L>, grid, F::T, F::smem, st, *s);
+    else if (op == FS_TRUNC) mfx::launch_pdl(k_fs_trunc<L>, grid, F::T, F::smem, st, *s);
+    else if (op == FS_C2R_PAD) mfx::launch_pdl(k_fs_c2r<L, true>, grid, F::T, F::smem, st, *r);
+    else if (op == FS_R2C) mfx::launch_pdl(k_fs_r2c<L>, grid, F::T, F::smem, st, *r);
+    else done = op == FS_PREPARE;
+  }
+  if constexpr (GRID) {
+    if (op == FS_PREPARE) {
+      limit((const void *)k_fs_inv<L, false>);
+      limit((const void *)k_fs_c2r<L, false>);
+    }
+    if (op == FS_INV) {
+      mfx::launch_pdl(k_fs_inv<L, false>, grid, F::T, F::smem, st, *s);
+      done = true;
+    } else if (op == FS_C2R) {
+      mfx::launch_pdl(k_fs_c2r<L, false>, grid, F::T, F::smem, st, *r);
+      done = true;
+    }
+  }
+  if (!done) return cudaErrorInvalidValue;
+  return e == cudaSuccess ? cudaGetLastError() : e;
+}
 
 }  // namespace fx

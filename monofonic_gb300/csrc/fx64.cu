@@ -31,7 +31,7 @@ namespace fx {
 // plans
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int kRadices[] = {12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+constexpr int kRadices[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
 constexpr int kSmemMax = 220 * 1024;
 
 // rough cost of a point: real multiplications (three products each, measured
@@ -41,7 +41,7 @@ double radix_cost(int R) {
     case 2: case 4: return 0.0;
     case 3: return 0.67; case 5: return 2.0; case 6: return 0.67; case 7: return 5.1;
     case 8: return 0.5; case 9: return 2.0; case 10: return 2.0; case 12: return 0.67;
-    default: return 0.0;
+    case 14: return 5.1; case 15: return 2.67; default: return 1.25;  // 16
   }
 }
 
@@ -96,21 +96,14 @@ bool fx_plan(int L, FxKind kind, FxPlan *p) {
     ns *= best[q];
   }
   p->B = fx_bits(p->R, n, kind);
-  for (int P : {8, 4, 2}) {
-    // threads: at least what the steps' butterflies need, and enough of them
-    // that short pencils still fill a few warps
-    int need = 32, most = 32;
-    for (int q = 0; q < n; ++q) {
-      const int items = P * (L / p->R[q]), mu = radix_mult(p->R[q]);
-      need = std::max(need, (items + mu - 1) / mu);
-      most = std::max(most, items);
-    }
-    int T = std::max(need, std::min(most, 256));
-    T = (T + 31) / 32 * 32;
+  for (int P : {8, 4, 2, 1}) {
+    int need = 32;  // threads: a butterfly each
+    for (int q = 0; q < n; ++q) need = std::max(need, P * (L / p->R[q]));
+    const int T = (need + 31) / 32 * 32;
     const int smem = L * P * 16 + P * 8;
-    if (T > 384 || smem > kSmemMax) continue;
+    if (T > 768 || smem > kSmemMax) continue;
     p->P = P;
-    p->lgP = P == 8 ? 3 : (P == 4 ? 2 : 1);
+    p->lgP = P == 8 ? 3 : (P == 4 ? 2 : P - 1);
     p->T = T;
     p->smem = smem;
     return true;
@@ -170,56 +163,42 @@ struct Core {
 
 __device__ __forceinline__ int slot(int e, int q, int lgP) { return (e << lgP) + (q ^ (e & ((1 << lgP) - 1))); }
 
-// one Stockham step of radix R over the CTA's pencils; raw: the values are
-// still doubles (sh: the conversion of this thread's pencil)
+// one Stockham step of radix R over the CTA's pencils, a butterfly a thread; raw:
+// the values are still doubles (sh: the conversion of this thread's pencil)
 template <int R>
 __device__ __noinline__ void step(const longlong2 *tw, int L, int lgP, int NS, unsigned magic, bool raw, int sh) {
   extern __shared__ __align__(16) longlong2 s[];
-  constexpr int MU = radix_mult(R);
-  const int T = blockDim.x, t = threadIdx.x;
-  const int nb = L / R, items = nb << lgP;
-  const int pen = t & ((1 << lgP) - 1);
+  const int t = threadIdx.x, nb = L / R, pen = t & ((1 << lgP) - 1), j = t >> lgP;
+  const bool live = t < (nb << lgP);
   const Tw3 t3 = tw3_of(tw, L);
-  I2 v[MU][R];
-  int jn[MU];
+  I2 v[R];
+  int at = 0;
+  if (live) {
 #pragma unroll
-  for (int m = 0; m < MU; ++m) {
-    const int it = t + m * T;
-    jn[m] = -1;
-    if (it < items) {
-      const int j = it >> lgP;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const longlong2 w = s[slot(j + r * nb, pen, lgP)];
-        v[m][r] = {w.x, w.y};
-      }
-      if (NS == 1) {
-        jn[m] = j * R;
-        if (raw) {
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            v[m][r].x = to_fixed_p(v[m][r].x, sh);
-            v[m][r].y = to_fixed_p(v[m][r].y, sh);
-          }
-        }
-      } else {
-        const int hi = int(__umulhi(unsigned(j), magic)), lo = j - hi * NS;
-        jn[m] = hi * NS * R + lo;
-        const int inc = lo * (nb / NS);  // lo L / (NS R)
-        v[m][0] = eighth(v[m][0]);
-#pragma unroll
-        for (int r = 1; r < R; ++r) v[m][r] = twiddle8(v[m][r], t3, r * inc);
-      }
-      Dft<R>::run(v[m]);
+    for (int r = 0; r < R; ++r) {
+      const longlong2 w = s[slot(j + r * nb, pen, lgP)];
+      v[r] = {w.x, w.y};
     }
+    if (NS == 1) {
+      at = j * R;
+      if (raw) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = {to_fixed_p(v[r].x, sh), to_fixed_p(v[r].y, sh)};
+      }
+    } else {
+      const int hi = int(__umulhi(unsigned(j), magic)), lo = j - hi * NS, inc = lo * (nb / NS);  // lo L / (NS R)
+      at = hi * NS * R + lo;
+      v[0] = eighth(v[0]);
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = twiddle8(v[r], t3, r * inc);
+    }
+    Dft<R>::run(v);
   }
   __syncthreads();
+  if (live) {
 #pragma unroll
-  for (int m = 0; m < MU; ++m)
-    if (jn[m] >= 0) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) s[slot(jn[m] + r * NS, pen, lgP)] = make_longlong2(v[m][r].x, v[m][r].y);
-    }
+    for (int r = 0; r < R; ++r) s[slot(at + r * NS, pen, lgP)] = make_longlong2(v[r].x, v[r].y);
+  }
   __syncthreads();
 }
 
@@ -241,6 +220,9 @@ __device__ __forceinline__ void transform(const Core &c, bool raw, int sh) {
       case 9: step<9>(c.tw, L, lgP, NS, mg, rw, sh); break;
       case 10: step<10>(c.tw, L, lgP, NS, mg, rw, sh); break;
       case 12: step<12>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 14: step<14>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 15: step<15>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 16: step<16>(c.tw, L, lgP, NS, mg, rw, sh); break;
     }
   }
 }
@@ -250,7 +232,7 @@ struct SArgs {
   Strided s;
 };
 
-__global__ void __launch_bounds__(384) k_fx_strided(const __grid_constant__ SArgs a) {
+__global__ void __launch_bounds__(768) k_fx_strided(const __grid_constant__ SArgs a) {
   mfx::pdl_begin();
   extern __shared__ __align__(16) longlong2 sm[];
   const Strided &d = a.s;
@@ -366,7 +348,7 @@ struct RArgs {
 
 // spectra -> real rows: rows 2q and 2q + 1 as the real and imaginary part of
 // one pencil, Z[k] = A[k] + i B[k], Z[L - k] = conj A[k] + i conj B[k]
-__global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a) {
+__global__ void __launch_bounds__(768) k_fx_c2r(const __grid_constant__ RArgs a) {
   mfx::pdl_begin();
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
@@ -446,7 +428,7 @@ __global__ void __launch_bounds__(384) k_fx_c2r(const __grid_constant__ RArgs a)
 }
 
 // real rows -> spectra of kz < kc, two rows a pencil
-__global__ void __launch_bounds__(384) k_fx_r2c(const __grid_constant__ RArgs a) {
+__global__ void __launch_bounds__(768) k_fx_r2c(const __grid_constant__ RArgs a) {
   mfx::pdl_begin();
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;

@@ -332,8 +332,6 @@ FX_HD double to_double(long long v, int S) {
 // plans
 // ---------------------------------------------------------------------------
 constexpr int kMaxSteps = 6;
-// butterflies of a step that one thread holds at once (16 complex values at most)
-constexpr int radix_mult(int R) { return R > 8 ? 1 : 16 / R; }
 
 struct FxPlan {
   int L;                // length

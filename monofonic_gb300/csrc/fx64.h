@@ -82,5 +82,9 @@ cudaError_t run_r2c32(const Rows &r, cudaStream_t st);
 // float2 (cos, -sin)(2 pi t / L), t < L (host memory, kept for the process)
 const float2 *twiddles32(int L);
 cudaError_t prepare_device32(int dev);
+// lengths whose single-precision passes beat cuFFT: the instances, and short ones
+// with the run-time kernels (36^3 3LPT 0.24 against 0.43 ms; without instances
+// 300^3 2LPT would take 16.4 ms against 9.3, 400^3 26.0 against 25.8)
+bool length_fast32(int L, bool padded);
 
 }  // namespace fx

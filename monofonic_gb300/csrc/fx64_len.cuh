@@ -726,48 +726,52 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_f
 // three), as grid length, or both
 enum FxOp { FX_OP_PREPARE = 0, FX_OP_INV_PAD, FX_OP_CUT, FX_OP_TRUNC, FX_OP_C2R_PAD, FX_OP_R2C, FX_OP_INV, FX_OP_C2R };
 
+// (defined outside the class: an inline member would be instantiated, kernels and
+// all, wherever its address is taken)
 template <int L, bool PADDED, bool GRID> struct Launch {
-  static cudaError_t run(FxOp op, const void *args, dim3 grid, cudaStream_t st) {
-    using F = Fft<L, false>;
-    const LArgs *s = static_cast<const LArgs *>(args);
-    const LRows *r = static_cast<const LRows *>(args);
-    cudaError_t e = cudaSuccess;
-    auto limit = [&](const void *f) {
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem);
-    };
-    bool done = op == FX_OP_PREPARE;
-    if constexpr (PADDED) {
-      if (op == FX_OP_PREPARE) {
-        limit((const void *)k_fx_inv<L, true>);
-        limit((const void *)k_fx_cut<L>);
-        limit((const void *)k_fx_trunc<L>);
-        limit((const void *)k_fx_c2r_l<L, true>);
-        limit((const void *)k_fx_r2c_l<L>);
-      }
-      done = true;
-      if (op == FX_OP_INV_PAD) mfx::launch_pdl(k_fx_inv<L, true>, grid, F::T, F::smem, st, *s);
-      else if (op == FX_OP_CUT) mfx::launch_pdl(k_fx_cut<L>, grid, F::T, F::smem, st, *s);
-      else if (op == FX_OP_TRUNC) mfx::launch_pdl(k_fx_trunc<L>, grid, F::T, F::smem, st, *s);
-      else if (op == FX_OP_C2R_PAD) mfx::launch_pdl(k_fx_c2r_l<L, true>, grid, F::T, F::smem, st, *r);
-      else if (op == FX_OP_R2C) mfx::launch_pdl(k_fx_r2c_l<L>, grid, F::T, F::smem, st, *r);
-      else done = op == FX_OP_PREPARE;
-    }
-    if constexpr (GRID) {
-      if (op == FX_OP_PREPARE) {
-        limit((const void *)k_fx_inv<L, false>);
-        limit((const void *)k_fx_c2r_l<L, false>);
-      }
-      if (op == FX_OP_INV) {
-        mfx::launch_pdl(k_fx_inv<L, false>, grid, F::T, F::smem, st, *s);
-        done = true;
-      } else if (op == FX_OP_C2R) {
-        mfx::launch_pdl(k_fx_c2r_l<L, false>, grid, F::T, F::smem, st, *r);
-        done = true;
-      }
-    }
-    if (!done) return cudaErrorInvalidValue;
-    return e == cudaSuccess ? cudaGetLastError() : e;
-  }
+  static cudaError_t run(FxOp op, const void *args, dim3 grid, cudaStream_t st);
 };
+template <int L, bool PADDED, bool GRID>
+cudaError_t Launch<L, PADDED, GRID>::run(FxOp op, const void *args, dim3 grid, cudaStream_t st) {
+  using F = Fft<L, false>;
+  const LArgs *s = static_cast<const LArgs *>(args);
+  const LRows *r = static_cast<const LRows *>(args);
+  cudaError_t e = cudaSuccess;
+  auto limit = [&](const void *f) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem);
+  };
+  bool done = op == FX_OP_PREPARE;
+  if constexpr (PADDED) {
+    if (op == FX_OP_PREPARE) {
+      limit((const void *)k_fx_inv<L, true>);
+      limit((const void *)k_fx_cut<L>);
+      limit((const void *)k_fx_trunc<L>);
+      limit((const void *)k_fx_c2r_l<L, true>);
+      limit((const void *)k_fx_r2c_l<L>);
+    }
+    done = true;
+    if (op == FX_OP_INV_PAD) mfx::launch_pdl(k_fx_inv<L, true>, grid, F::T, F::smem, st, *s);
+    else if (op == FX_OP_CUT) mfx::launch_pdl(k_fx_cut<L>, grid, F::T, F::smem, st, *s);
+    else if (op == FX_OP_TRUNC) mfx::launch_pdl(k_fx_trunc<L>, grid, F::T, F::smem, st, *s);
+    else if (op == FX_OP_C2R_PAD) mfx::launch_pdl(k_fx_c2r_l<L, true>, grid, F::T, F::smem, st, *r);
+    else if (op == FX_OP_R2C) mfx::launch_pdl(k_fx_r2c_l<L>, grid, F::T, F::smem, st, *r);
+    else done = op == FX_OP_PREPARE;
+  }
+  if constexpr (GRID) {
+    if (op == FX_OP_PREPARE) {
+      limit((const void *)k_fx_inv<L, false>);
+      limit((const void *)k_fx_c2r_l<L, false>);
+    }
+    if (op == FX_OP_INV) {
+      mfx::launch_pdl(k_fx_inv<L, false>, grid, F::T, F::smem, st, *s);
+      done = true;
+    } else if (op == FX_OP_C2R) {
+      mfx::launch_pdl(k_fx_c2r_l<L, false>, grid, F::T, F::smem, st, *r);
+      done = true;
+    }
+  }
+  if (!done) return cudaErrorInvalidValue;
+  return e == cudaSuccess ? cudaGetLastError() : e;
+}
 
 }  // namespace fx
