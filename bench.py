@@ -61,9 +61,6 @@ LATNAME = {0: "sc", 1: "bcc", 2: "fcc"}
 # --steps/--warmup run stays within a few minutes)
 CPU_SAMPLE = {"fcc768": 384, "fcc512": 256, "fcc384": 384, "bcc256": 256, "bcc128": 128, "sc64": 64}
 REF_SAMPLE = {"fcc768": 192, "fcc512": 192, "fcc384": 192, "bcc256": 256, "bcc128": 128, "sc64": 64}
-# GB300 FP64 (non-tensor) arithmetic rate, NVIDIA's published figure (FLOP/s):
-# the ceiling of the plain FP64 form's cuFFT transforms
-FP64_PEAK_SPEC = 1.25e12
 
 
 def describe(name, prec):
@@ -441,7 +438,7 @@ def run_ours(args):
         roof = {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_src + " (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured" else "fallback",
                 "traffic": traffic, "alg_bytes_per_launch": d[1] / d[2], "launches": d[2]}
-        fft = {k: v for k, v in prof_tot.items() if k.startswith("cufft")}
+        fft = {k: v for k, v in prof_tot.items() if k.startswith(("fx_", "cufft"))}
         fft_ms = sum(v[0] for v in fft.values())
         fft_bytes = sum(v[1] for v in fft.values())
         alg_total = job.algorithmic_bytes()
@@ -818,14 +815,14 @@ def fp64_and_error(args, eng, inp, plt_tab, out):
                 j.run()
                 ms.append(sum(j.stage_times()))
                 for k, (kms, kby, kcnt) in j.kernel_profile().items():
-                    if k.startswith("cufft"):
+                    if k.startswith(("fx_", "cufft")):
                         a = fft.setdefault(k, [0.0, 0.0])
                         a[0] += kms
                         a[1] += kby
             j.set_profiling(False)
             res["fp64_form"] = {"value": j.num_particles / (np.mean(ms) * 1e-3), "unit": "particles/s",
                                 "ms_per_step": float(np.mean(ms)), "steps": len(ms)}
-            res["fp64_form"]["fft_rate"] = fp64_fft_rate(fft, inp["n"], len(ms), float(np.mean(ms)))
+            res["fp64_form"]["fft_rate"] = fp64_fft_rate(fft, len(ms), float(np.mean(ms)))
         # compared particles: all of them up to 64M (16M per order), else the first ones
         count = min(j.num_particles, 1 << 26)
         count_o = min(j.num_particles, 1 << 24)
@@ -850,27 +847,14 @@ def fp64_and_error(args, eng, inp, plt_tab, out):
     return res
 
 
-def fp64_fft_rate(fft, n, steps, ms_step):
-    """FLOP rate of the plain FP64 form's cuFFT transforms: 2.5 L log2 L per
-    real transform of L points (the usual split-radix count), transforms
-    counted from the bytes each execution moves (2 x the padded field)."""
-    m = 3 * n // 2
-    out = {}
-    flops = ms = 0.0
-    for k, (kms, kby) in fft.items():
-        length = m if k.endswith("_M") else n
-        field = (length + 2) * length * length * 8.0
-        count = kby / (2.0 * field) / steps
-        f = count * 2.5 * length ** 3 * np.log2(float(length) ** 3)
-        out[k] = {"transforms_per_step": count, "ms_per_step": kms / steps,
-                  "gflops": f / (kms / steps * 1e-3) / 1e9 if kms else None}
-        flops += f
-        ms += kms / steps
-    rate = flops / (ms * 1e-3) if ms else None
-    return {"kernels": out, "fft_ms_per_step": ms, "share_of_step": ms / ms_step if ms_step else None,
-            "fft_tflops": rate / 1e12 if rate else None, "fp64_peak_tflops": FP64_PEAK_SPEC / 1e12,
-            "frac_of_fp64_peak": rate / FP64_PEAK_SPEC if rate else None,
-            "peak_source": "GB300 FP64 published rate (spec figure, not measured)"}
+def fp64_fft_rate(fft, steps, ms_step):
+    """The plain FP64 form's transform passes: time and field traffic of each
+    (the pruned passes are fixed point and run at the integer multipliers'
+    rate, so a FLOP rate would not say how busy they are)."""
+    ms = sum(v[0] for v in fft.values()) / steps
+    return {"kernels": {k: {"ms_per_step": kms / steps, "alg_GBps": kby / (kms * 1e-3) / 1e9 if kms else None}
+                        for k, (kms, kby) in fft.items()},
+            "fft_ms_per_step": ms, "share_of_step": ms / ms_step if ms_step else None}
 
 
 def cpu_restatement(n_sample, name, plt_tab=None, seed_offset=0):

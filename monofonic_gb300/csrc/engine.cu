@@ -3,6 +3,10 @@
 //
 // Pipeline of one job (reference: ic_generator.cc:288-1060):
 //   noise -> phi1                               k_noise_phi1
+// then, in the FP32 form, the fused transforms (fused.cuh); in the FP64 form and
+// the FP32 jobs that have none, the pruned passes of fx64.h around k_src2,
+// k_pairs3a, k_src3 and k_assemble_rows; and for grids with prime factors that
+// the pruned passes lack, cuFFT:
 //   phi1 Hessians (6, padded M^3)              k_pad_hessian + 6 c2r
 //   phi2 source -> r2c -> unpad/invLap         k_src2, r2c, k_unpad_invlap
 //   phi3a: 5 pairwise products, each           k_mul, r2c, k_trunc_repad, c2r, k_acc3a
@@ -411,8 +415,8 @@ static int check_desc(const mfx_job_desc *d) {
 
 // The FP32 form runs the padded convolutions through the pruned, fused
 // transforms (fused.cuh) for every padded length they are built for; the
-// plain FP64 form and other sizes use cuFFT.  MFX_FUSED=0 in the environment
-// sends the FP32 form through cuFFT as well (for comparisons).
+// plain FP64 form and other sizes see fx_supported.  MFX_FUSED=0 in the
+// environment sends everything through cuFFT (for comparisons).
 static bool fused_supported(const mfx_job_desc *d) {
   if (d->precision != MFX_FP32C || d->lpt_order < 2) return false;
   // the pruned transforms take phi(1) with empty Nyquist planes (NGenIC's
@@ -2368,8 +2372,8 @@ int mfx_job_footprint(mfx_engine *eng, const mfx_job_desc *desc, size_t *bytes) 
   GUARD_BEGIN
   TRY(check_desc(desc));
   if (!bytes) return set_error(MFX_EINVAL, "null output");
-  // FFT work areas are bounded by the largest transform's data size: the
-  // padded cuFFT transforms (plain form), the batch of six N-grid c2r
+  // cuFFT work areas, where it runs, are bounded by the largest transform's data
+  // size: the padded transforms, the batch of six N-grid c2r
   const int M = 3 * desc->ngrid / 2;
   const size_t rs = desc->precision == MFX_FP64 ? 8 : 4;
   const bool fused = fused_supported(desc) || fx_supported(desc);

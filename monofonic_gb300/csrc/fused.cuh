@@ -38,13 +38,14 @@
 // outputs straight to their destination, so the x/y passes move each element
 // through shared memory once.
 #pragma once
-#include "pdl.cuh"
 #include <stdint.h>
 
 #include <type_traits>
 #include <utility>
 #if defined(__CUDACC__)
 #include <cuda_runtime.h>
+
+#include "pdl.cuh"
 #define MFX_HD __host__ __device__ __forceinline__
 #define MFX_CX __host__ __device__ constexpr
 #else

@@ -6,7 +6,7 @@
 // n+2 reals; the same buffer holds the k-space field as n x n x (n/2+1)
 // complex values, kelem(i,j,k) = c[(i*n + j)*(n/2+1) + k].  N-grid fields are
 // the LPT potentials, M-grid (M = 3N/2) fields the Orszag-padded products.
-// FFTs are unnormalised cuFFT transforms; the unitary 1/sqrt(n^3) of the
+// The transforms are unnormalised; the unitary 1/sqrt(n^3) of the
 // reference (grid_fft.cc:69, 199-270) is folded into the kernel before or
 // after each transform.
 #pragma once
