@@ -702,7 +702,7 @@ template <typename R> static int launch_music(mfx_job *j, int mode, void *out) {
     c.nc = n / c.cs;
     c.row = 2LL * (n / 2 + 1);
     KBEGIN(j);
-    music::k_music_cubes<R><<<unsigned(c.nc) * c.nc * c.nc, 32, 0, j->stream>>>(c, (R *)buf);
+    music::k_music_cubes<R><<<unsigned(c.nc) * c.nc * c.nc, 32 * music::kCubeWarps, 0, j->stream>>>(c, (R *)buf);
     KEND(j, "music_cubes", double(n) * n * n * sizeof(R));
     return exec_fft(j, plan, buf, true);
   };

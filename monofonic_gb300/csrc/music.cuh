@@ -54,51 +54,19 @@ __device__ __forceinline__ uint32_t mt_temper(uint32_t y) {
   return y;
 }
 
-// Regenerates the 624-word block in place.  Element k of the sequential
+// Regenerates the 624-word block.  Element k of the sequential
 // twist reads x[k], x[k+1] and x[(k+397) mod 624]; the last of these is an
 // old word for k < 227 and a new one (x[k-227]) after that, and x[0] is new
-// for k = 623.  Each phase reads all its inputs before any lane writes.
-__device__ __forceinline__ void mt_twist(uint32_t *x, int lane) {
+// for k = 623.  y[] receives the next state of x[], by a CTA of at least P1 threads.
+__device__ __forceinline__ void mt_twist(const uint32_t *x, uint32_t *y, int k) {
   constexpr int P1 = kMtN - kMtM;  // 227
-  uint32_t t[8];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int k = lane + 32 * r;
-    if (k < P1) t[r] = mt_mix(x[k], x[k + 1], x[k + kMtM]);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int k = lane + 32 * r;
-    if (k < P1) x[k] = t[r];
-  }
-  __syncwarp();
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int k = P1 + lane + 32 * r;
-    if (k < 2 * P1) t[r] = mt_mix(x[k], x[k + 1], x[k - P1]);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int k = P1 + lane + 32 * r;
-    if (k < 2 * P1) x[k] = t[r];
-  }
-  __syncwarp();
-#pragma unroll
-  for (int r = 0; r < 6; ++r) {
-    const int k = 2 * P1 + lane + 32 * r;
-    if (k < kMtN - 1) t[r] = mt_mix(x[k], x[k + 1], x[k - P1]);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int r = 0; r < 6; ++r) {
-    const int k = 2 * P1 + lane + 32 * r;
-    if (k < kMtN - 1) x[k] = t[r];
-  }
-  __syncwarp();
-  if (lane == 0) x[kMtN - 1] = mt_mix(x[kMtN - 1], x[0], x[kMtM - 1]);
-  __syncwarp();
+  if (k < P1) y[k] = mt_mix(x[k], x[k + 1], x[k + kMtM]);
+  __syncthreads();
+  if (k < P1) y[k + P1] = mt_mix(x[k + P1], x[k + P1 + 1], y[k]);
+  __syncthreads();
+  if (k < kMtN - 1 - 2 * P1) y[k + 2 * P1] = mt_mix(x[k + 2 * P1], x[k + 2 * P1 + 1], y[k + P1]);
+  if (k == kMtN - 1 - 2 * P1) y[kMtN - 1] = mt_mix(x[kMtN - 1], y[0], y[kMtM - 1]);
+  __syncthreads();
 }
 
 // The ratio method's acceptance of one pair of outputs, in the operation
@@ -158,15 +126,22 @@ struct CubeArgs {
   long long row;     // real elements between consecutive k-rows (2 (N/2 + 1))
 };
 
-// One warp per cube: blockDim.x == 32, gridDim.x == nc^3.  Writes cube cells
-// into the padded real layout of an in-place r2c transform.
-template <typename R> __global__ void __launch_bounds__(32) k_music_cubes(CubeArgs a, R *out) {
-  __shared__ uint32_t x[kMtN];
-  const int lane = threadIdx.x;
+// One CTA per cube (gridDim.x == nc^3), a thread for each of the 312 pairs of a
+// state.  Writes cube cells into the padded real layout of an in-place r2c
+// transform.  A cube is one chain of states, 144 of them for 32^3 cells; on
+// grids of a few hundred cubes its latency is the kernel's time.  With one
+// warp a cube the ten groups of pairs of a state followed one another: a 256^3
+// 3LPT FP32 pass took 9.87 ms, 9.42 with ten warps a cube.
+constexpr int kCubeWarps = (kMtN / 2 + 31) / 32;
+template <typename R> __global__ void __launch_bounds__(32 * kCubeWarps) k_music_cubes(CubeArgs a, R *out) {
+  __shared__ uint32_t state[2][kMtN];
+  __shared__ int cnt[kCubeWarps];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const long long icube = blockIdx.x;
   const int nc = a.nc, cs = a.cs;
   const int ic = int(icube / (nc * nc)), jc = int((icube / nc) % nc), kc = int(icube % nc);
-  if (lane == 0) {
+  uint32_t *x = state[0], *y = state[1];
+  if (t == 0) {
     // gsl_rng_set(mt19937, baseseed + icube): the seed as an unsigned long,
     // its low 32 bits used
     const unsigned long long cseed = static_cast<unsigned long long>(*a.seed + icube);
@@ -177,33 +152,39 @@ template <typename R> __global__ void __launch_bounds__(32) k_music_cubes(CubeAr
       x[k] = s;
     }
   }
-  __syncwarp();
+  __syncthreads();
   const int total = cs * cs * cs, cs2 = cs * cs;
   R *base = out + (size_t(ic) * cs * a.N + size_t(jc) * cs) * size_t(a.row) + size_t(kc) * cs;
   int produced = 0;
   const unsigned lt = (1u << lane) - 1u;
   while (produced < total) {
-    mt_twist(x, lane);
-    for (int p0 = 0; p0 < kMtN / 2 && produced < total; p0 += 32) {
-      const int p = p0 + lane;
-      bool acc = false;
-      uint32_t w1 = 0, w2 = 0;
-      float uf = 1.f, vf = 0.f;
-      if (p < kMtN / 2) {
-        w1 = mt_temper(x[2 * p]);
-        w2 = mt_temper(x[2 * p + 1]);
-        leva_uv_f(w1, w2, uf, vf);
-        acc = leva_accept(w1, w2, uf, vf);
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, acc);
-      const int c = produced + __popc(m & lt);
-      if (acc && c < total) {
-        const int ii = c / cs2, jj = (c / cs) % cs, kk = c % cs;
-        base[(size_t(ii) * a.N + jj) * size_t(a.row) + kk] = leva_value<R>(w1, w2, uf, vf);
-      }
-      produced += __popc(m);
+    mt_twist(x, y, t);
+    uint32_t *z = x;
+    x = y, y = z;
+    bool acc = false;
+    uint32_t w1 = 0, w2 = 0;
+    float uf = 1.f, vf = 0.f;
+    if (t < kMtN / 2) {
+      w1 = mt_temper(x[2 * t]);
+      w2 = mt_temper(x[2 * t + 1]);
+      leva_uv_f(w1, w2, uf, vf);
+      acc = leva_accept(w1, w2, uf, vf);
     }
-    __syncwarp();
+    const unsigned m = __ballot_sync(0xffffffffu, acc);
+    if (lane == 0) cnt[w] = __popc(m);
+    __syncthreads();
+    // cnt is written again after the next state's barriers
+    int c = produced + __popc(m & lt);
+#pragma unroll
+    for (int q = 0; q < kCubeWarps; ++q) {
+      const int n = cnt[q];
+      if (q < w) c += n;
+      produced += n;
+    }
+    if (acc && c < total) {
+      const int ii = c / cs2, jj = (c / cs) % cs, kk = c % cs;
+      base[(size_t(ii) * a.N + jj) * size_t(a.row) + kk] = leva_value<R>(w1, w2, uf, vf);
+    }
   }
 }
 
