@@ -27,104 +27,11 @@
 
 namespace fx {
 
-// ---------------------------------------------------------------------------
-// plans
-// ---------------------------------------------------------------------------
-namespace {
-constexpr int kRadices[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
-constexpr int kSmemMax = 220 * 1024;
-
-// rough cost of a point: real multiplications (three products each, measured
-// 4 a clock) and the shared-memory round trip of a step
-double radix_cost(int R) {
-  switch (R) {
-    case 2: case 4: return 0.0;
-    case 3: return 0.67; case 5: return 2.0; case 6: return 0.67; case 7: return 5.1;
-    case 8: return 0.5; case 9: return 2.0; case 10: return 2.0; case 12: return 0.67;
-    case 14: return 5.1; case 15: return 2.67; default: return 1.25;  // 16
-  }
-}
-
-// best factorisation: fewest steps, then least cost, then smallest largest radix
-void search(int rest, int depth, double cost, int *cur, int &best_n, double &best_c, int *best) {
-  if (rest == 1) {
-    int mx = 0;
-    for (int q = 0; q < depth; ++q) mx = std::max(mx, cur[q]);
-    const double c = cost + 0.02 * mx;
-    if (depth < best_n || (depth == best_n && c < best_c)) {
-      best_n = depth;
-      best_c = c;
-      std::copy(cur, cur + depth, best);
-    }
-    return;
-  }
-  if (depth == kMaxSteps || depth >= best_n) return;
-  for (int R : kRadices)
-    if (rest % R == 0 && (depth == 0 || R <= cur[depth - 1])) {
-      cur[depth] = R;
-      search(rest / R, depth + 1, cost + radix_cost(R), cur, best_n, best_c, best);
-    }
-}
-}  // namespace
-
-int fx_bits(const int *R, int steps, FxKind kind) {
-  double m = kind == FX_C2R ? 1.5 : 0.5, top = m;
-  for (int q = 0; q < steps; ++q) {
-    if (q) m -= 3.0;
-    m += std::log2(double(R[q]));
-    top = std::max(top, m);
-  }
-  if (kind == FX_R2C) top = std::max(top, m + 1.0);
-  return std::min(60, int(std::floor(62.7 - top)));
-}
-
-bool fx_plan(int L, FxKind kind, FxPlan *p) {
-  *p = FxPlan{};
-  p->L = L;
-  int cur[kMaxSteps], best[kMaxSteps], n = kMaxSteps + 1;
-  double c = 1e30;
-  search(L, 0, 0.0, cur, n, c, best);
-  if (n > kMaxSteps) return false;
-  p->steps = n;
-  // smallest radix first: its butterflies, the most, carry no twiddles
-  std::sort(best, best + n);
-  int ns = 1;
-  for (int q = 0; q < n; ++q) {
-    p->R[q] = best[q];
-    p->NS[q] = ns;
-    p->magic[q] = unsigned((0x100000000ULL + unsigned(ns) - 1) / unsigned(ns));
-    ns *= best[q];
-  }
-  p->B = fx_bits(p->R, n, kind);
-  for (int P : {8, 4, 2, 1}) {
-    int need = 32;  // threads: a butterfly each
-    for (int q = 0; q < n; ++q) need = std::max(need, P * (L / p->R[q]));
-    const int T = (need + 31) / 32 * 32;
-    const int smem = L * P * 16 + P * 8;
-    if (T > 768 || smem > kSmemMax) continue;
-    p->P = P;
-    p->lgP = P == 8 ? 3 : (P == 4 ? 2 : P - 1);
-    p->T = T;
-    p->smem = smem;
-    return true;
-  }
-  return false;
-}
-
-// (cos, -sin)(2 pi t / L) 2^61, t < L, then the three constants of the products
-// with them, split into signed halves: c and s + c, then s - c (fx64_len.cuh Tw3)
-static void make_twiddles(int L, longlong2 *out) {
-  int4 *cp = reinterpret_cast<int4 *>(out + L);
+// for each t < L the three constants of a product with its twiddle, c and s + c
+// of all t, then s - c (fx64_len.cuh Tw3)
+static void make_twiddles(int L, int4 *cp) {
   int2 *m = reinterpret_cast<int2 *>(cp + L);
-  auto lo = [](long long w) { return int(w); };
-  auto hi = [](long long w) { return int(w >> 32) + int(unsigned(int(w)) >> 31); };
-  for (int t = 0; t < L; ++t) {
-    const CS w = q62_turn(t, L);
-    const long long c = (long long)((w.c + 1) >> 1), s = (long long)((-w.s + 1) >> 1);
-    out[t] = make_longlong2(c, s);
-    cp[t] = make_int4(hi(c), lo(c), hi(s + c), lo(s + c));
-    m[t] = make_int2(hi(s - c), lo(s - c));
-  }
+  for (int t = 0; t < L; ++t) twiddle_constants(t, L, &cp[t], &m[t]);
 }
 
 bool length_supported(int L) { return fx_supported(L); }
@@ -141,13 +48,13 @@ const float2 *twiddles32(int L) {
   return t.data();
 }
 
-const longlong2 *twiddles(int L) {
+const void *twiddles(int L) {
   static std::mutex mu;
-  static std::map<int, std::vector<longlong2>> tables;
+  static std::map<int, std::vector<int4>> tables;
   std::lock_guard<std::mutex> lk(mu);
-  std::vector<longlong2> &t = tables[L];
+  std::vector<int4> &t = tables[L];
   if (t.empty()) {
-    t.resize(twiddle_bytes(L) / sizeof(longlong2));
+    t.resize(twiddle_bytes(L) / sizeof(int4));
     make_twiddles(L, t.data());
   }
   return t.data();
@@ -158,15 +65,16 @@ const longlong2 *twiddles(int L) {
 // ---------------------------------------------------------------------------
 struct Core {
   FxPlan p;
-  const longlong2 *tw;
+  const void *tw;
 };
 
 __device__ __forceinline__ int slot(int e, int q, int lgP) { return (e << lgP) + (q ^ (e & ((1 << lgP) - 1))); }
 
 // one Stockham step of radix R over the CTA's pencils, a butterfly a thread; raw:
-// the values are still doubles (sh: the conversion of this thread's pencil)
+// the values are still doubles (sh: the conversion of this thread's pencil); twice:
+// inputs doubled before their twiddles
 template <int R>
-__device__ __noinline__ void step(const longlong2 *tw, int L, int lgP, int NS, unsigned magic, bool raw, int sh) {
+__device__ __noinline__ void step(const void *tw, int L, int lgP, int NS, unsigned magic, bool raw, int sh, bool twice) {
   extern __shared__ __align__(16) longlong2 s[];
   const int t = threadIdx.x, nb = L / R, pen = t & ((1 << lgP) - 1), j = t >> lgP;
   const bool live = t < (nb << lgP);
@@ -188,9 +96,13 @@ __device__ __noinline__ void step(const longlong2 *tw, int L, int lgP, int NS, u
     } else {
       const int hi = int(__umulhi(unsigned(j), magic)), lo = j - hi * NS, inc = lo * (nb / NS);  // lo L / (NS R)
       at = hi * NS * R + lo;
-      v[0] = eighth(v[0]);
+      if (twice) {
 #pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = twiddle8(v[r], t3, r * inc);
+        for (int r = 0; r < R; ++r) v[r] = v[r] + v[r];
+      }
+      v[0] = quarter(v[0]);
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = twiddle4(v[r], t3, r * inc);
     }
     Dft<R>::run(v);
   }
@@ -206,25 +118,54 @@ __device__ __noinline__ void step(const longlong2 *tw, int L, int lgP, int NS, u
 __device__ __forceinline__ void transform(const Core &c, bool raw, int sh) {
 #pragma unroll 1
   for (int q = 0; q < c.p.steps; ++q) {
-    const bool rw = raw && q == 0;
+    const bool rw = raw && q == 0, tw2 = doubled(q, c.p.steps);
     const int L = c.p.L, lgP = c.p.lgP, NS = c.p.NS[q];
     const unsigned mg = c.p.magic[q];
     switch (c.p.R[q]) {
-      case 2: step<2>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 3: step<3>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 4: step<4>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 5: step<5>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 6: step<6>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 7: step<7>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 8: step<8>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 9: step<9>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 10: step<10>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 12: step<12>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 14: step<14>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 15: step<15>(c.tw, L, lgP, NS, mg, rw, sh); break;
-      case 16: step<16>(c.tw, L, lgP, NS, mg, rw, sh); break;
+      case 2: step<2>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 3: step<3>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 4: step<4>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 5: step<5>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 6: step<6>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 7: step<7>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 8: step<8>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 9: step<9>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 10: step<10>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 12: step<12>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 14: step<14>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 15: step<15>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
+      case 16: step<16>(c.tw, L, lgP, NS, mg, rw, sh, tw2); break;
     }
   }
+}
+
+// maximum or sum over the CTA per pencil (threads of equal t mod P), in a fixed
+// order; two barriers
+template <class S, class F> __device__ __forceinline__ S over_pencil(S v, int P, S *ws, F &&f) {
+  const int t = threadIdx.x, pen = t & (P - 1), W = blockDim.x >> 5;
+  for (int off = P; off < 32; off <<= 1) v = f(v, __shfl_xor_sync(0xffffffffu, v, off));
+  if ((t & 31) < P) ws[(t >> 5) * P + pen] = v;
+  __syncthreads();
+  v = ws[pen];
+  for (int w = 1; w < W; ++w) v = f(v, ws[w * P + pen]);
+  __syncthreads();
+  return v;
+}
+struct Max {
+  __device__ int operator()(int a, int b) const { return max(a, b); }
+};
+struct Sum {
+  template <class S> __device__ S operator()(S a, S b) const { return a + b; }
+};
+__device__ __forceinline__ int scale(const Core &c, int top, int sum) {
+  return pencil_scale(top, sum, c.p.steps, [&](int q) { return c.p.lg[q]; });
+}
+
+// of the pencil of rows 2 p and 2 p + 1
+__device__ __forceinline__ int row_scale(const Core &c, const int *rmax, const float *rsum, int p, int shift, int &em) {
+  const int t0 = rmax[2 * p], t1 = rmax[2 * p + 1], top = max(t0, t1);
+  em = top >> 20;
+  return scale(c, top, sum_word(sum_rebase(rsum[2 * p], t0, top) + sum_rebase(rsum[2 * p + 1], t1, top), top) + shift);
 }
 
 struct SArgs {
@@ -237,7 +178,7 @@ __global__ void __launch_bounds__(768) k_fx_strided(const __grid_constant__ SArg
   extern __shared__ __align__(16) longlong2 sm[];
   const Strided &d = a.s;
   const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x;
-  int *emax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));
+  void *norm_at = sm + (size_t(L) << lgP);
   const int kblocks = (d.kc + P - 1) >> lgP;
   const int o = blockIdx.x / kblocks, kz0 = (blockIdx.x - o * kblocks) << lgP;
   const int pen = t & (P - 1), kz = kz0 + pen;
@@ -245,8 +186,6 @@ __global__ void __launch_bounds__(768) k_fx_strided(const __grid_constant__ SArg
   const int n = d.n, nh = n >> 1;
   const int step_l = T >> lgP;
   for (int op = d.first[blockIdx.y]; op < d.first[blockIdx.y + 1]; ++op) {
-    if (t < P) emax[t] = 0;
-    __syncthreads();
     // load
     const double2 *src = static_cast<const double2 *>(d.src[op]) + (long long)o * d.in_outer + kz;
     const int pr = d.pr[op], pk = d.pk[op];
@@ -265,45 +204,51 @@ __global__ void __launch_bounds__(768) k_fx_strided(const __grid_constant__ SArg
           v.y *= f;
         }
       }
-      em = max(em, max(mag(__double_as_longlong(v.x)), mag(__double_as_longlong(v.y))));
+      em = max(em, mag(I2{__double_as_longlong(v.x), __double_as_longlong(v.y)}));
       sm[slot(l, pen, lgP)] = d.inverse ? make_longlong2(__double_as_longlong(v.y), __double_as_longlong(v.x))
                                         : make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
     }
-    for (int off = P; off < 32; off <<= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, off));
-    if ((t & 31) < P) atomicMax(&emax[pen], em);
-    __syncthreads();
-    em = emax[pen] >> 20;
-    int S = em - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1);
-    transform(a.c, true, shift_of(em, a.c.p.B));
+    em = over_pencil(em, P, static_cast<int *>(norm_at), Max());
+    float sum = 0.f;
+    for (int l = t >> lgP; l < L; l += step_l) {
+      const longlong2 w = sm[slot(l, pen, lgP)];
+      sum += sum_term(mag(I2{w.x, w.y}), sum_base(em));
+    }
+    sum = over_pencil(sum, P, static_cast<float *>(norm_at), Sum());
+    const int k = scale(a.c, em, sum_word(sum, em) + kSqrt2);
+    em >>= 20;
+    const int lost = bits_lost(a.c.p.steps - 1, a.c.p.steps);
+    int S = lost - k;
+    transform(a.c, true, shift_of(em, k));
     bool inverse = d.inverse;
     if (d.truncate) {
-      // keep the N-grid modes, bring the largest back below 2^B, swap for the
-      // inverse transform (inverse = swap, forward, swap)
-      int bits = 0;
+      // keep the N-grid modes, scale for the way back (fx64_len.cuh k_fx_trunc),
+      // swap for the inverse transform (inverse = swap, forward, swap)
+      FixedNorm norm;
       for (int l = t >> lgP; l < L; l += step_l) {
         const bool keep = l < nh || l > n;
         longlong2 &w = sm[slot(l, pen, lgP)];
         const longlong2 v = w;
-        if (keep) bits = max(bits, 64 - min(__clzll(v.x ^ (v.x >> 63)), __clzll(v.y ^ (v.y >> 63))));
+        if (keep) {
+          norm.add(v.x);
+          norm.add(v.y);
+        }
         w = keep ? make_longlong2(v.y, v.x) : make_longlong2(0, 0);
       }
-      if (t < P) emax[t] = 0;
-      __syncthreads();
-      for (int off = P; off < 32; off <<= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, off));
-      if ((t & 31) < P) atomicMax(&emax[pen], bits);
-      __syncthreads();
-      const int down = emax[pen] - a.c.p.B;
+      const int top2 = over_pencil(int(norm.top) + 1, P, static_cast<int *>(norm_at), Max());
+      const unsigned sum2 = over_pencil(norm.thread_sum(), P, static_cast<unsigned *>(norm_at), Sum());
+      const int k2 = scale(a.c, high_word(top2, 32), high_word(sum2, 47) - 0x3ff00000);
       for (int l = t >> lgP; l < L; l += step_l) {
         longlong2 &w = sm[slot(l, pen, lgP)];
-        if (down > 0) {
-          const long long half = 1LL << (down - 1);
-          w = make_longlong2((w.x + half) >> down, (w.y + half) >> down);
+        if (k2 < 0) {
+          const long long half = 1LL << (-k2 - 1);
+          w = make_longlong2((w.x + half) >> -k2, (w.y + half) >> -k2);
         } else {
-          w = make_longlong2(w.x << -down, w.y << -down);
+          w = make_longlong2(w.x << k2, w.y << k2);
         }
       }
       __syncthreads();
-      S += down + 3 * (a.c.p.steps - 1);
+      S += lost - k2;
       transform(a.c, false, 0);
       inverse = true;
     }
@@ -353,12 +298,12 @@ __global__ void __launch_bounds__(768) k_fx_c2r(const __grid_constant__ RArgs a)
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
   const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
-  int *emax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));
+  int *rmax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));  // per row
+  float *rsum = reinterpret_cast<float *>(rmax + 2 * P);
   double *base = static_cast<double *>(d.field[blockIdx.y]);
   const long long row0 = (long long)blockIdx.x * 2 * P;
   const int h = L >> 1, kc = min(d.kc, h);  // the Nyquist value, if any, is handled apart
   const bool nyq = d.kc > h;
-  if (t < P) emax[t] = 0;
   // zero the elements without a mode
   for (int e = t; e < ((L - 2 * kc + 1) << lgP); e += T) sm[slot(kc + (e >> lgP), e & (P - 1), lgP)] = make_longlong2(0, 0);
   __syncthreads();
@@ -376,41 +321,59 @@ __global__ void __launch_bounds__(768) k_fx_c2r(const __grid_constant__ RArgs a)
         em = max(em, mag(__double_as_longlong(v.x)));
         reinterpret_cast<double *>(&sm[slot(0, pen, lgP)])[second] = v.x;
       } else {
-        em = max(em, max(mag(__double_as_longlong(v.x)), mag(__double_as_longlong(v.y))));
+        em = max(em, mag(I2{__double_as_longlong(v.x), __double_as_longlong(v.y)}));
         sm[slot(second ? L - k : k, pen, lgP)] = make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
       }
     }
+    int nyq_word = 0;
     if (nyq && lane == 0) {
       const double v = live ? src[h].x : 0.0;
-      em = max(em, mag(__double_as_longlong(v)));
+      nyq_word = mag(__double_as_longlong(v));
+      em = max(em, nyq_word);
       reinterpret_cast<double *>(&sm[slot(h, pen, lgP)])[second] = v;
     }
     em = __reduce_max_sync(0xffffffffu, unsigned(em));
-    if (lane == 0) atomicMax(&emax[pen], em);
+    const int sb = sum_base(em);
+    float sum = sum_term(nyq_word, sb);
+    for (int k = lane; k < kc; k += 32) {  // what this lane has just written
+      const longlong2 w = sm[slot(second && k ? L - k : k, pen, lgP)];
+      sum += sum_term(k ? mag(I2{w.x, w.y}) : mag(second ? w.y : w.x), sb);
+    }
+    sum = warp_sum(sum);
+    if (lane == 0) {
+      rmax[q] = em;
+      rsum[q] = sum;
+    }
   }
   __syncthreads();
+  // every mode but k = 0 and L / 2 stands in the pencil twice
+  auto scale_of = [&](int p, int &em) { return row_scale(a.c, rmax, rsum, p, kSqrt2 + kTwice, em); };
   {
     // Z of both rows in fixed point, real and imaginary part exchanged (the
     // inverse transform)
-    const int pen = t & (P - 1), sh = shift_of(emax[pen] >> 20, a.c.p.B);
+    const int pen = t & (P - 1);
+    int em;
+    const int k8 = scale_of(pen, em), sh = shift_of(em, k8);
+    const bool round = a.c.p.steps > 2;
+    auto fix = [&](long long b) { return round ? to_fixed_r(b, sh) : to_fixed_p(b, sh); };
     for (int k = t >> lgP; k < kc; k += T >> lgP) {
       longlong2 &wa = sm[slot(k, pen, lgP)];
       const longlong2 va = wa;
-      const long long ax = to_fixed_p(va.x, sh), ay = to_fixed_p(va.y, sh);
+      const long long ax = fix(va.x), ay = fix(va.y);
       if (k == 0) {
         wa = make_longlong2(ay, ax);
         continue;
       }
       longlong2 &wb = sm[slot(L - k, pen, lgP)];
       const longlong2 vb = wb;
-      const long long bx = to_fixed_p(vb.x, sh), by = to_fixed_p(vb.y, sh);
+      const long long bx = fix(vb.x), by = fix(vb.y);
       wa = make_longlong2(ay + bx, ax - by);
       wb = make_longlong2(bx - ay, ax + by);
     }
     if (nyq && t < P) {
       longlong2 &w = sm[slot(h, t, lgP)];
       const longlong2 v = w;
-      w = make_longlong2(to_fixed_p(v.y, sh), to_fixed_p(v.x, sh));
+      w = make_longlong2(fix(v.y), fix(v.x));
     }
   }
   __syncthreads();
@@ -420,8 +383,9 @@ __global__ void __launch_bounds__(768) k_fx_c2r(const __grid_constant__ RArgs a)
     if (row >= d.rows) break;
     double *dst = base + row * d.pitch;
     const int pen = q >> 1, second = q & 1;
-    const int em = emax[pen] >> 20;
-    const OutScale os = out_scale(em, em - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1));
+    int em;
+    const int k = scale_of(pen, em);
+    const OutScale os = out_scale(em, bits_lost(a.c.p.steps - 1, a.c.p.steps) - k);
     for (int e = lane; e < L; e += 32)  // exchanged again: the first row is the imaginary part
       dst[e] = to_double_p(reinterpret_cast<const long long *>(&sm[slot(e, pen, lgP)])[1 - second], os);
   }
@@ -433,11 +397,10 @@ __global__ void __launch_bounds__(768) k_fx_r2c(const __grid_constant__ RArgs a)
   extern __shared__ __align__(16) longlong2 sm[];
   const Rows &d = a.r;
   const int L = a.c.p.L, lgP = a.c.p.lgP, P = 1 << lgP, T = blockDim.x, t = threadIdx.x, lane = t & 31;
-  int *emax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));
+  int *rmax = reinterpret_cast<int *>(sm + (size_t(L) << lgP));  // per row
+  float *rsum = reinterpret_cast<float *>(rmax + 2 * P);
   double *base = static_cast<double *>(d.field[blockIdx.y]);
   const long long row0 = (long long)blockIdx.x * 2 * P;
-  if (t < P) emax[t] = 0;
-  __syncthreads();
   for (int q = t >> 5; q < 2 * P; q += T >> 5) {
     const long long row = row0 + q;
     const bool live = row < d.rows;
@@ -451,10 +414,23 @@ __global__ void __launch_bounds__(768) k_fx_r2c(const __grid_constant__ RArgs a)
       reinterpret_cast<double *>(&sm[slot(e, pen, lgP)])[second] = v;
     }
     em = __reduce_max_sync(0xffffffffu, unsigned(em));
-    if (lane == 0) atomicMax(&emax[pen], em);
+    const int sb = sum_base(em);
+    float sum = 0.f;
+    for (int e = lane; e < L; e += 32)  // what this lane has just written
+      sum += sum_term(mag(reinterpret_cast<const long long *>(&sm[slot(e, pen, lgP)])[second]), sb);
+    sum = warp_sum(sum);
+    if (lane == 0) {
+      rmax[q] = em;
+      rsum[q] = sum;
+    }
   }
   __syncthreads();
-  transform(a.c, true, shift_of(emax[t & (P - 1)] >> 20, a.c.p.B));
+  auto scale_of = [&](int p, int &em) { return row_scale(a.c, rmax, rsum, p, 0, em); };
+  {
+    int em;
+    const int k = scale_of(t & (P - 1), em);
+    transform(a.c, true, shift_of(em, k));
+  }
   const int kc = d.kc;
   for (int q = t >> 5; q < 2 * P; q += T >> 5) {
     const long long row = row0 + q;
@@ -462,8 +438,9 @@ __global__ void __launch_bounds__(768) k_fx_r2c(const __grid_constant__ RArgs a)
     double2 *dst = reinterpret_cast<double2 *>(base + row * d.pitch);
     const int pen = q >> 1, second = q & 1;
     // the sums below are twice the spectra
-    const int em = emax[pen] >> 20;
-    const OutScale os = out_scale(em, em - 1022 - a.c.p.B + 3 * (a.c.p.steps - 1) - 1);
+    int em;
+    const int ks = scale_of(pen, em);
+    const OutScale os = out_scale(em, bits_lost(a.c.p.steps - 1, a.c.p.steps) - ks - 1);
     for (int k = lane; k < kc; k += 32) {
       const longlong2 u = sm[slot(k, pen, lgP)], w = sm[slot(k ? L - k : 0, pen, lgP)];
       // A = (Z[k] + conj Z[L-k]) / 2, B = (Z[k] - conj Z[L-k]) / 2i
@@ -482,120 +459,16 @@ struct LenEntry {
   int L;
   bool padded, grid;
   LenFn fn;
-  int steps, R[3];  // in the order of a forward transform
 };
-extern template struct Launch<16, false, true>;
-extern template struct Launch<24, true, true>;
-extern template struct Launch<32, false, true>;
-extern template struct Launch<48, true, true>;
-extern template struct Launch<64, false, true>;
-extern template struct Launch<72, true, true>;
-extern template struct Launch<96, true, true>;
-extern template struct Launch<128, false, true>;
-extern template struct Launch<144, true, true>;
-extern template struct Launch<192, true, true>;
-extern template struct Launch<256, false, true>;
-extern template struct Launch<288, true, false>;
-extern template struct Launch<384, true, true>;
-extern template struct Launch<512, false, true>;
-extern template struct Launch<576, true, false>;
-extern template struct Launch<768, true, true>;
-extern template struct Launch<1152, true, false>;
-extern template struct Launch<56, false, true>;
-extern template struct Launch<60, false, true>;
-extern template struct Launch<80, false, true>;
-extern template struct Launch<84, true, true>;
-extern template struct Launch<90, true, false>;
-extern template struct Launch<100, false, true>;
-extern template struct Launch<108, true, true>;
-extern template struct Launch<112, false, true>;
-extern template struct Launch<120, true, true>;
-extern template struct Launch<126, true, false>;
-extern template struct Launch<140, false, true>;
-extern template struct Launch<150, true, false>;
-extern template struct Launch<160, false, true>;
-extern template struct Launch<162, true, false>;
-extern template struct Launch<168, true, true>;
-extern template struct Launch<180, true, true>;
-extern template struct Launch<196, false, true>;
-extern template struct Launch<200, false, true>;
-extern template struct Launch<210, true, false>;
-extern template struct Launch<216, true, true>;
-extern template struct Launch<224, false, true>;
-extern template struct Launch<240, true, true>;
-extern template struct Launch<252, true, true>;
-extern template struct Launch<270, true, false>;
-extern template struct Launch<294, true, false>;
-extern template struct Launch<300, true, false>;
-extern template struct Launch<324, true, false>;
-extern template struct Launch<336, true, false>;
-extern template struct Launch<360, true, false>;
-extern template struct Launch<378, true, false>;
-template <int L, bool PADDED, bool GRID> static LenEntry entry() {
-  return {L, PADDED, GRID, Launch<L, PADDED, GRID>::run, Len<L>::steps, {Len<L>::R(0), Len<L>::R(1), Len<L>::R(2)}};
-}
-static const LenEntry kLens[] = {entry<16, false, true>(),
-                                 entry<24, true, true>(),
-                                 entry<32, false, true>(),
-                                 entry<48, true, true>(),
-                                 entry<64, false, true>(),
-                                 entry<72, true, true>(),
-                                 entry<96, true, true>(),
-                                 entry<128, false, true>(),
-                                 entry<144, true, true>(),
-                                 entry<192, true, true>(),
-                                 entry<256, false, true>(),
-                                 entry<288, true, false>(),
-                                 entry<384, true, true>(),
-                                 entry<512, false, true>(),
-                                 entry<576, true, false>(),
-                                 entry<768, true, true>(),
-                                 entry<1152, true, false>(),
-                                 entry<56, false, true>(),
-                                 entry<60, false, true>(),
-                                 entry<80, false, true>(),
-                                 entry<84, true, true>(),
-                                 entry<90, true, false>(),
-                                 entry<100, false, true>(),
-                                 entry<108, true, true>(),
-                                 entry<112, false, true>(),
-                                 entry<120, true, true>(),
-                                 entry<126, true, false>(),
-                                 entry<140, false, true>(),
-                                 entry<150, true, false>(),
-                                 entry<160, false, true>(),
-                                 entry<162, true, false>(),
-                                 entry<168, true, true>(),
-                                 entry<180, true, true>(),
-                                 entry<196, false, true>(),
-                                 entry<200, false, true>(),
-                                 entry<210, true, false>(),
-                                 entry<216, true, true>(),
-                                 entry<224, false, true>(),
-                                 entry<240, true, true>(),
-                                 entry<252, true, true>(),
-                                 entry<270, true, false>(),
-                                 entry<294, true, false>(),
-                                 entry<300, true, false>(),
-                                 entry<324, true, false>(),
-                                 entry<336, true, false>(),
-                                 entry<360, true, false>(),
-                                 entry<378, true, false>()};
+#define FX_EXTERN(L, PADDED, GRID) extern template struct Launch<L, PADDED, GRID>;
+FX_LENGTHS(FX_EXTERN)
+#define FX_ENTRY(L, PADDED, GRID) {L, PADDED, GRID, Launch<L, PADDED, GRID>::run},
+static const LenEntry kLens[] = {FX_LENGTHS(FX_ENTRY)};
 static const LenEntry *find_len(int L) {
   for (const LenEntry &e : kLens)
     if (e.L == L) return &e;
   return nullptr;
 }
-// B of an instance; an inverse transform takes the radices backwards
-static int len_bits(const LenEntry &l, FxKind kind, bool forward, bool inverse) {
-  int rev[3];
-  for (int q = 0; q < l.steps; ++q) rev[q] = l.R[l.steps - 1 - q];
-  int b = 60;
-  if (forward) b = std::min(b, fx_bits(l.R, l.steps, kind));
-  if (inverse) b = std::min(b, fx_bits(rev, l.steps, kind));
-  return b;
-}
-
 static __global__ void k_fx_tables(int n, double *mode, double *rinv, double *root, int len) {
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < len; q += gridDim.x * blockDim.x) {
     rinv[q] = q ? 1.0 / double(q) : 0.0;
@@ -643,13 +516,13 @@ cudaError_t run_strided(const Strided &s, cudaStream_t st) {
     if (s.inverse && !s.cut_out && !s.truncate) op = s.pad_in ? (p ? FX_OP_INV_PAD : op) : (l->grid ? FX_OP_INV : op);
     else if (!s.inverse && !s.pad_in && single) op = !p ? op : (s.truncate ? FX_OP_TRUNC : (s.cut_out ? FX_OP_CUT : op));
     if (op != FX_OP_PREPARE) {
-      const LArgs a{static_cast<const longlong2 *>(s.tw), len_bits(*l, FX_STRIDED, !s.inverse, s.inverse || s.truncate), s};
+      const LArgs a{s.tw, s};
       return l->fn(op, &a, dim3(unsigned(s.outer * ((s.kc + 7) / 8)), unsigned(s.groups)), st);
     }
   }
   SArgs a;
   if (!fx_plan(s.L, FX_STRIDED, &a.c.p)) return cudaErrorInvalidValue;
-  a.c.tw = static_cast<const longlong2 *>(s.tw);
+  a.c.tw = s.tw;
   a.s = s;
   const int kb = (s.kc + a.c.p.P - 1) / a.c.p.P;
   mfx::launch_pdl(k_fx_strided, dim3(unsigned(s.outer * kb), unsigned(s.groups)), a.c.p.T, a.c.p.smem, st, a);
@@ -662,13 +535,13 @@ static cudaError_t run_rows(const Rows &r, FxKind kind, cudaStream_t st) {
     if (kind == FX_C2R) op = l->padded && r.kc <= r.L / 3 + 1 ? FX_OP_C2R_PAD : (l->grid ? FX_OP_C2R : op);
     else if (l->padded && r.kc <= r.L / 3) op = FX_OP_R2C;
     if (op != FX_OP_PREPARE) {
-      const LRows a{static_cast<const longlong2 *>(r.tw), len_bits(*l, kind, kind == FX_R2C, kind == FX_C2R), r};
+      const LRows a{r.tw, r};
       return l->fn(op, &a, dim3(unsigned((r.rows + 15) / 16), unsigned(r.count)), st);
     }
   }
   RArgs a;
   if (!fx_plan(r.L, kind, &a.c.p)) return cudaErrorInvalidValue;
-  a.c.tw = static_cast<const longlong2 *>(r.tw);
+  a.c.tw = r.tw;
   a.r = r;
   const long long per = 2 * a.c.p.P;
   const dim3 grid(unsigned((r.rows + per - 1) / per), unsigned(r.count));

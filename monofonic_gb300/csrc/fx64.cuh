@@ -1,25 +1,29 @@
 // 64-bit fixed-point pencil transforms of the plain FP64 form: the arithmetic,
-// the in-register DFTs and the transform plans (the kernels and their launches
-// are in fx64.cu).
+// the in-register DFTs, the scale of a pencil and the transform plans (the
+// kernels and their launches are in fx64.cu and fx64_len.cuh).
 //
 // GB300 runs FP64 at two fused multiply-adds per SM and clock (measured 1.9)
 // against 64 - 128 integer operations, so an FP64 FFT is bound by the FP64
 // pipe and not by HBM: cuFFT's D2Z / Z2D ran at 0.13 TB/s (256^3, padded 384).
 // A pencil (one 1D transform) is therefore transformed in 64-bit integers with
-// one exponent per pencil: every value is scaled by the same power of two so
-// that the largest |re|, |im| lies just below 2^B, and B leaves room for the
-// growth of the steps, so that nothing can overflow (FxPlan::B).  Additions are
+// one exponent per pencil: every value is scaled by the same power of two,
+// chosen from the pencil's sum of magnitudes and its largest component so that
+// no intermediate can leave 64 bits (pencil_scale).  Additions are
 // exact; a multiplication by a twiddle or an internal constant is rounded at
-// the last bit of a 61-63 bit integer.  The error is absolute and below
-// 2^-53 of the pencil's rms at the lengths used, where an FP64 FFT's is a few
-// 2^-53: measured against 64-bit references it is no larger than cuFFT's
-// (fields 1e-16 - 1e-15 of their norm).  Multiplications (three 32x32+64
+// the last bit of a 61-63 bit integer.  What is lost is absolute, a few units
+// of the last place for every step.  Against long double, relative to the
+// output's norm and rounded to double, pencils with amplitudes from flat to k^-4
+// are off by 5e-17 to 1.0e-16 in two steps, to 1.5e-16 in three and as c2r to
+// 1.8e-16; numpy's FP64 transforms of them by 1.1e-16 to 2.8e-16, and in no case
+// by less (tests/test_fx64_range.py).  Multiplications (three 32x32+64
 // products each, 12.7 a clock and SM measured) cost more than additions here,
 // which is what the radices and the rotations below are chosen for.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <cmath>
 #include <utility>
 
 namespace fx {
@@ -301,8 +305,122 @@ template <> struct Dft<7> {
   }
 };
 
-// v / 8, rounded (the element that a step's twiddles leave alone)
-FX_HD I2 eighth(I2 v) { return {(v.x + 4) >> 3, (v.y + 4) >> 3}; }
+// Twiddle constants are held as w 2^62, so a product with one is a quarter of
+// v w; the element that a step's twiddles leave alone is quartered like them.
+// Three products: c = cos, s = -sin, the constants c, s + c and s - c split into
+// signed halves (hi, lo)
+FX_HD I2 quarter(I2 v) { return {(v.x + 2) >> 2, (v.y + 2) >> 2}; }
+FX_HD I2 twiddle4(I2 v, int4 c_p, int2 m) {
+  const long long k = mulq(v.x + v.y, c_p.x, c_p.y);
+  return {k - mulq(v.y, c_p.z, c_p.w), k + mulq(v.x, m.x, m.y)};
+}
+// the constants of (cos, -sin)(2 pi t / L)
+inline void twiddle_constants(int t, int L, int4 *c_p, int2 *m) {
+  const CS w = q62_turn(t, L);
+  const long long c = (long long)w.c, s = (long long)-w.s;
+  auto lo = [](long long w) { return int(w); };
+  auto hi = [](long long w) { return int(w >> 32) + int(unsigned(int(w)) >> 31); };
+  *c_p = make_int4(hi(c), lo(c), hi(s + c), lo(s + c));
+  *m = make_int2(hi(s - c), lo(s - c));
+}
+
+// ---------------------------------------------------------------------------
+// scale of a pencil
+// ---------------------------------------------------------------------------
+// log2 v in Q20, rounded up
+FX_HD constexpr int log2_q20(int v) {
+  double m = v;
+  int r = 0;
+  for (; m >= 2.0; m *= 0.5) r += 1 << 20;
+  for (int bit = 1 << 19; bit; bit >>= 1)
+    if ((m *= m) >= 2.0) {
+      m *= 0.5;
+      r += bit;
+    }
+  return r + 1;
+}
+// The power k of two that a pencil's values are multiplied by.  `top` is the high
+// word of its largest component, `sum` a high word without the bias of its sum of
+// magnitudes (or of a bound of it); a double's high word, taken as a number, is a
+// logarithm to base 2 in Q20 that is low by at most 0.0861.  Every intermediate of step q is a sum of inputs times
+// factors of modulus at most one, each input once, over 2^bits_lost(q): its
+// modulus stays below the pencil's sum of magnitudes, and below the product of the
+// radices so far times sqrt(2) times the largest component (lg[q], its logarithm).  The
+// largest operand that the arithmetic makes of an intermediate of modulus A is
+// 2 sqrt(2) A (the doubled sum of both components in an eighth turn), so
+// A < 2^61.5 keeps all of them below 2^63.  The first bound is the smaller one
+// where a few modes hold the pencil, the steep spectra of potentials and
+// displacements, which then keep all their bits; the second one is for flat
+// spectra, whose sums grow by the root of the length.  Scaled by the second bound
+// alone, less what the steps lose, a flat pencil at length 72 left the range, and
+// k^-2 pencils were off by 2e-16 at length 256 and 4e-16 at 384.  The sums cost 1%
+// of a 256^3 3LPT pass (27.9 -> 28.2 ms) and 3% at 64^3 (203 -> 209 us).
+// The twiddles of a step quarter its inputs.  Of three steps, where an intermediate
+// of few large terms has not grown yet, the second one's are doubled before (half
+// lost): k^-1 spectra of three-step c2r transforms are off by up to 1.8e-16 so,
+// 2.7e-16 with quarters only, numpy's FP64 transforms of them by 2.3e-16.
+FX_HD constexpr int bits_lost(int q, int steps) { return q == 0 ? 0 : (steps > 2 ? 2 * q - 1 : 2 * q); }
+constexpr bool doubled(int q, int steps) { return q == 1 && steps > 2; }
+constexpr int kScaleTop = int((61.5 - 0.0862) * 1048576.0);
+template <class G> FX_HD int pencil_scale(int top, int sum, int steps, G lg) {
+  const int m = top - 0x3ff00000 + 1, s = sum + 1;
+  int v = -0x7fffffff;
+#pragma unroll
+  for (int q = 0; q < steps; ++q) {
+    const int g = m + lg(q);
+    const int b = (s < g ? s : g) - (bits_lost(q, steps) << 20);
+    v = b > v ? b : v;
+  }
+  return (kScaleTop - v) >> 20;
+}
+// Magnitudes are summed in single precision, whose pipe is idle in these kernels
+// (FP64 additions made the passes 14% longer at 256^3, a third at 64^3): high words
+// relative to a base 120 binades below the largest one are moved to a float's
+// place.  What lies below the base counts as it, which is nothing.
+FX_HD int sum_base(int top) { return (top & 0x7ff00000) - (120 << 20); }
+FX_HD float as_float(int b) {
+#ifdef __CUDA_ARCH__
+  return __int_as_float(b);
+#else
+  float f;
+  __builtin_memcpy(&f, &b, 4);
+  return f;
+#endif
+}
+FX_HD int as_int(float f) {
+#ifdef __CUDA_ARCH__
+  return __float_as_int(f);
+#else
+  int b;
+  __builtin_memcpy(&b, &f, 4);
+  return b;
+#endif
+}
+FX_HD float sum_term(int word, int base) { return as_float(((word > base ? word : base) - base) << 3); }
+// a sum taken to the base of `top`, brought to the base of a larger `to`
+FX_HD float sum_rebase(float f, int top, int to) {
+  const int e = 127 - ((to >> 20) - (top >> 20));
+  return f * as_float(e > 0 ? e << 23 : 0);
+}
+// the high word without the bias of a sum
+FX_HD int sum_word(float f, int top) { return (as_int(f) >> 3) + (sum_base(top) - 0x3ff00000); }
+constexpr int kSqrt2 = 1 << 19, kTwice = 1 << 20;  // added to a sum's word: times sqrt(2), times two
+
+// conversion of a pencil whose largest component has the biased exponent em:
+// scale -> right shift of to_fixed_p.  A pencil whose values all lie below
+// 2^-959 counts as zero.
+FX_HD int shift_of(int em, int k) { return em < 64 ? 8192 : 1085 - k; }
+FX_HD long long to_fixed_p(long long b, int sh) {
+  const int d0 = sh - (int(b >> 52) & 0x7ff), d = d0 < 63 ? d0 : 63;
+  const long long m = (long long)(((unsigned long long)((b & 0xfffffffffffffLL) | 0x10000000000000LL) << 10) >> d);
+  const long long sg = b >> 63;
+  return (m ^ sg) - sg;
+}
+// rounded: for c2r transforms of three steps, whose values are sums of two
+FX_HD long long to_fixed_r(long long b, int sh) {
+  const long long t = to_fixed_p(b & 0x7fffffffffffffffLL, sh - 1), m = (t + 1) >> 1, sg = b >> 63;
+  return (m ^ sg) - sg;
+}
 
 // v 2^S -> double, rounded to nearest; S + 1086 is the biased exponent of bit 63
 FX_HD double to_double(long long v, int S) {
@@ -341,19 +459,85 @@ struct FxPlan {
   unsigned magic[kMaxSteps];  // ceil(2^32 / NS): j / NS by a multiplication
   int P, lgP;           // pencils per CTA
   int T;                // threads per CTA
-  int B;                // largest component of the input lies below 2^B
+  int lg[kMaxSteps];    // growth bound after a step (pencil_scale)
   int smem;             // bytes
 };
 
+// a c2r pencil's components are sums of two of its rows' components
 enum FxKind { FX_STRIDED = 0, FX_C2R = 1, FX_R2C = 2 };
 
-// B of a transform of the given radices: a step of radix R lets a modulus grow
-// by R, the twiddles after it take three bits off; a c2r pencil holds two rows,
-// an r2c pencil's spectra are separated by sums.  62.7 bits at most
-int fx_bits(const int *R, int steps, FxKind kind);
+constexpr int kSmemMax = 220 * 1024;
+
+// rough cost of a point: real multiplications (three products each, measured
+// 4 a clock) and the shared-memory round trip of a step
+inline double radix_cost(int R) {
+  switch (R) {
+    case 2: case 4: return 0.0;
+    case 3: return 0.67; case 5: return 2.0; case 6: return 0.67; case 7: return 5.1;
+    case 8: return 0.5; case 9: return 2.0; case 10: return 2.0; case 12: return 0.67;
+    case 14: return 5.1; case 15: return 2.67; default: return 1.25;  // 16
+  }
+}
+
+// best factorisation: fewest steps, then least cost, then smallest largest radix
+inline void plan_search(int rest, int depth, double cost, int *cur, int &best_n, double &best_c, int *best) {
+  constexpr int kRadices[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  if (rest == 1) {
+    int mx = 0;
+    for (int q = 0; q < depth; ++q) mx = std::max(mx, cur[q]);
+    const double c = cost + 0.02 * mx;
+    if (depth < best_n || (depth == best_n && c < best_c)) {
+      best_n = depth;
+      best_c = c;
+      std::copy(cur, cur + depth, best);
+    }
+    return;
+  }
+  if (depth == kMaxSteps || depth >= best_n) return;
+  for (int R : kRadices)
+    if (rest % R == 0 && (depth == 0 || R <= cur[depth - 1])) {
+      cur[depth] = R;
+      plan_search(rest / R, depth + 1, cost + radix_cost(R), cur, best_n, best_c, best);
+    }
+}
+
+// lg of a step: the radices up to it, sqrt(2), and 2 for a c2r pencil
+FX_HD constexpr int growth(int radices, FxKind kind) { return log2_q20(radices) + (1 << 19) + (kind == FX_C2R ? 1 << 20 : 0); }
 
 // false where a length has a prime factor above 7 or fits no CTA
-bool fx_plan(int L, FxKind kind, FxPlan *p);
+inline bool fx_plan(int L, FxKind kind, FxPlan *p) {
+  *p = FxPlan{};
+  p->L = L;
+  int cur[kMaxSteps], best[kMaxSteps], n = kMaxSteps + 1;
+  double c = 1e30;
+  plan_search(L, 0, 0.0, cur, n, c, best);
+  if (n > kMaxSteps) return false;
+  p->steps = n;
+  // smallest radix first: its butterflies, the most, carry no twiddles
+  std::sort(best, best + n);
+  int ns = 1;
+  for (int q = 0; q < n; ++q) {
+    p->R[q] = best[q];
+    p->NS[q] = ns;
+    p->magic[q] = unsigned((0x100000000ULL + unsigned(ns) - 1) / unsigned(ns));
+    ns *= best[q];
+    p->lg[q] = growth(ns, kind);
+  }
+  for (int P : {8, 4, 2, 1}) {
+    int need = 32;  // threads: a butterfly each
+    for (int q = 0; q < n; ++q) need = std::max(need, P * (L / p->R[q]));
+    const int T = (need + 31) / 32 * 32;
+    // pencils, then a number for each warp and pencil, or two for each row
+    const int smem = L * P * 16 + std::max(T / 32, 4) * P * 4;
+    if (T > 768 || smem > kSmemMax) continue;
+    p->P = P;
+    p->lgP = P == 8 ? 3 : (P == 4 ? 2 : P - 1);
+    p->T = T;
+    p->smem = smem;
+    return true;
+  }
+  return false;
+}
 inline bool fx_supported(int L) {
   FxPlan p;
   return L >= 8 && L % 2 == 0 && fx_plan(L, FX_STRIDED, &p) && fx_plan(L, FX_C2R, &p) && fx_plan(L, FX_R2C, &p);

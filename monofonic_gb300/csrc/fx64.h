@@ -13,8 +13,8 @@ namespace fx {
 bool length_supported(int L);
 // twiddle tables of a length (host memory, kept for the process: some KB for
 // each length that was asked for)
-const longlong2 *twiddles(int L);
-inline size_t twiddle_bytes(int L) { return (size_t(L) * 40 + 15) / 16 * 16; }
+const void *twiddles(int L);
+inline size_t twiddle_bytes(int L) { return (size_t(L) * 24 + 15) / 16 * 16; }
 // device tables of a grid: mode[0..1][n] (Strided::mode), mode[2][n] the
 // fractional part and mode[4][n] (as int) the integer part of the PLT table
 // coordinate x = i * (64 / n), mode[3][n] the signed mode index that x stands for,

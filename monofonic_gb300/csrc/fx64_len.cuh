@@ -81,36 +81,57 @@ FX_LEN(336, 2, 14, 24, 1, 192, 2, 3)
 FX_LEN(360, 2, 20, 18, 1, 160, 3, 4)
 FX_LEN(378, 2, 18, 21, 1, 192, 2, 3)
 #undef FX_LEN
+// the instances: length, as padded length, as grid length
+#define FX_LENGTHS(X) \
+  X(16, false, true) X(24, true, true) X(32, false, true) X(48, true, true) X(64, false, true) X(72, true, true) \
+  X(96, true, true) X(128, false, true) X(144, true, true) X(192, true, true) X(256, false, true) \
+  X(288, true, false) X(384, true, true) X(512, false, true) X(576, true, false) X(768, true, true) \
+  X(1152, true, false) X(56, false, true) X(60, false, true) X(80, false, true) X(84, true, true) \
+  X(90, true, false) X(100, false, true) X(108, true, true) X(112, false, true) X(120, true, true) \
+  X(126, true, false) X(140, false, true) X(150, true, false) X(160, false, true) X(162, true, false) \
+  X(168, true, true) X(180, true, true) X(196, false, true) X(200, false, true) X(210, true, false) \
+  X(216, true, true) X(224, false, true) X(240, true, true) X(252, true, true) X(270, true, false) \
+  X(294, true, false) X(300, true, false) X(324, true, false) X(336, true, false) X(360, true, false) \
+  X(378, true, false)
 
-// the three constants of a twiddle product (fx64.cuh twiddle8), each split into
-// signed 32-bit halves
+// the constants of the twiddle products (fx64.cuh twiddle4) of a length
 struct Tw3 {
   const int4 *cp;  // c: hi, lo; s + c: hi, lo
   const int2 *m;   // s - c: hi, lo
 };
-__device__ __forceinline__ Tw3 tw3_of(const longlong2 *table, int L) {
-  const int4 *cp = reinterpret_cast<const int4 *>(table + L);
+__device__ __forceinline__ Tw3 tw3_of(const void *table, int L) {
+  const int4 *cp = static_cast<const int4 *>(table);
   return {cp, reinterpret_cast<const int2 *>(cp + L)};
 }
-__device__ __forceinline__ I2 twiddle8(I2 v, const Tw3 &t, int at) {
-  const int4 cp = __ldg(&t.cp[at]);
-  const int2 m = __ldg(&t.m[at]);
-  const long long k = mulq(v.x + v.y, cp.x, cp.y);
-  return {k - mulq(v.y, cp.z, cp.w), k + mulq(v.x, m.x, m.y)};
-}
+__device__ __forceinline__ I2 twiddle4(I2 v, const Tw3 &t, int at) { return twiddle4(v, __ldg(&t.cp[at]), __ldg(&t.m[at])); }
 
 // high word without the sign: its maximum has the largest exponent
 __device__ __forceinline__ int mag(long long b) { return int(b >> 32) & 0x7fffffff; }
+// the larger component's of a value that is still a double; sqrt(2) times it is no
+// less than the modulus
+__device__ __forceinline__ int mag(I2 v) { return max(mag(v.x), mag(v.y)); }
 
-// conversion of a pencil: largest exponent em -> right shift of to_fixed_p.
-// A pencil whose values all lie below 2^-959 counts as zero.
-__device__ __forceinline__ int shift_of(int em, int B) { return em < 64 ? 8192 : em + 63 - B; }
-__device__ __forceinline__ long long to_fixed_p(long long b, int sh) {
-  const int d = min(sh - (int(b >> 52) & 0x7ff), 63);
-  const long long m = (long long)(((unsigned long long)((b & 0xfffffffffffffLL) | 0x10000000000000LL) << 10) >> d);
-  const long long sg = b >> 63;
-  return (m ^ sg) - sg;
+// high word, with and without the bias, of a double that is v 2^e rounded up
+__device__ __forceinline__ int high_word(unsigned v, int e) {
+  return (__float_as_int(__uint2float_ru(v)) >> 3) + ((1023 - 127 + e) << 20);
 }
+// Magnitudes of a pencil in fixed point, for the scale of the transform that
+// follows: the largest |high word| and their sum, taken in units of 2^39 a value
+// and 2^47 a thread, rounded up.
+struct FixedNorm {
+  unsigned top = 0, sum = 0;
+  __device__ __forceinline__ void add(long long v) {
+    const unsigned h = unsigned(int(v >> 32) ^ int(v >> 63));
+    top = max(top, h);
+    sum += (h >> 7) + 1;
+  }
+  __device__ __forceinline__ unsigned thread_sum() const { return (sum >> 8) + 1; }
+};
+// over a warp, in a fixed order; f < 2^7
+__device__ __forceinline__ float warp_sum(float f) {
+  return float(int(__reduce_add_sync(0xffffffffu, unsigned(__float2int_ru(f * 524288.f))))) * (1.f / 524288.f);
+}
+
 // Back: values times 2^S; where the exponents leave the range of a double, or
 // the input was not finite, every value of the pencil is alt (high word).  The
 // conversion is the FP64 pipe's, which has nothing else to do in these kernels
@@ -141,9 +162,18 @@ template <int L, bool REV> struct Fft {
   static FX_HD constexpr int NS(int q) { return q == 0 ? 1 : NS(q - 1) * R(q - 1); }
   // butterflies of step q a thread holds
   static FX_HD constexpr int MU(int q) { return (P * (L / R(q)) + T - 1) / T; }
-  static constexpr int last = D::steps - 1;
-  // pencils, two sets of per-warp maxima
-  static constexpr int smem = L * P * 16 + 2 * W * 8 * 4;
+  static constexpr int last = D::steps - 1, lost = bits_lost(last, steps);
+  // pencils, then a maximum and a sum of each warp and pencil, twice (k_fx_trunc),
+  // or of each of the 16 rows
+  static constexpr int norms = W * P * 16 > 128 ? W * P * 16 : 128;
+  static constexpr int smem = L * P * 16 + norms;
+  // scale of a pencil (fx64.cuh)
+  template <FxKind KIND> static __device__ __forceinline__ int scale(int top, int sum) {
+    return pencil_scale(top, sum, steps, [](int q) {
+      constexpr int lg[3] = {growth(R(0), KIND), growth(R(0) * R(1), KIND), growth(L, KIND)};
+      return lg[q];
+    });
+  }
 
   static __device__ __forceinline__ int slot(int e, int pen) { return (e << lgP) + (pen ^ (e & (P - 1))); }
 
@@ -192,9 +222,13 @@ template <int L, bool REV> struct Fft {
       if (live<Q>(m)) {
         if constexpr (Q > 0) {
           const int inc = (jof<Q>(m) % ns) * (L / (ns * R(Q)));
-          g.v[m][0] = eighth(g.v[m][0]);
+          if constexpr (doubled(Q, steps)) {
 #pragma unroll
-          for (int r = 1; r < R(Q); ++r) g.v[m][r] = twiddle8(g.v[m][r], tw, r * inc);
+            for (int r = 0; r < R(Q); ++r) g.v[m][r] = g.v[m][r] + g.v[m][r];
+          }
+          g.v[m][0] = quarter(g.v[m][0]);
+#pragma unroll
+          for (int r = 1; r < R(Q); ++r) g.v[m][r] = twiddle4(g.v[m][r], tw, r * inc);
         }
         Dft<R(Q)>::run(g.v[m]);
       }
@@ -213,17 +247,84 @@ template <int L, bool REV> struct Fft {
       out(g);
     }
   }
-  // largest value over the CTA per pencil (lanes of equal low three bits)
-  static __device__ __forceinline__ int pencil_max(int v, int *wm) {
+  // Maximum and sum over the CTA per pencil (lanes of equal low three bits): a
+  // warp's four lanes of a pencil first, then the warps, split among these lanes
+  // again.  The order is fixed: the scale that comes of it is the same every run.
+  static __device__ __forceinline__ int lanes_max(int v) {
     v = max(v, __shfl_xor_sync(0xffffffffu, v, 8));
-    v = max(v, __shfl_xor_sync(0xffffffffu, v, 16));
+    return max(v, __shfl_xor_sync(0xffffffffu, v, 16));
+  }
+  template <class S> static __device__ __forceinline__ S lanes_sum(S v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v + __shfl_xor_sync(0xffffffffu, v, 16);
+  }
+  static __device__ __forceinline__ float rebase(float f, int top, int to) { return sum_rebase(f, top, to); }
+  static __device__ __forceinline__ unsigned rebase(unsigned f, int, int) { return f; }
+  template <class S> static __device__ __forceinline__ void pencil_norm(int &top, S &sum, int *wm) {
     const int t = threadIdx.x;
-    if ((t & 31) < 8) wm[(t >> 5) * 8 + (t & 7)] = v;
-    __syncthreads();
-    v = wm[t & 7];
+    S *ws = reinterpret_cast<S *>(wm + W * P);
+    int own = top;
+    top = lanes_max(own);
+    sum = lanes_sum(rebase(sum, own, top));
+    if constexpr (W > 1) {
+      if ((t & 31) < 8) {
+        wm[(t >> 5) * 8 + (t & 7)] = top;
+        ws[(t >> 5) * 8 + (t & 7)] = sum;
+      }
+      __syncthreads();
+      constexpr int N = (W + 3) / 4;
+      int wt[N];
+      own = 0;
 #pragma unroll
-    for (int w = 1; w < W; ++w) v = max(v, wm[w * 8 + (t & 7)]);
-    return v;
+      for (int q = 0; q < N; ++q) {
+        const int w = 4 * q + ((t >> 3) & 3);
+        wt[q] = W % 4 == 0 || w < W ? wm[w * 8 + (t & 7)] : 0;
+        own = max(own, wt[q]);
+      }
+      top = lanes_max(own);
+      sum = 0;
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const int w = 4 * q + ((t >> 3) & 3);
+        if (W % 4 == 0 || w < W) sum += rebase(ws[w * 8 + (t & 7)], wt[q], top);
+      }
+      sum = lanes_sum(sum);
+    }
+  }
+  // scale of the strided passes' pencils from the inputs r that `take` names, and
+  // the exponent of their largest component
+  template <class G, class T> static __device__ __forceinline__ int norm_scale(const G &g, longlong2 *sm, int &em, T &&take) {
+    em = 0;
+#pragma unroll
+    for (int m = 0; m < MU(0); ++m)
+      if (live<0>(m)) {
+#pragma unroll
+        for (int r = 0; r < R(0); ++r)
+          if (take(r)) em = max(em, mag(g.v[m][r]));
+      }
+    const int base = sum_base(em);
+    float sum = 0.f;
+#pragma unroll
+    for (int m = 0; m < MU(0); ++m)
+      if (live<0>(m)) {
+#pragma unroll
+        for (int r = 0; r < R(0); ++r)
+          if (take(r)) sum += sum_term(mag(g.v[m][r]), base);
+      }
+    pencil_norm(em, sum, norm_at(sm));
+    const int k = scale<FX_STRIDED>(em, sum_word(sum, em) + kSqrt2);
+    em >>= 20;
+    return k;
+  }
+  // where the norms lie: [warp][pencil], the z passes' [row]
+  static __device__ __forceinline__ int *norm_at(longlong2 *sm) { return reinterpret_cast<int *>(sm + L * P); }
+  static __device__ __forceinline__ float *row_sums(longlong2 *sm) { return reinterpret_cast<float *>(norm_at(sm) + 2 * P); }
+  // scale of the pencil of rows 2 p and 2 p + 1
+  template <FxKind KIND> static __device__ __forceinline__ int row_scale(longlong2 *sm, int p, int shift, int &em) {
+    const int t0 = norm_at(sm)[2 * p], t1 = norm_at(sm)[2 * p + 1], top = max(t0, t1);
+    const float sum = sum_rebase(row_sums(sm)[2 * p], t0, top) + sum_rebase(row_sums(sm)[2 * p + 1], t1, top);
+    em = top >> 20;
+    return scale<KIND>(top, sum_word(sum, top) + shift);
   }
 };
 
@@ -236,13 +337,11 @@ template <int R> FX_HD constexpr Zone zone(int r) {
 }
 
 struct LArgs {
-  const longlong2 *tw;
-  int B;
+  const void *tw;
   Strided s;
 };
 struct LRows {
-  const longlong2 *tw;
-  int B;
+  const void *tw;
   Rows r;
 };
 
@@ -255,7 +354,6 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_inv(const __grid
   const Strided &d = a.s;
   constexpr int R0 = F::R(0), nb = L / R0, nh = L / 3, n = 2 * nh;
   const int t = threadIdx.x, pen = t & 7;
-  int *wm = reinterpret_cast<int *>(sm + L * 8);
   const Tw3 tw = tw3_of(a.tw, L);
   const int kblocks = (d.kc + 7) >> 3;
   const int o = blockIdx.x / kblocks, kz = ((blockIdx.x - o * kblocks) << 3) + pen;
@@ -301,16 +399,9 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_inv(const __grid
           }
         }
     }
-    int em = 0;
-#pragma unroll
-    for (int m = 0; m < F::MU(0); ++m)
-      if (F::template live<0>(m)) {
-#pragma unroll
-        for (int r = 0; r < R0; ++r)
-          if (!PAD || zone<R0>(r) != Z_PAD) em = max(em, max(mag(g.v[m][r].x), mag(g.v[m][r].y)));
-      }
-    em = F::pencil_max(em, wm) >> 20;
-    const int sh = shift_of(em, a.B);
+    int em;
+    const int k = F::norm_scale(g, sm, em, [](int r) { return !PAD || zone<R0>(r) != Z_PAD; });
+    const int sh = shift_of(em, k);
     // inverse transform: real and imaginary part exchanged, here and at the end
 #pragma unroll
     for (int m = 0; m < F::MU(0); ++m)
@@ -323,7 +414,7 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx_inv(const __grid
     F::template butterfly<0>(g, tw);
     F::template store<0>(g, sm, pen);
     __syncthreads();
-    const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1));
+    const OutScale os = out_scale(em, F::lost - k);
     double2 *dst = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + kz;
     F::template rest<1>(sm, pen, tw, [&](auto &h) {
       constexpr int Q = F::last;
@@ -350,7 +441,6 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   const Strided &d = a.s;
   constexpr int R0 = F::R(0), nb = L / R0, nh = L / 3, n = 2 * nh;
   const int t = threadIdx.x, pen = t & 7;
-  int *wm = reinterpret_cast<int *>(sm + L * 8);
   const Tw3 tw = tw3_of(a.tw, L);
   const int kblocks = (d.kc + 7) >> 3;
   const int o = blockIdx.x / kblocks, kz0 = (blockIdx.x - o * kblocks) << 3, kz = kz0 + pen;
@@ -370,15 +460,9 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
         g.v[m][r] = {__double_as_longlong(v.x), __double_as_longlong(v.y)};
       }
     }
-  int em = 0;
-#pragma unroll
-  for (int m = 0; m < F::MU(0); ++m)
-    if (F::template live<0>(m)) {
-#pragma unroll
-      for (int r = 0; r < R0; ++r) em = max(em, max(mag(g.v[m][r].x), mag(g.v[m][r].y)));
-    }
-  em = F::pencil_max(em, wm) >> 20;
-  const int sh = shift_of(em, a.B);
+  int em;
+  const int k = F::norm_scale(g, sm, em, [](int) { return true; });
+  const int sh = shift_of(em, k);
 #pragma unroll
   for (int m = 0; m < F::MU(0); ++m)
     if (F::template live<0>(m)) {
@@ -388,7 +472,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   F::template butterfly<0>(g, tw);
   F::template store<0>(g, sm, pen);
   __syncthreads();
-  const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1));
+  const OutScale os = out_scale(em, F::lost - k);
   double2 *dst = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + kz;
   F::template rest<1>(sm, pen, tw, [&](auto &h) {
     constexpr int Q = F::last, RL = F::R(Q);
@@ -433,16 +517,16 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   extern __shared__ __align__(16) longlong2 sm[];
   const Strided &d = a.s;
   constexpr int R0 = F::R(0), nb = L / R0, RL = F::R(F::last);
+  static_assert(F::W > 1, "the second norm's barrier stands before shared memory is written again");
   static_assert(RL == I::R(0), "the forward transform's last radix is the inverse one's first");
   const int t = threadIdx.x, pen = t & 7;
-  int *wm = reinterpret_cast<int *>(sm + L * 8);
   const Tw3 tw = tw3_of(a.tw, L);
   const int kblocks = (d.kc + 7) >> 3;
   const int o = blockIdx.x / kblocks, kz = ((blockIdx.x - o * kblocks) << 3) + pen;
   const bool lv = kz < d.kc;
   const int op = blockIdx.y;
   typename I::template Regs<0> h;
-  int em, S;
+  int em, k;
   {
     const double2 *src = static_cast<const double2 *>(d.src[op]) + (long long)o * d.in_outer + kz;
     typename F::template Regs<0> g;
@@ -458,15 +542,8 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
           g.v[m][r] = {__double_as_longlong(v.x), __double_as_longlong(v.y)};
         }
       }
-    em = 0;
-#pragma unroll
-    for (int m = 0; m < F::MU(0); ++m)
-      if (F::template live<0>(m)) {
-#pragma unroll
-        for (int r = 0; r < R0; ++r) em = max(em, max(mag(g.v[m][r].x), mag(g.v[m][r].y)));
-      }
-    em = F::pencil_max(em, wm) >> 20;
-    const int sh = shift_of(em, a.B);
+    k = F::norm_scale(g, sm, em, [](int) { return true; });
+    const int sh = shift_of(em, k);
 #pragma unroll
     for (int m = 0; m < F::MU(0); ++m)
       if (F::template live<0>(m)) {
@@ -479,7 +556,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   }
   // the modes outside the N-grid and on its Nyquist row fall away; real and
   // imaginary part are exchanged for the inverse transform
-  int bits = 0;
+  FixedNorm norm;
   F::template rest<1>(sm, pen, tw, [&](auto &g) {
 #pragma unroll
     for (int m = 0; m < F::MU(F::last); ++m)
@@ -490,15 +567,19 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
           const Zone z = zone<RL>(r);
           I2 v = g.v[m][r];
           if (z == Z_NYQ || z == Z_PAD || (z == Z_EDGE && j == 0)) v = {0, 0};
-          bits |= int((v.x ^ (v.x >> 63)) >> 32) | int((v.y ^ (v.y >> 63)) >> 32);
+          norm.add(v.x);
+          norm.add(v.y);
           h.v[m][r] = {v.y, v.x};
         }
       }
   });
-  // bring the largest back below 2^B.  Its high word decides: a pencil whose
-  // values all lie below 2^32 is far below the rounding of the first transform
-  bits = 32 - __clz(I::pencil_max(bits, wm + F::W * 8)) + 32;
-  const int down = bits - a.B, dn = max(down, 0), up = max(-down, 0);
+  // the scale of the way back, from the high words: a pencil whose values all lie
+  // below 2^32 is far below the rounding of the first transform
+  int top2 = int(norm.top) + 1;
+  unsigned sum2 = norm.thread_sum();
+  I::pencil_norm(top2, sum2, I::norm_at(sm) + 2 * F::W * 8);
+  const int k2 = I::template scale<FX_STRIDED>(high_word(top2, 32), high_word(sum2, 47) - 0x3ff00000);
+  const int dn = max(-k2, 0), up = max(k2, 0);
   const long long half = dn ? 1LL << (dn - 1) : 0;
 #pragma unroll
   for (int m = 0; m < I::MU(0); ++m)
@@ -511,8 +592,7 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   I::template butterfly<0>(h, tw);
   I::template store<0>(h, sm, pen);
   __syncthreads();
-  S = em - 1022 - a.B + down + 6 * (F::steps - 1);
-  const OutScale os = out_scale(em, S);
+  const OutScale os = out_scale(em, 2 * F::lost - k - k2);
   double2 *dst = static_cast<double2 *>(d.dst[op]) + (long long)o * d.out_outer + kz;
   I::template rest<1>(sm, pen, tw, [&](auto &g) {
     constexpr int Q = I::last;
@@ -537,7 +617,6 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_c2r_l(const __g
   const Rows &d = a.r;
   constexpr int h = L / 2, kmax = PAD ? L / 3 + 1 : h, NL = (kmax + 31) / 32;
   const int t = threadIdx.x, lane = t & 31, pen = t & 7;
-  int *rmax = reinterpret_cast<int *>(sm + L * 8);  // per row
   const Tw3 tw = tw3_of(a.tw, L);
   double *base = static_cast<double *>(d.field[blockIdx.y]);
   const long long row0 = (long long)blockIdx.x * 16;
@@ -563,42 +642,56 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_c2r_l(const __g
       const int k = lane + 32 * c;
       if (k >= (PAD ? kmax : h)) continue;
       const longlong2 b = make_longlong2(__double_as_longlong(v[c].x), __double_as_longlong(v[c].y));
-      em = max(em, max(mag(b.x), mag(b.y)));
+      em = max(em, mag(I2{b.x, b.y}));
       if (k == 0) reinterpret_cast<long long *>(&sm[F::slot(0, p)])[second] = b.x;
       else sm[F::slot(second ? L - k : k, p)] = b;
     }
+    int nyq_word = 0;
     if (!PAD && lane == 0) {
       // the Nyquist value (zero where the spectrum ends before it)
       const double x = nyq && lv ? src[h].x : 0.0;
-      em = max(em, mag(__double_as_longlong(x)));
+      nyq_word = mag(__double_as_longlong(x));
+      em = max(em, nyq_word);
       reinterpret_cast<double *>(&sm[F::slot(h, p)])[second] = x;
     }
     em = int(__reduce_max_sync(0xffffffffu, unsigned(em)));
-    if (lane == 0) rmax[q] = em;
+    const int sb = sum_base(em);
+    float sum = sum_term(nyq_word, sb);
+#pragma unroll
+    for (int c = 0; c < NL; ++c)  // zero beyond the last mode
+      sum += sum_term(mag(I2{__double_as_longlong(v[c].x), __double_as_longlong(v[c].y)}), sb);
+    sum = warp_sum(sum);
+    if (lane == 0) {
+      F::norm_at(sm)[q] = em;
+      F::row_sums(sm)[q] = sum;
+    }
   }
   __syncthreads();
-  const int em8 = max(rmax[2 * pen], rmax[2 * pen + 1]) >> 20;
+  // every mode but k = 0 and L / 2 stands in the pencil twice
+  auto scale_of = [&](int p, int &em) { return F::template row_scale<FX_C2R>(sm, p, kSqrt2 + kTwice, em); };
   {
-    const int sh = shift_of(em8, a.B);
+    int em;
+    const int k8 = scale_of(pen, em), sh = shift_of(em, k8);
+    auto fix = [&](long long b) { return F::steps > 2 ? to_fixed_r(b, sh) : to_fixed_p(b, sh); };
     constexpr int kend = PAD ? kmax : h;
     for (int k = t >> 3; k < kend; k += F::T / 8) {
       longlong2 &wa = sm[F::slot(k, pen)];
       const longlong2 va = wa;
-      const long long ax = to_fixed_p(va.x, sh), ay = to_fixed_p(va.y, sh);
+      const long long ax = fix(va.x), ay = fix(va.y);
       if (k == 0) {
         wa = make_longlong2(ay, ax);
         continue;
       }
       longlong2 &wb = sm[F::slot(L - k, pen)];
       const longlong2 vb = wb;
-      const long long bx = to_fixed_p(vb.x, sh), by = to_fixed_p(vb.y, sh);
+      const long long bx = fix(vb.x), by = fix(vb.y);
       wa = make_longlong2(ay + bx, ax - by);
       wb = make_longlong2(bx - ay, ax + by);
     }
     if (!PAD && t < 8) {
       longlong2 &w = sm[F::slot(h, t)];
       const longlong2 v = w;
-      w = make_longlong2(to_fixed_p(v.y, sh), to_fixed_p(v.x, sh));
+      w = make_longlong2(fix(v.y), fix(v.x));
     }
   }
   __syncthreads();
@@ -635,8 +728,9 @@ __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_fx_c2r_l(const __g
     if (row >= d.rows) break;
     double *dst = base + row * d.pitch;
     const int p = q >> 1, second = q & 1;
-    const int em = max(rmax[2 * p], rmax[2 * p + 1]) >> 20;
-    const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1));
+    int em;
+    const int k = scale_of(p, em);
+    const OutScale os = out_scale(em, F::lost - k);
 #pragma unroll 4
     for (int e = lane; e < L; e += 32)  // exchanged again: the first row is the imaginary part
       dst[e] = to_double_p(reinterpret_cast<const long long *>(&sm[F::slot(e, p)])[1 - second], os);
@@ -651,7 +745,6 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_f
   const Rows &d = a.r;
   constexpr int NL = (L + 31) / 32;
   const int t = threadIdx.x, lane = t & 31, pen = t & 7;
-  int *rmax = reinterpret_cast<int *>(sm + L * 8);
   const Tw3 tw = tw3_of(a.tw, L);
   double *base = static_cast<double *>(d.field[blockIdx.y]);
   const long long row0 = (long long)blockIdx.x * 16;
@@ -678,11 +771,21 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_f
       }
     }
     em = int(__reduce_max_sync(0xffffffffu, unsigned(em)));
-    if (lane == 0) rmax[q] = em;
+    const int sb = sum_base(em);
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < NL; ++c) sum += sum_term(mag(__double_as_longlong(v[c])), sb);
+    sum = warp_sum(sum);
+    if (lane == 0) {
+      F::norm_at(sm)[q] = em;
+      F::row_sums(sm)[q] = sum;
+    }
   }
   __syncthreads();
+  auto scale_of = [&](int p, int &em) { return F::template row_scale<FX_R2C>(sm, p, 0, em); };
   {
-    const int sh = shift_of(max(rmax[2 * pen], rmax[2 * pen + 1]) >> 20, a.B);
+    int em;
+    const int k8 = scale_of(pen, em), sh = shift_of(em, k8);
     typename F::template Regs<0> g;
     F::template load<0>(g, sm, pen);
 #pragma unroll
@@ -709,9 +812,10 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::zctas) k_f
     if (row >= d.rows) break;
     double2 *dst = reinterpret_cast<double2 *>(base + row * d.pitch);
     const int p = q >> 1, second = q & 1;
-    const int em = max(rmax[2 * p], rmax[2 * p + 1]) >> 20;
     // the sums below are twice the spectra
-    const OutScale os = out_scale(em, em - 1022 - a.B + 3 * (F::steps - 1) - 1);
+    int em;
+    const int ks = scale_of(p, em);
+    const OutScale os = out_scale(em, F::lost - ks - 1);
 #pragma unroll 2
     for (int k = lane; k < kc; k += 32) {
       const longlong2 u = sm[F::slot(k, p)], w = sm[F::slot(k ? L - k : 0, p)];
