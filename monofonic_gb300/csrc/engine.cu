@@ -142,7 +142,7 @@ struct mfx_engine {
   // 32^3 pass).  One 64-byte line a job; a job that finds none free has its word
   // in its arena.
   static constexpr int kStatusLines = 1024;
-  std::atomic<int> running{0};  // jobs with a run that has not been waited for
+  std::atomic<int> running{0};  // jobs and batches with a run that is not known to be done
   int *status_host = nullptr;
   std::vector<int> status_free;
 };
@@ -187,7 +187,8 @@ struct mfx_job {
   // of every plain FP64 job (fx::fill_tables)
   double *fx_mode = nullptr, *fx_rinv = nullptr, *fx_root = nullptr;
   int *dstatus = nullptr;      // status word (device address): nonzero when a kernel's bounded wait ran out
-  bool running = false;        // counted in the engine's running jobs
+  std::atomic<bool> running{false};  // counted in the engine's running jobs
+  bool capturing = false;      // its launches are being recorded, not run
   bool shared_gpu = false;     // a server's job: others run beside it
   int status_line = -1;        // its line of the engine's page-locked words, -1: in the arena
   size_t rsize = 8;
@@ -1590,14 +1591,24 @@ static void ring_point(mfx_job *j, int s) {
 // requests took 7.1 instead of 6.5 ms with it, three 128^3 jobs in turn 2.73
 // instead of 2.60 ms a round; alone, 32^3 2LPT goes from 77 to 59 us, 64^3 3LPT
 // from 308 to 226 us.
-static void job_idle(mfx_job *j) {
-  if (j->running) j->eng->running.fetch_sub(1, std::memory_order_relaxed);
-  j->running = false;
+// A job counts from its run, or its graph's launch, until it is known to be done: at
+// a wait, at any call that waits for its stream, when the server finds its ticket
+// done.  A batch counts as one.  Recording a graph runs nothing.
+static void count_in(mfx_engine *eng, std::atomic<bool> &running) {
+  if (!running.exchange(true, std::memory_order_relaxed)) eng->running.fetch_add(1, std::memory_order_relaxed);
+}
+static void count_out(mfx_engine *eng, std::atomic<bool> &running) {
+  if (running.exchange(false, std::memory_order_relaxed)) eng->running.fetch_sub(1, std::memory_order_relaxed);
+}
+static void job_idle(mfx_job *j) { count_out(j->eng, j->running); }
+static cudaError_t job_sync(mfx_job *j) {
+  const cudaError_t e = cudaStreamSynchronize(j->stream);
+  if (e == cudaSuccess) job_idle(j);
+  return e;
 }
 static void pdl_rule(mfx_job *j) {
-  if (!j->running) j->eng->running.fetch_add(1, std::memory_order_relaxed);
-  j->running = true;
-  pdl_enabled() = !j->shared_gpu && j->eng->running.load(std::memory_order_relaxed) == 1;
+  if (!j->capturing) count_in(j->eng, j->running);
+  pdl_enabled() = !j->capturing && !j->shared_gpu && j->eng->running.load(std::memory_order_relaxed) == 1;
 }
 
 template <typename R> static int run_pipeline(mfx_job *j) {
@@ -1871,7 +1882,7 @@ static void free_job(mfx_job *j) {
   if (!j) return;
   join_id_fill(j);
   if (j->stream) cudaStreamSynchronize(j->stream);
-  if (j->eng && j->running) j->eng->running.fetch_sub(1, std::memory_order_relaxed);
+  if (j->eng) job_idle(j);
   if (j->gexec) cudaGraphExecDestroy(j->gexec);
   if (j->graph) cudaGraphDestroy(j->graph);
   if (j->eng) {
@@ -2246,6 +2257,13 @@ static int create_job(mfx_engine *eng, const mfx_job_desc *d, mfx_job **out, int
   return MFX_OK;
 }
 
+// one pass on the job's stream; what failed counts no longer
+static int run_job(mfx_job *j) {
+  const int rc = j->fp64 ? run_pipeline<double>(j) : run_pipeline<float>(j);
+  if (rc != MFX_OK) job_idle(j);
+  return rc;
+}
+
 // Records the job's whole pipeline into a CUDA graph (stream capture on the
 // job stream).  Per-stage events and per-launch profiling stay out of graphs.
 static int capture_pipeline(mfx_job *j, cudaGraph_t *out) {
@@ -2258,7 +2276,9 @@ static int capture_pipeline(mfx_job *j, cudaGraph_t *out) {
     j->timed = timed;
     return set_error(MFX_ECUDA, "cudaStreamBeginCapture: %s", cudaGetErrorString(e));
   }
+  j->capturing = true;
   const int rc = j->fp64 ? run_pipeline<double>(j) : run_pipeline<float>(j);
+  j->capturing = false;
   cudaGraph_t g = nullptr;
   e = cudaStreamEndCapture(j->stream, &g);
   j->prof = prof;
@@ -2284,11 +2304,13 @@ struct mfx_batch {
   cudaStream_t stream = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   bool ran = false;
+  std::atomic<bool> running{false};  // counted in the engine's running jobs
 };
 
 static void free_batch(mfx_batch *b) {
   if (!b) return;
   if (b->stream) cudaStreamSynchronize(b->stream);
+  if (b->eng) count_out(b->eng, b->running);
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->parent) cudaGraphDestroy(b->parent);
   for (auto g : b->children)
@@ -2418,11 +2440,12 @@ int mfx_job_run(mfx_job *job) {
   CU(cudaSetDevice(job->eng->device));
   if (job->gexec) {
     CU(cudaGraphLaunch(job->gexec, job->stream));
+    count_in(job->eng, job->running);
     job->has_run = true;
     job->noise_only = false;
     return MFX_OK;
   }
-  return job->fp64 ? run_pipeline<double>(job) : run_pipeline<float>(job);
+  return run_job(job);
   GUARD_END
 }
 
@@ -2437,9 +2460,12 @@ int mfx_job_assemble(mfx_job *job, int orders_mask) {
   job->prof_recs.clear();
   if (job->fetched) CU(cudaStreamWaitEvent(job->stream, job->fetched, 0));  // downloads of these particles
   pdl_rule(job);
-  TRY(job->fp64 ? assemble_stage<double>(job, orders_mask) : assemble_stage<float>(job, orders_mask));
-  CU(cudaStreamSynchronize(job->stream));
-  job_idle(job);
+  const int rc = job->fp64 ? assemble_stage<double>(job, orders_mask) : assemble_stage<float>(job, orders_mask);
+  if (rc != MFX_OK) {
+    job_idle(job);
+    return rc;
+  }
+  CU(job_sync(job));
   return MFX_OK;
   GUARD_END
 }
@@ -2477,7 +2503,7 @@ int mfx_job_set_species(mfx_job *job, const mfx_species_desc *sp) {
   CU(cudaSetDevice(job->eng->device));
   for (auto &x : job->xfer)
     if (x) CU(cudaStreamSynchronize(x));
-  CU(cudaStreamSynchronize(job->stream));
+  CU(job_sync(job));
   release_species(job);
   if (sp) {
     static const double kSecond[3][3] = {{0.5, 0.5, 0.5}, {0.5, 0.5, 0.0}, {0.5, 0.5, 0.5}};
@@ -2558,7 +2584,7 @@ int mfx_job_set_species(mfx_job *job, const mfx_species_desc *sp) {
       CF(cufftSetWorkArea(job->rho_c2r.h, job->rho_work));
       CF(cufftSetStream(job->rho_c2r.h, job->stream));
     }
-    CU(cudaStreamSynchronize(job->stream));
+    CU(job_sync(job));
   }
   TRY(upload_shift_tables(job));
   return MFX_OK;
@@ -2572,7 +2598,7 @@ int mfx_job_fetch_masses(mfx_job *job, size_t first, size_t count, void *out) {
   if (first > job->npart || count > job->npart - first)
     return set_error(MFX_EINVAL, "range [%zu, %zu) outside the %zu particles", first, first + count, job->npart);
   CU(cudaSetDevice(job->eng->device));
-  CU(cudaStreamSynchronize(job->stream));
+  CU(job_sync(job));
   const size_t es = job->d.pos64 ? 8 : 4;
   CU(cudaMemcpy(out, static_cast<char *>(job->mass) + es * first, es * count, cudaMemcpyDefault));
   return MFX_OK;
@@ -2637,6 +2663,8 @@ int mfx_job_run_noise(mfx_job *job, int raw) {
   if (rc == MFX_OK) {
     job->noise_only = true;
     job->has_run = true;
+  } else {
+    job_idle(job);
   }
   return rc;
   GUARD_END
@@ -2657,8 +2685,7 @@ int mfx_job_wait(mfx_job *job, int timeout_ms) {
   GUARD_BEGIN
   if (!job) return set_error(MFX_EINVAL, "null job");
   if (timeout_ms < 0) {
-    CU(cudaStreamSynchronize(job->stream));
-    job_idle(job);
+    CU(job_sync(job));
     return check_status(job);
   }
   // bounded host-side poll
@@ -2711,6 +2738,7 @@ static int download(mfx_job *j, const Xfer *xs, int n) {
   }
   cudaEventDestroy(ready);
   if (e != cudaSuccess) return set_error(MFX_ECUDA, "particle download: %s", cudaGetErrorString(e));
+  job_idle(j);  // the copies waited for it
   return MFX_OK;
 }
 
@@ -2772,12 +2800,12 @@ int mfx_job_set_host_positions(mfx_job *job, int on) {
   join_id_fill(job);
   for (auto &x : job->xfer)
     if (x) CU(cudaStreamSynchronize(x));
-  CU(cudaStreamSynchronize(job->stream));
+  CU(job_sync(job));
   job->host_q = on != 0;
   // the particles of the last run, in the new form
   if (job->has_run && !job->noise_only) {
     TRY(assemble_stage<float>(job, 7));
-    CU(cudaStreamSynchronize(job->stream));
+    CU(job_sync(job));
   }
   return MFX_OK;
   GUARD_END
@@ -2793,11 +2821,11 @@ int mfx_job_set_output_ring(mfx_job *job, int on) {
   if (on == job->ring_sets) return MFX_OK;
   for (auto &x : job->xfer)
     if (x) CU(cudaStreamSynchronize(x));
-  CU(cudaStreamSynchronize(job->stream));
+  CU(job_sync(job));
   mfx_engine *eng = job->eng;
   if (job->ring) {
     CU(cudaFreeAsync(job->ring, job->stream));
-    CU(cudaStreamSynchronize(job->stream));
+    CU(job_sync(job));
     job->ring = nullptr;
     {
       std::lock_guard<std::mutex> lk(eng->mu);
@@ -2910,7 +2938,7 @@ int mfx_job_particles_device(mfx_job *job, const void **pos, const void **vel, c
         CU(cudaMallocAsync(&job->ids_dev, job->npart * (job->d.id64 ? 8 : 4), job->stream));
       }
       TRY(fill_ids_device(job, 0, job->npart, job->ids_dev, job->stream));
-      CU(cudaStreamSynchronize(job->stream));
+      CU(job_sync(job));
       *ids = job->ids_dev;
     }
   }
@@ -2941,7 +2969,7 @@ int mfx_job_fetch_field(mfx_job *job, int field_id, double *out) {
   if (field_id != MFX_FIELD_NOISE && job->noise_only) return set_error(MFX_ESTATE, "only the noise was run");
   if (!job->nf[slot]) return set_error(MFX_EINVAL, "field %d not computed at LPT order %d", field_id, job->d.lpt_order);
   const size_t nc = size_t(job->N) * job->N * job->nk;
-  CU(cudaStreamSynchronize(job->stream));
+  CU(job_sync(job));
   if (job->fp64) {
     CU(cudaMemcpy(out, job->nf[slot], nc * 16, cudaMemcpyDeviceToHost));
     if (scale != 1.0)
@@ -2958,7 +2986,7 @@ int mfx_job_fetch_field(mfx_job *job, int field_id, double *out) {
 int mfx_job_stage_times(mfx_job *job, double *ms, int max_stages) {
   if (!job || !ms) return set_error(MFX_EINVAL, "null argument");
   if (!job->has_run || job->noise_only) return 0;
-  if (cudaStreamSynchronize(job->stream) != cudaSuccess) return set_error(MFX_ECUDA, "sync failed");
+  if (job_sync(job) != cudaSuccess) return set_error(MFX_ECUDA, "sync failed");
   int n = 0;
   for (int s = 0; s < 4 && n < max_stages; ++s) {
     // below third order the phi2 stage ends where the (empty) phi3 stage would:
@@ -3007,7 +3035,7 @@ int mfx_job_set_profiling(mfx_job *job, int on) {
 
 int mfx_job_kernel_profile(mfx_job *job, int max_entries, char *names, double *ms, double *bytes, int *launches) {
   if (!job) return set_error(MFX_EINVAL, "null job");
-  if (cudaStreamSynchronize(job->stream) != cudaSuccess) return set_error(MFX_ECUDA, "sync failed");
+  if (job_sync(job) != cudaSuccess) return set_error(MFX_ECUDA, "sync failed");
   std::vector<std::string> keys;
   std::vector<double> t, b;
   std::vector<int> c;
@@ -3086,6 +3114,7 @@ int mfx_batch_run(mfx_batch *b) {
   CU(cudaSetDevice(b->eng->device));
   CU(cudaEventRecord(b->e0, b->stream));
   CU(cudaGraphLaunch(b->exec, b->stream));
+  count_in(b->eng, b->running);
   CU(cudaEventRecord(b->e1, b->stream));
   for (auto j : b->jobs) {
     j->has_run = true;
@@ -3100,6 +3129,7 @@ int mfx_batch_wait(mfx_batch *b, double *device_ms) {
   GUARD_BEGIN
   if (!b) return set_error(MFX_EINVAL, "null batch");
   CU(cudaStreamSynchronize(b->stream));
+  count_out(b->eng, b->running);
   if (device_ms) {
     float ms = 0;
     if (b->ran) CU(cudaEventElapsedTime(&ms, b->e0, b->e1));
@@ -3269,6 +3299,7 @@ static void server_loop(mfx_server *s) {
         t->rc = MFX_ECUDA;
         t->err = cudaGetErrorString(q);
       }
+      job_idle(t->job);
       --(t->small ? s->inflight_small : s->inflight);
       s->cv.notify_all();
     }
@@ -3319,7 +3350,7 @@ static void setup_loop(mfx_server *s) {
     int rc = create_job(s->eng, &t->d, &j, s->size_priority ? stream_priority_for(t->footprint, s->small_first) : 0);
     std::string err = rc == MFX_OK ? "" : g_last_error;
     if (rc == MFX_OK) j->shared_gpu = true;
-    if (rc == MFX_OK) rc = j->fp64 ? run_pipeline<double>(j) : run_pipeline<float>(j);
+    if (rc == MFX_OK) rc = run_job(j);
     if (rc == MFX_OK && cudaEventRecord(t->done, j->stream) != cudaSuccess) rc = MFX_ECUDA;
     if (rc != MFX_OK && err.empty()) err = g_last_error;
     if (rc != MFX_OK && j) {
