@@ -240,12 +240,7 @@ __global__ void __launch_bounds__(768) k_fx_strided(const __grid_constant__ SArg
       const int k2 = scale(a.c, high_word(top2, 32), high_word(sum2, 47) - 0x3ff00000);
       for (int l = t >> lgP; l < L; l += step_l) {
         longlong2 &w = sm[slot(l, pen, lgP)];
-        if (k2 < 0) {
-          const long long half = 1LL << (-k2 - 1);
-          w = make_longlong2((w.x + half) >> -k2, (w.y + half) >> -k2);
-        } else {
-          w = make_longlong2(w.x << k2, w.y << k2);
-        }
+        w = make_longlong2(rescale(w.x, k2), rescale(w.y, k2));
       }
       __syncthreads();
       S += lost - k2;

@@ -122,8 +122,20 @@ template <long long W> FX_HD long long mulk(long long a) {
   return mulq(a + a, wh, wl);
 }
 template <long long W> FX_HD I2 mulk(I2 a) { return {mulk<W>(a.x), mulk<W>(a.y)}; }
-FX_HD I2 minus_half(I2 a, I2 b) { return {a.x - (b.x >> 1), a.y - (b.y >> 1)}; }
-FX_HD I2 minus_quarter(I2 a, I2 b) { return {a.x - (b.x >> 2), a.y - (b.y >> 2)}; }
+// Halves and quarters are rounded to even: an offset, as of a floor, would be the
+// same in every pencil, and the passes that follow would sum it over the grid into
+// the modes along an axis (phi(2)'s lowest modes at 288^3 were off by 4e-15 of its
+// norm, with cuFFT by 5e-16).
+FX_HD long long minus_half(long long a, long long b) {
+  const long long h = b >> 1;
+  return a - h - (h & b & 1);
+}
+FX_HD long long minus_quarter(long long a, long long b) {
+  const long long h = b >> 2;
+  return a - h - ((b >> 1) & (b | h) & 1);
+}
+FX_HD I2 minus_half(I2 a, I2 b) { return {minus_half(a.x, b.x), minus_half(a.y, b.y)}; }
+FX_HD I2 minus_quarter(I2 a, I2 b) { return {minus_quarter(a.x, b.x), minus_quarter(a.y, b.y)}; }
 
 // the same DFTs in single precision (fs32.cuh)
 struct F2 {
@@ -309,15 +321,25 @@ template <> struct Dft<7> {
 // v w; the element that a step's twiddles leave alone is quartered like them.
 // Three products: c = cos, s = -sin, the constants c, s + c and s - c split into
 // signed halves (hi, lo)
-FX_HD I2 quarter(I2 v) { return {(v.x + 2) >> 2, (v.y + 2) >> 2}; }
+FX_HD long long quarter(long long v) { return (v + 1 + ((v >> 2) & 1)) >> 2; }
+FX_HD I2 quarter(I2 v) { return {quarter(v.x), quarter(v.y)}; }
+// v 2^k, rounded, halves away from zero: modes of either sign, no offset
+FX_HD long long rescale(long long v, int k) {
+  const int dn = k < 0 ? -k : 0;
+  const long long half = dn ? (1LL << (dn - 1)) + (v >> 63) : 0;
+  return dn ? (v + half) >> dn : v << k;
+}
 FX_HD I2 twiddle4(I2 v, int4 c_p, int2 m) {
   const long long k = mulq(v.x + v.y, c_p.x, c_p.y);
   return {k - mulq(v.y, c_p.z, c_p.w), k + mulq(v.x, m.x, m.y)};
 }
-// the constants of (cos, -sin)(2 pi t / L)
+// The constants of (cos, -sin)(2 pi t / L).  Powers of two (1, 1/2) are one unit
+// smaller: their products would end in halves, which mulq rounds up, an offset in
+// the modes 0 of all pencils; so these halves round towards zero.
 inline void twiddle_constants(int t, int L, int4 *c_p, int2 *m) {
   const CS w = q62_turn(t, L);
-  const long long c = (long long)w.c, s = (long long)-w.s;
+  auto inexact = [](long long v) { return (v & 0xffffffffLL) || v == 0 ? v : (v > 0 ? v - 1 : v + 1); };
+  const long long c = inexact((long long)w.c), s = inexact((long long)-w.s);
   auto lo = [](long long w) { return int(w); };
   auto hi = [](long long w) { return int(w >> 32) + int(unsigned(int(w)) >> 31); };
   *c_p = make_int4(hi(c), lo(c), hi(s + c), lo(s + c));

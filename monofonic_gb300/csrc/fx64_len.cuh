@@ -579,15 +579,17 @@ template <int L> __global__ void __launch_bounds__(Len<L>::T, Len<L>::ctas) k_fx
   unsigned sum2 = norm.thread_sum();
   I::pencil_norm(top2, sum2, I::norm_at(sm) + 2 * F::W * 8);
   const int k2 = I::template scale<FX_STRIDED>(high_word(top2, 32), high_word(sum2, 47) - 0x3ff00000);
+  // rescale() without a branch per value
   const int dn = max(-k2, 0), up = max(k2, 0);
-  const long long half = dn ? 1LL << (dn - 1) : 0;
+  const long long half = dn ? 1LL << (dn - 1) : 0, sign = dn ? -1 : 0;
 #pragma unroll
   for (int m = 0; m < I::MU(0); ++m)
     if (I::template live<0>(m)) {
 #pragma unroll
       for (int r = 0; r < RL; ++r)
         if (zone<RL>(r) != Z_NYQ && zone<RL>(r) != Z_PAD)
-          h.v[m][r] = {((h.v[m][r].x + half) >> dn) << up, ((h.v[m][r].y + half) >> dn) << up};
+          h.v[m][r] = {((h.v[m][r].x + half + ((h.v[m][r].x >> 63) & sign)) >> dn) << up,
+                       ((h.v[m][r].y + half + ((h.v[m][r].y >> 63) & sign)) >> dn) << up};
     }
   I::template butterfly<0>(h, tw);
   I::template store<0>(h, sm, pen);

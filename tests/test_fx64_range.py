@@ -115,3 +115,21 @@ def test_no_less_precise_than_fp64(harness, power):
         ours, fp64 = rel(run(exe, L, kind, radices, x), want), rel(transform(kind, x, L), want)
         rms = [float(np.sqrt(np.mean(e ** 2))) for e in (ours, fp64)]
         assert rms[0] <= rms[1], (L, kind, radices, rms)
+
+
+@pytest.mark.parametrize("L", [64, 72, 96, 100, 150, 288, 384, 432, 512, 576])
+def test_errors_have_no_offset(harness, L):
+    """The mean error of each output over many pencils is zero: the passes that
+    follow sum an offset over the whole grid.  The mean of n errors exceeds t of
+    their standard deviations with a probability below 2 exp(-n t^2 / 2); 0.1 at
+    n = 4000 is 1e-4 for all outputs here together."""
+    exe, plans = harness
+    n = 4000
+    for length, kind, radices in plans:
+        if length != L:
+            continue
+        x = layout(spectra(L, np.random.default_rng(L), 0, n), kind, L)
+        err = (run(exe, L, kind, radices, x) - transform(kind, wide(x), L)).astype(complex)
+        sd = np.sqrt(np.mean(np.abs(err) ** 2, axis=0))
+        off = np.abs(np.mean(err, axis=0)) / np.where(sd > 0, sd, 1)
+        assert off.max() < 0.1, (kind, radices, off.max(), int(off.argmax()))
