@@ -465,6 +465,7 @@ static const LenEntry *find_len(int L) {
   return nullptr;
 }
 static __global__ void k_fx_tables(int n, double *mode, double *rinv, double *root, int len) {
+  mfx::pdl_begin();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < len; q += gridDim.x * blockDim.x) {
     rinv[q] = q ? 1.0 / double(q) : 0.0;
     root[q] = sqrt(double(q));
