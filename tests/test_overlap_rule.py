@@ -8,9 +8,9 @@ CSRC = pathlib.Path(__file__).resolve().parent.parent / "monofonic_gb300" / "csr
 
 
 def bodies(text):
-    """{kernel: body} of the __global__ functions of a source."""
+    """{name: body} of the kernels and of the z passes that some of them consist of."""
     out = {}
-    for m in re.finditer(r"__global__[^;{]*?\b(k_\w+)\s*\([^;{]*?\)\s*\{", text):
+    for m in re.finditer(r"(?:__global__[^;{]*?\b(?=k_)|__device__[^;{]*?\b(?=z_rows))(\w+)\s*\([^;{]*?\)\s*\{", text):
         depth, end = 1, m.end()
         while depth:
             depth += {"{": 1, "}": -1}.get(text[end], 0)
@@ -26,4 +26,8 @@ def test_overlapping_launches_wait():
         kernels.update(bodies(text))
         launched |= set(re.findall(r"(?:launch_pdl|MFX_FF_PERSISTENT)\(\(?(k_\w+)", text))
     assert len(launched) >= 39 and launched <= set(kernels), launched - set(kernels)
-    assert not [k for k in sorted(launched) if not re.search(r"pdl_begin\(\)|load_tw(_steps)?<", kernels[k])]
+    waits = re.compile(r"pdl_begin\(\)|load_tw(_steps)?<")
+    parts = [k for k in kernels if not k.startswith("k_") and waits.search(kernels[k])]
+    assert len(parts) == 2
+    waits = re.compile("|".join([waits.pattern] + [p + "<" for p in parts]))
+    assert not [k for k in sorted(launched) if not waits.search(kernels[k])]
