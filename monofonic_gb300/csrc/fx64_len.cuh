@@ -4,9 +4,10 @@
 // shared-memory exchange for two steps).  Lengths without an instance take the
 // run-time kernels of fx64.cu.
 //
-// What bounds them: integer instructions (the ALU pipe was 63% busy in the z
-// passes, issue 56%, HBM 26%, before the zero third was skipped), so what they
-// save is instructions.
+// What bounds them: at 384 the ALU pipe is 54% busy in the z passes (FP64, the
+// conversions back, 20 - 30%, HBM 30%), 37% in the x and y passes (FP64 45%, HBM 20 -
+// 25%), the rest is latency at the 12 - 18 warps that their registers leave an SM.
+// So what they save is instructions.
 //  * A padded length L = 3N/2 is split so that the step at its N-grid side (the
 //    first of an inverse transform, the last of a forward one) has a radix
 //    divisible by three: inputs r of R / 3 < r < 2R / 3 of that step are the
